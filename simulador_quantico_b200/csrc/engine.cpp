@@ -289,8 +289,7 @@ int hgm_measure_qubit(hgm_state *s, int qubit, double sample, int *outcome, doub
     if (qubit < 0 || qubit >= st->qubits) return fail(HGM_ERR_INVALID, "qubit %d outside state", qubit);
     const int bit = st->qubits - 1 - qubit;
     double total = 0, one = 0;
-    int rc = reduce_norm(st, &total, nullptr);
-    if (!rc) rc = reduce_prob_one(st, bit, &one, nullptr);
+    int rc = reduce_split(st, bit, &total, &one, nullptr);
     if (rc) return rc;
     const double zero = total - one;
     // DGM::measure: outcome 0 iff P(0) > sample (dgm_core.cpp:97-113)
@@ -313,8 +312,7 @@ int hgm_collapse_qubit(hgm_state *s, int qubit, int value, double *prob) {
     if (value != 0 && value != 1) return fail(HGM_ERR_INVALID, "value %d is not 0 or 1", value);
     const int bit = st->qubits - 1 - qubit;
     double total = 0, one = 0;
-    int rc = reduce_norm(st, &total, nullptr);
-    if (!rc) rc = reduce_prob_one(st, bit, &one, nullptr);
+    int rc = reduce_split(st, bit, &total, &one, nullptr);
     if (rc) return rc;
     const double p = value ? one : total - one;
     if (!(p > 0)) return fail(HGM_ERR_INVALID, "collapse onto a value of zero probability");

@@ -336,6 +336,8 @@ const void *chain_error_word(const Plan *p);
 int launch_set_basis(State *s, int64_t index, void *stream);
 int reduce_norm(State *s, double *out, void *stream);
 int reduce_prob_one(State *s, int bit, double *out, void *stream);
+// The norm and the probability that `bit` is 1, in one read of the state.
+int reduce_split(State *s, int bit, double *total, double *one, void *stream);
 int collapse(State *s, int bit, int value, double inv_norm, void *stream);
 int measure_update(State *s, int bit, int value, double inv_norm, void *stream);
 int marginal_argmax(State *s, uint64_t mask, int64_t *arg, double *prob, void *stream);

@@ -25,18 +25,21 @@ namespace hgm {
 namespace {
 constexpr int RED_BLOCKS = REDUCE_SCRATCH_BLOCKS;   // 8 x 148 SMs
 constexpr int RED_THREADS = 256;
+constexpr size_t MARGINAL_SCRATCH = size_t(2) << 20;
 
 struct Ctx {
     int device = -1;
     cudaStream_t stream = nullptr;
     double *partials = nullptr;    // RED_BLOCKS * 2 doubles
     long long *partial_idx = nullptr;
-    double *result = nullptr;      // 4 doubles (device)
-    double *host_result = nullptr; // 4 doubles (pinned)
+    double *host_result = nullptr; // 4 doubles (pinned; kernels write it)
+    double *marginal = nullptr;    // MARGINAL_SCRATCH bytes
     cudaEvent_t t0 = nullptr, t1 = nullptr;
 };
 Ctx g_ctx;
 std::mutex g_ctx_mu;
+// held by a synchronous reduction while it uses the context's scratch
+std::mutex g_reduce_mu;
 std::atomic<long long> g_launches{0};
 }  // namespace
 
@@ -55,7 +58,7 @@ static int ensure_ctx() {
         return fail(HGM_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
     if ((e = cudaMalloc(&g_ctx.partials, RED_BLOCKS * 2 * sizeof(double))) != cudaSuccess ||
         (e = cudaMalloc(&g_ctx.partial_idx, RED_BLOCKS * sizeof(long long))) != cudaSuccess ||
-        (e = cudaMalloc(&g_ctx.result, 4 * sizeof(double))) != cudaSuccess ||
+        (e = cudaMalloc(&g_ctx.marginal, MARGINAL_SCRATCH)) != cudaSuccess ||
         (e = cudaMallocHost(&g_ctx.host_result, 4 * sizeof(double))) != cudaSuccess ||
         (e = cudaEventCreate(&g_ctx.t0)) != cudaSuccess || (e = cudaEventCreate(&g_ctx.t1)) != cudaSuccess)
         return fail(HGM_ERR_CUDA, "context setup: %s", cudaGetErrorString(e));
@@ -612,7 +615,8 @@ int scale_state(State *s, double f, void *stream) {
 // FP64 reductions (fixed grid, fixed combine order)
 // ---------------------------------------------------------------------------
 
-enum RedMode { RED_NORM = 0, RED_PROB1 = 1, RED_INNER = 2, RED_MAXDIFF = 3 };
+// RED_SPLIT: the norm and, of it, the share where `bit` is 1, in one read
+enum RedMode { RED_NORM = 0, RED_PROB1 = 1, RED_INNER = 2, RED_MAXDIFF = 3, RED_SPLIT = 4 };
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -636,6 +640,10 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(const typename V2<R
             s0 += (double)x.x * x.x + (double)x.y * x.y;
         } else if (MODE == RED_PROB1) {
             if ((i >> bit) & 1) s0 += (double)x.x * x.x + (double)x.y * x.y;
+        } else if (MODE == RED_SPLIT) {
+            const double q = (double)x.x * x.x + (double)x.y * x.y;
+            s0 += q;
+            if ((i >> bit) & 1) s1 += q;
         } else if (MODE == RED_INNER) {
             const typename V2<RB>::T y = b[i];
             // conj(x) * y
@@ -671,30 +679,54 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(const typename V2<R
     }
 }
 
+// Combines the block partials: one block, each thread its strided share, then
+// the warps' sums, in a fixed order.  (One thread walking the 1184 partials
+// alone took 82 us, twice the 41 us that reading a 256 MiB state takes; this
+// takes 5 us.)
 template <int MODE>
-__global__ void reduce_final(const double *partials, int nblocks, double *out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double t0 = 0.0, t1 = 0.0;
-        for (int k = 0; k < nblocks; k++) {
-            if (MODE == RED_MAXDIFF) t0 = fmax(t0, partials[2 * k]);
-            else t0 += partials[2 * k];
-            t1 += partials[2 * k + 1];
+__global__ void __launch_bounds__(RED_THREADS) reduce_final(const double *partials, int nblocks, double *out,
+                                                            int n_out) {
+    double t0 = 0.0, t1 = 0.0;
+    for (int k = threadIdx.x; k < nblocks; k += RED_THREADS) {
+        if (MODE == RED_MAXDIFF) t0 = fmax(t0, partials[2 * k]);
+        else t0 += partials[2 * k];
+        t1 += partials[2 * k + 1];
+    }
+    if (MODE == RED_MAXDIFF) t0 = warp_max(t0);
+    else t0 = warp_sum(t0);
+    t1 = warp_sum(t1);
+    __shared__ double sh[2][RED_THREADS / 32];
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = t0;
+        sh[1][threadIdx.x >> 5] = t1;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        t0 = t1 = 0.0;
+        for (int k = 0; k < RED_THREADS / 32; k++) {
+            if (MODE == RED_MAXDIFF) t0 = fmax(t0, sh[0][k]);
+            else t0 += sh[0][k];
+            t1 += sh[1][k];
         }
         out[0] = t0;
-        out[1] = t1;
+        if (n_out > 1) out[1] = t1;
     }
 }
 
+// Synchronous reductions share the context's scratch and its page-locked
+// result words, which the last kernel writes itself (no copy behind it).
 template <typename RA, typename RB, int MODE>
 static int run_reduce(const void *a, const void *b, int qubits, int bit, double *o0, double *o1, cudaStream_t st) {
     const long long N = 1ll << qubits;
     const unsigned g = grid_for(N);
+    std::lock_guard<std::mutex> lk(g_reduce_mu);
     reduce_kernel<RA, RB, MODE><<<g, RED_THREADS, 0, st>>>((const typename V2<RA>::T *)a,
                                                            (const typename V2<RB>::T *)b, N, bit, g_ctx.partials);
-    reduce_final<MODE><<<1, 32, 0, st>>>(g_ctx.partials, (int)g, g_ctx.result);
+    reduce_final<MODE><<<1, RED_THREADS, 0, st>>>(g_ctx.partials, (int)g, g_ctx.host_result, 2);
     count_launch(2);
-    cudaMemcpyAsync(g_ctx.host_result, g_ctx.result, 2 * sizeof(double), cudaMemcpyDeviceToHost, st);
+    int rc = check("reduction launch");
     cudaError_t e = cudaStreamSynchronize(st);
+    if (rc) return rc;
     if (e != cudaSuccess) return fail(HGM_ERR_CUDA, "reduction: %s", cudaGetErrorString(e));
     if (o0) *o0 = g_ctx.host_result[0];
     if (o1) *o1 = g_ctx.host_result[1];
@@ -709,7 +741,7 @@ int launch_norm_async(State *s, double *partials, double *out, void *stream) {
         reduce_kernel<double, double, RED_NORM><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, nullptr, N, 0, partials);
     else
         reduce_kernel<float, float, RED_NORM><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, nullptr, N, 0, partials);
-    reduce_final<RED_NORM><<<1, 32, 0, st>>>(partials, (int)g, out);
+    reduce_final<RED_NORM><<<1, RED_THREADS, 0, st>>>(partials, (int)g, out, 2);
     count_launch(2);
     return check("norm reduction launch");
 }
@@ -727,6 +759,14 @@ int reduce_prob_one(State *s, int bit, double *out, void *stream) {
     if (bit < 0 || bit >= s->qubits) return fail(HGM_ERR_INVALID, "bit %d outside state", bit);
     return s->precision == HGM_F64 ? run_reduce<double, double, RED_PROB1>(s->d, nullptr, s->qubits, bit, out, nullptr, st)
                                    : run_reduce<float, float, RED_PROB1>(s->d, nullptr, s->qubits, bit, out, nullptr, st);
+}
+
+int reduce_split(State *s, int bit, double *total, double *one, void *stream) {
+    cudaStream_t st = pick(stream);
+    if (!st) return HGM_ERR_CUDA;
+    if (bit < 0 || bit >= s->qubits) return fail(HGM_ERR_INVALID, "bit %d outside state", bit);
+    return s->precision == HGM_F64 ? run_reduce<double, double, RED_SPLIT>(s->d, nullptr, s->qubits, bit, total, one, st)
+                                   : run_reduce<float, float, RED_SPLIT>(s->d, nullptr, s->qubits, bit, total, one, st);
 }
 
 template <int MODE>
@@ -751,202 +791,266 @@ int max_abs_diff(State *a, State *b, double *out, void *stream) {
     return two_state<RED_MAXDIFF>(a, b, out, nullptr, st);
 }
 
-// Marginal argmax: for every value x of the bits in `mask`, p(x) = sum over
-// the other bits of |a|^2; returns the x with the largest p (lowest on ties).
-// Each thread owns marginal values x and walks the complement bits.
-template <typename Real>
+// ---- marginals ---------------------------------------------------------------
+// For every value x of the bits in `mask` (bit j of x is the j-th lowest mask
+// bit), p(x) = sum over the other bits of |a|^2; either all of them
+// (DGM::measure(vector), src/core/dgm_core.cpp:150-162) or the x with the
+// largest p (lowest on ties).
+//
+// A block reads whole runs of the lowest 11 index bits (16 KiB FP32, 32 KiB
+// FP64): lanes and warps are bits 0..7, each thread's eight accumulators bits
+// 8..10, so loads are contiguous whatever the mask is and eight are in flight
+// a thread.  A unit is one value of the mask bits above those and one of `nch`
+// equal chunks of the other high bits; the block walks the chunk by adding to
+// a masked index, ((c | ~mask) + 1) & mask, which steps through the deposited
+// values without depositing bits one by one.  At the unit's end the sums are
+// folded over the accumulators, lanes and warps whose bit is outside the
+// mask, always in the same order.
+// Bound by reading the state once.  25 qubits FP32, 11 bits: 52 us, 5.2 TB/s (one
+// thread per value before, 8 blocks, a bit deposit per element: 17.9 ms; a
+// block's warps on scattered 256-byte runs: 113 us, waiting on DRAM).  The
+// argmax over all 25 bits: 1064 us before, now 42-45 us (6 TB/s).
+constexpr int MARG_WARPS = RED_THREADS / 32;
+constexpr int MARG_LOW = 11, MARG_ACC = 8;
+
+__device__ __forceinline__ unsigned long long deposit_bits(unsigned long long v, unsigned long long mask) {
+    unsigned long long out = 0;
+    while (mask) {
+        const unsigned long long low = mask & (0ull - mask);
+        if (v & 1ull) out |= low;
+        v >>= 1;
+        mask ^= low;
+    }
+    return out;
+}
+
+// The better of two (probability, value) candidates: the larger probability,
+// then the lower value; a NaN never wins.
+__device__ __forceinline__ void keep_best(double &p, long long &i, double q, long long j) {
+    if (q > p || (q == p && j < i)) {
+        p = q;
+        i = j;
+    }
+}
+
+// Block-wide best; the result is valid in thread 0.
+__device__ __forceinline__ void block_best(double &p, long long &i) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const double q = __shfl_xor_sync(0xffffffffu, p, o);
+        const long long j = __shfl_xor_sync(0xffffffffu, i, o);
+        keep_best(p, i, q, j);
+    }
+    __shared__ double sp[MARG_WARPS];
+    __shared__ long long si[MARG_WARPS];
+    if ((threadIdx.x & 31) == 0) {
+        sp[threadIdx.x >> 5] = p;
+        si[threadIdx.x >> 5] = i;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = 1; k < MARG_WARPS; k++) keep_best(p, i, sp[k], si[k]);
+}
+
+// ARGMAX: block b's best to pbest[b], ibest[b] (nch must be 1); otherwise
+// unit (x, chunk)'s sum to out[x * nch + chunk].
+template <typename Real, bool ARGMAX>
 __global__ void __launch_bounds__(RED_THREADS) marginal_kernel(const typename V2<Real>::T *__restrict__ s, int n,
-                                                                unsigned long long mask, int m, double *pbest,
-                                                                long long *ibest) {
-    const unsigned long long comp = ~mask & ((n >= 64) ? ~0ull : ((1ull << n) - 1));
-    const long long M = 1ll << m, C = 1ll << (n - m);
+                                                                unsigned long long mask, int nch, double *out,
+                                                                double *pbest, long long *ibest) {
+    const int tid = threadIdx.x;
+    const int lb = n < MARG_LOW ? n : MARG_LOW, nh = n - lb;
+    const uint32_t mlo = (uint32_t)mask & ((1u << lb) - 1u);
+    const unsigned long long mhi = mask >> lb, chi = ~mhi & ((1ull << nh) - 1ull);
+    const int m_lo = __popc(mlo);
+    const long long units = (1ll << __popcll(mhi)) * nch, count = (1ll << __popcll(chi)) / nch;
+    const int accs = lb > 8 ? 1 << (lb - 8) : 1;  // accumulators in use
+    const bool live = tid < (1 << lb);
+    __shared__ double sh[MARG_ACC][RED_THREADS];
     double best = -1.0;
     long long besti = 0;
-    for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < M; x += (long long)gridDim.x * blockDim.x) {
-        // deposit x into mask bits
-        unsigned long long base = 0, src = (unsigned long long)x, mm = mask;
-        while (mm) {
-            int g = __ffsll((long long)mm) - 1;
-            mm &= mm - 1;
-            base |= (src & 1ull) << g;
-            src >>= 1;
-        }
-        double p = 0.0;
-        for (long long c = 0; c < C; c++) {
-            unsigned long long idx = base, cs = (unsigned long long)c, cm = comp;
-            while (cm) {
-                int g = __ffsll((long long)cm) - 1;
-                cm &= cm - 1;
-                idx |= (cs & 1ull) << g;
-                cs >>= 1;
+    for (long long u = blockIdx.x; u < units; u += gridDim.x) {
+        const long long xh = u / nch, chunk = u % nch;
+        const unsigned long long hi = deposit_bits((unsigned long long)xh, mhi);
+        unsigned long long c = deposit_bits((unsigned long long)(chunk * count), chi);
+        double p[MARG_ACC];
+#pragma unroll
+        for (int k = 0; k < MARG_ACC; k++) p[k] = 0.0;
+        if (accs == MARG_ACC) {
+#pragma unroll 2
+            for (long long j = 0; j < count; j++) {
+                const typename V2<Real>::T *__restrict__ src = s + ((hi | c) << MARG_LOW) + tid;
+#pragma unroll
+                for (int k = 0; k < MARG_ACC; k++) {
+                    const typename V2<Real>::T v = __ldcs(src + k * RED_THREADS);
+                    p[k] += (double)v.x * v.x + (double)v.y * v.y;
+                }
+                c = ((c | ~chi) + 1ull) & chi;
             }
-            const typename V2<Real>::T v = s[idx];
-            p += (double)v.x * v.x + (double)v.y * v.y;
+        } else if (live) {  // a state of fewer than 11 qubits: one run
+            for (int k = 0; k < accs; k++) {
+                const typename V2<Real>::T v = s[tid + k * RED_THREADS];
+                const double q = (double)v.x * v.x + (double)v.y * v.y;
+#pragma unroll
+                for (int r = 0; r < MARG_ACC; r++)
+                    if (r == k) p[r] = q;
+            }
         }
+        // fold over the accumulators, lanes and warps outside the mask; an
+        // unused accumulator, lane or warp holds zero
+#pragma unroll
+        for (int b = 0; b < 3; b++)
+            if (!((mlo >> (8 + b)) & 1u)) {
+#pragma unroll
+                for (int k = 0; k < MARG_ACC; k++)
+                    if (!(k & (1 << b))) p[k] += p[k | (1 << b)];
+            }
+        for (int b = 0; b < 5; b++)
+            if (!((mlo >> b) & 1u)) {
+#pragma unroll
+                for (int k = 0; k < MARG_ACC; k++) p[k] += __shfl_xor_sync(0xffffffffu, p[k], 1 << b);
+            }
+#pragma unroll
+        for (int k = 0; k < MARG_ACC; k++) sh[k][tid] = p[k];
+        __syncthreads();
+        const uint32_t over = ~mlo & 0xe0u;  // warp bits outside the mask
+        if (live && !((uint32_t)tid & ~mlo)) {
+            for (int k = 0; k < accs; k++) {
+                if (((uint32_t)k << 8) & ~mlo) continue;
+                double t = 0.0;
+                uint32_t w = 0;
+                do {
+                    t += sh[k][(uint32_t)tid | w];
+                    w = ((w | ~over) + 1u) & over;
+                } while (w);
+                uint32_t xl = 0;  // this run position's mask bits, packed
+                const uint32_t pos = (uint32_t)tid | ((uint32_t)k << 8);
+                for (uint32_t m = mlo, j = 0; m; m &= m - 1, j++) xl |= ((pos >> (__ffs((int)m) - 1)) & 1u) << j;
+                const long long x = (xh << m_lo) | xl;
+                if (ARGMAX) keep_best(best, besti, t, x);
+                else out[x * nch + chunk] = t;
+            }
+        }
+        __syncthreads();
+    }
+    if (ARGMAX) {
+        block_best(best, besti);
+        if (threadIdx.x == 0) {
+            pbest[blockIdx.x] = best;
+            ibest[blockIdx.x] = besti;
+        }
+    }
+}
+
+// Argmax over every index bit (a search without ancilla): no sums, one
+// streaming read.
+template <typename Real>
+__global__ void __launch_bounds__(RED_THREADS) argmax_all_kernel(const typename V2<Real>::T *__restrict__ s,
+                                                                  long long N, double *pbest, long long *ibest) {
+    double best = -1.0;
+    long long besti = 0;
+#pragma unroll 4
+    for (long long i = blockIdx.x * (long long)RED_THREADS + threadIdx.x; i < N; i += (long long)gridDim.x * RED_THREADS) {
+        const typename V2<Real>::T v = __ldcs(s + i);
+        const double p = (double)v.x * v.x + (double)v.y * v.y;
         if (p > best) {
             best = p;
-            besti = x;
+            besti = i;
         }
     }
-    __shared__ double sp[RED_THREADS];
-    __shared__ long long si[RED_THREADS];
-    sp[threadIdx.x] = best;
-    si[threadIdx.x] = besti;
-    __syncthreads();
+    block_best(best, besti);
     if (threadIdx.x == 0) {
-        double b = -1.0;
-        long long bi = 0;
-        for (int k = 0; k < RED_THREADS; k++)
-            if (sp[k] > b || (sp[k] == b && si[k] < bi)) {
-                b = sp[k];
-                bi = si[k];
-            }
-        pbest[blockIdx.x] = b;
-        ibest[blockIdx.x] = bi;
+        pbest[blockIdx.x] = best;
+        ibest[blockIdx.x] = besti;
     }
 }
 
-__global__ void marginal_final(const double *pbest, const long long *ibest, int nb, double *out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double b = -1.0;
-        long long bi = 0;
-        for (int k = 0; k < nb; k++)
-            if (pbest[k] > b || (pbest[k] == b && ibest[k] < bi)) {
-                b = pbest[k];
-                bi = ibest[k];
-            }
+__global__ void __launch_bounds__(RED_THREADS) marginal_final(const double *pbest, const long long *ibest, int nb,
+                                                               double *out) {
+    double b = -1.0;
+    long long bi = 0;
+    for (int k = threadIdx.x; k < nb; k += RED_THREADS) keep_best(b, bi, pbest[k], ibest[k]);
+    block_best(b, bi);
+    if (threadIdx.x == 0) {
         out[0] = b;
         out[1] = (double)bi;
     }
 }
 
-// Marginal argmax for a small mask (2^m <= RED_BLOCKS values): block b
-// handles value x = b / nch over the (b % nch)-th chunk of the complement
-// indices, its threads striding over the chunk, and writes that chunk's
-// probability; marginal_chunks_final sums each value's chunks in order.  With
-// the per-value kernel above, a thread would walk all 2^(n-m) complement
-// indices of its value alone (minutes for a few-bit mask on a 32-qubit state).
-template <typename Real>
-__global__ void __launch_bounds__(RED_THREADS) marginal_chunk_kernel(const typename V2<Real>::T *__restrict__ s, int n,
-                                                                      unsigned long long mask, int nch,
-                                                                      double *partial) {
-    const unsigned long long comp = ~mask & ((n >= 64) ? ~0ull : ((1ull << n) - 1));
-    const long long C = 1ll << (n - __popcll(mask));
-    const long long x = blockIdx.x / nch, chunk = blockIdx.x % nch;
-    const long long cs = (C + nch - 1) / nch, c0 = chunk * cs, c1 = c0 + cs < C ? c0 + cs : C;
-    unsigned long long base = 0, src = (unsigned long long)x, mm = mask;
-    while (mm) {
-        const int g = __ffsll((long long)mm) - 1;
-        mm &= mm - 1;
-        base |= (src & 1ull) << g;
-        src >>= 1;
-    }
+// Sums each value's chunks, one warp a value.
+__device__ __forceinline__ double chunk_sum(const double *partial, long long x, int nch) {
     double p = 0.0;
-    for (long long c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        unsigned long long idx = base, cv = (unsigned long long)c, cm = comp;
-        while (cm) {
-            const int g = __ffsll((long long)cm) - 1;
-            cm &= cm - 1;
-            idx |= (cv & 1ull) << g;
-            cv >>= 1;
-        }
-        const typename V2<Real>::T v = s[idx];
-        p += (double)v.x * v.x + (double)v.y * v.y;
-    }
-    p = warp_sum(p);
-    __shared__ double sh[RED_THREADS / 32];
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = p;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int k = 0; k < RED_THREADS / 32; k++) t += sh[k];
-        partial[blockIdx.x] = t;
-    }
+    for (int k = threadIdx.x & 31; k < nch; k += 32) p += partial[x * nch + k];
+    return warp_sum(p);
 }
 
-__global__ void marginal_chunks_final(const double *partial, long long M, int nch, double *out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double b = -1.0;
-        long long bi = 0;
-        for (long long x = 0; x < M; x++) {
-            double p = 0.0;
-            for (int k = 0; k < nch; k++) p += partial[x * nch + k];
-            if (p > b) {  // lowest value on ties
-                b = p;
-                bi = x;
-            }
-        }
+__global__ void __launch_bounds__(RED_THREADS) marginal_chunks_final(const double *partial, long long M, int nch,
+                                                                      double *out) {
+    double b = -1.0;
+    long long bi = 0;
+    for (long long x = threadIdx.x >> 5; x < M; x += MARG_WARPS) keep_best(b, bi, chunk_sum(partial, x, nch), x);
+    block_best(b, bi);
+    if (threadIdx.x == 0) {
         out[0] = b;
         out[1] = (double)bi;
     }
+}
+
+__global__ void __launch_bounds__(RED_THREADS) marginal_chunks_sum(const double *partial, long long M, int nch,
+                                                                    double *out) {
+    for (long long x = (long long)blockIdx.x * MARG_WARPS + (threadIdx.x >> 5); x < M;
+         x += (long long)gridDim.x * MARG_WARPS) {
+        const double p = chunk_sum(partial, x, nch);
+        if ((threadIdx.x & 31) == 0) out[x] = p;
+    }
+}
+
+// Chunks a unit is split into: until there are blocks for every SM, while the
+// partial sums (M * nch) stay within `cap` and a chunk keeps four runs.
+static int marginal_chunks(int n, uint64_t mask, long long cap, long long *units) {
+    const int lb = n < MARG_LOW ? n : MARG_LOW;
+    const long long M = 1ll << __builtin_popcountll(mask), U = 1ll << __builtin_popcountll(mask >> lb);
+    const long long C = (1ll << (n - lb)) / U;
+    int nch = 1;
+    while (U * nch < RED_BLOCKS && C / nch >= 8 && 2 * M * nch <= cap) nch *= 2;
+    *units = U * nch;
+    return nch;
 }
 
 // Queues the marginal argmax of `mask` over state s: its probability and
-// value land in out[0], out[1].  Scratch: pbest / ibest of RED_BLOCKS entries.
+// value land in out[0], out[1].  Scratch: pbest of 2 * RED_BLOCKS entries,
+// ibest of RED_BLOCKS.
 static int queue_marginal(State *s, uint64_t mask, double *pbest, long long *ibest, double *out, cudaStream_t st) {
     const int n = s->qubits;
     if (n < 64 && (mask >> n)) return fail(HGM_ERR_INVALID, "mask beyond state bits");
-    const int m = __builtin_popcountll(mask);
-    const long long M = 1ll << m;
-    if (M <= RED_BLOCKS) {
-        const int nch = (int)(RED_BLOCKS / M);
-        const unsigned g = (unsigned)(M * nch);
+    const long long N = 1ll << n, M = 1ll << __builtin_popcountll(mask);
+    if (M == N) {
+        const unsigned g = grid_for(N);
         if (s->precision == HGM_F64)
-            marginal_chunk_kernel<double><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, nch, pbest);
+            argmax_all_kernel<double><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, N, pbest, ibest);
         else
-            marginal_chunk_kernel<float><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, nch, pbest);
-        marginal_chunks_final<<<1, 32, 0, st>>>(pbest, M, nch, out);
+            argmax_all_kernel<float><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, N, pbest, ibest);
+        marginal_final<<<1, RED_THREADS, 0, st>>>(pbest, ibest, (int)g, out);
     } else {
-        unsigned g = (unsigned)((M + RED_THREADS - 1) / RED_THREADS);
-        if (g > RED_BLOCKS) g = RED_BLOCKS;
-        if (s->precision == HGM_F64)
-            marginal_kernel<double><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, m, pbest, ibest);
-        else
-            marginal_kernel<float><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, m, pbest, ibest);
-        marginal_final<<<1, 32, 0, st>>>(pbest, ibest, (int)g, out);
+        long long units = 0;
+        const int nch = marginal_chunks(n, mask, 2 * RED_BLOCKS, &units);
+        const unsigned g = (unsigned)(units < RED_BLOCKS ? units : RED_BLOCKS);
+        if (nch > 1) {
+            if (s->precision == HGM_F64)
+                marginal_kernel<double, false><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, nch, pbest, nullptr, nullptr);
+            else
+                marginal_kernel<float, false><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, nch, pbest, nullptr, nullptr);
+            marginal_chunks_final<<<1, RED_THREADS, 0, st>>>(pbest, M, nch, out);
+        } else {
+            if (s->precision == HGM_F64)
+                marginal_kernel<double, true><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, 1, nullptr, pbest, ibest);
+            else
+                marginal_kernel<float, true><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, 1, nullptr, pbest, ibest);
+            marginal_final<<<1, RED_THREADS, 0, st>>>(pbest, ibest, (int)g, out);
+        }
     }
     count_launch(2);
     return check("argmax launch");
-}
-
-// The whole marginal distribution over the bits of `mask` (DGM::measure(vector),
-// src/core/dgm_core.cpp:150-162): out[x] = sum over the other bits of |a|^2,
-// for every value x of the mask bits (bit j of x is the j-th lowest mask bit).
-__global__ void marginal_chunks_sum(const double *partial, long long M, int nch, double *out) {
-    for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < M; x += (long long)gridDim.x * blockDim.x) {
-        double p = 0.0;
-        for (int k = 0; k < nch; k++) p += partial[x * nch + k];
-        out[x] = p;
-    }
-}
-
-template <typename Real>
-__global__ void __launch_bounds__(RED_THREADS) marginal_values_kernel(const typename V2<Real>::T *__restrict__ s, int n,
-                                                                       unsigned long long mask, int m, double *out) {
-    const unsigned long long comp = ~mask & ((n >= 64) ? ~0ull : ((1ull << n) - 1));
-    const long long M = 1ll << m, C = 1ll << (n - m);
-    for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < M; x += (long long)gridDim.x * blockDim.x) {
-        unsigned long long base = 0, src = (unsigned long long)x, mm = mask;
-        while (mm) {
-            const int g = __ffsll((long long)mm) - 1;
-            mm &= mm - 1;
-            base |= (src & 1ull) << g;
-            src >>= 1;
-        }
-        double p = 0.0;
-        for (long long c = 0; c < C; c++) {
-            unsigned long long idx = base, cs = (unsigned long long)c, cm = comp;
-            while (cm) {
-                const int g = __ffsll((long long)cm) - 1;
-                cm &= cm - 1;
-                idx |= (cs & 1ull) << g;
-                cs >>= 1;
-            }
-            const typename V2<Real>::T v = s[idx];
-            p += (double)v.x * v.x + (double)v.y * v.y;
-        }
-        out[x] = p;
-    }
 }
 
 int marginal_probs(State *s, uint64_t mask, double *host_out, void *stream) {
@@ -958,33 +1062,41 @@ int marginal_probs(State *s, uint64_t mask, double *host_out, void *stream) {
     const int m = __builtin_popcountll(mask);
     if (m > 26) return fail(HGM_ERR_UNSUPPORTED, "marginal over %d bits (at most 26)", m);
     const long long M = 1ll << m;
-    double *d_out = nullptr;
-    cudaError_t e = cudaMallocAsync(&d_out, (size_t)M * sizeof(double), st);
-    if (e != cudaSuccess) return fail(HGM_ERR_NOMEM, "marginal output: %s", cudaGetErrorString(e));
-    if (M <= RED_BLOCKS) {
-        const int nch = (int)(RED_BLOCKS / M);
-        const unsigned g = (unsigned)(M * nch);
-        if (s->precision == HGM_F64)
-            marginal_chunk_kernel<double><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, nch, g_ctx.partials);
-        else
-            marginal_chunk_kernel<float><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, nch, g_ctx.partials);
-        marginal_chunks_sum<<<(unsigned)((M + 255) / 256), 256, 0, st>>>(g_ctx.partials, M, nch, d_out);
-    } else {
-        unsigned g = (unsigned)((M + RED_THREADS - 1) / RED_THREADS);
-        if (g > RED_BLOCKS) g = RED_BLOCKS;
-        if (s->precision == HGM_F64)
-            marginal_values_kernel<double><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, m, d_out);
-        else
-            marginal_values_kernel<float><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, m, d_out);
+    long long units = 0;
+    const int nch = marginal_chunks(n, mask, 1 << 16, &units);
+    const unsigned g = (unsigned)(units < (1 << 16) ? units : (1 << 16));
+    // values, then the chunks' partial sums: from the context's scratch when
+    // they fit (freeing a stream-ordered allocation at every call's
+    // synchronisation returns its pages to the driver)
+    const size_t need = (size_t)(M + (nch > 1 ? M * nch : 0)) * sizeof(double);
+    std::lock_guard<std::mutex> lk(g_reduce_mu);
+    double *d_out = g_ctx.marginal;
+    cudaError_t e = cudaSuccess;
+    if (need > MARGINAL_SCRATCH) {
+        e = cudaMallocAsync(&d_out, need, st);
+        if (e != cudaSuccess) return fail(HGM_ERR_NOMEM, "marginal output: %s", cudaGetErrorString(e));
     }
-    count_launch(2);
+    double *sums = nch > 1 ? d_out + M : d_out;
+    if (s->precision == HGM_F64)
+        marginal_kernel<double, false><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, nch,
+                                                                        sums, nullptr, nullptr);
+    else
+        marginal_kernel<float, false><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, nch,
+                                                                       sums, nullptr, nullptr);
+    count_launch();
+    if (nch > 1) {
+        const long long blocks = (M + MARG_WARPS - 1) / MARG_WARPS;
+        marginal_chunks_sum<<<(unsigned)(blocks < RED_BLOCKS ? blocks : RED_BLOCKS), RED_THREADS, 0, st>>>(sums, M, nch,
+                                                                                                          d_out);
+        count_launch();
+    }
     int rc = check("marginal probabilities launch");
     if (!rc) {
         e = cudaMemcpyAsync(host_out, d_out, (size_t)M * sizeof(double), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) rc = fail(HGM_ERR_CUDA, "marginal probabilities: %s", cudaGetErrorString(e));
     }
-    cudaFreeAsync(d_out, st);
+    if (need > MARGINAL_SCRATCH) cudaFreeAsync(d_out, st);
     return rc;
 }
 
@@ -995,9 +1107,9 @@ int launch_argmax_async(State *s, uint64_t mask, double *pbest, long long *ibest
 int marginal_argmax(State *s, uint64_t mask, int64_t *arg, double *prob, void *stream) {
     cudaStream_t st = pick(stream);
     if (!st) return HGM_ERR_CUDA;
-    const int rc = queue_marginal(s, mask, g_ctx.partials, g_ctx.partial_idx, g_ctx.result, st);
+    std::lock_guard<std::mutex> lk(g_reduce_mu);
+    const int rc = queue_marginal(s, mask, g_ctx.partials, g_ctx.partial_idx, g_ctx.host_result, st);
     if (rc) return rc;
-    cudaMemcpyAsync(g_ctx.host_result, g_ctx.result, 2 * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(HGM_ERR_CUDA, "marginal argmax: %s", cudaGetErrorString(e));
     if (prob) *prob = g_ctx.host_result[0];
@@ -1038,16 +1150,6 @@ int marginal_argmax(State *s, uint64_t mask, int64_t *arg, double *prob, void *s
 //     call before any stream capture.
 constexpr int NOALLOC_PARTIALS = 2 * RED_BLOCKS;
 static __device__ __align__(256) double g_noalloc_partials[NOALLOC_PARTIALS];
-
-// Final step of the allocation-free norm: sums the block partials in the same
-// fixed order as reduce_final and writes the one result double.
-__global__ void noalloc_norm_final(const double *partials, int nblocks, double *out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double t0 = 0.0;
-        for (int k = 0; k < nblocks; k++) t0 += partials[2 * k];
-        out[0] = t0;
-    }
-}
 
 namespace {
 std::mutex g_noalloc_mu;
@@ -1091,7 +1193,7 @@ extern "C" int hgm_norm_noalloc(const void *d_state, int qubits, int precision, 
     else
         reduce_kernel<float, float, RED_NORM><<<g, RED_THREADS, 0, st>>>((const float2 *)d_state, nullptr, N, 0,
                                                                           partials);
-    noalloc_norm_final<<<1, 32, 0, st>>>(partials, (int)g, d_out);
+    reduce_final<RED_NORM><<<1, RED_THREADS, 0, st>>>(partials, (int)g, d_out, 1);  // one double, nothing after it
     count_launch(2);
     return check("hgm_norm_noalloc launch");
 }
