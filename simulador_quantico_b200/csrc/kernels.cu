@@ -504,6 +504,11 @@ int upload_plan(Plan *p) {
         if ((e = cudaMemcpy(p->d_chain_passes, dev.data(), pb, cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(HGM_ERR_CUDA, "plan chain passes copy: %s", cudaGetErrorString(e));
     }
+    // a copy from pageable memory may return before its last piece has
+    // reached the device, and the plan's launches go to non-blocking streams,
+    // which do not wait for it
+    if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess)
+        return fail(HGM_ERR_CUDA, "plan upload: %s", cudaGetErrorString(e));
     return HGM_OK;
 }
 
