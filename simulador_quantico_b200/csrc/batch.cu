@@ -27,7 +27,7 @@
 namespace hgm {
 
 struct BatchTask {
-    PassArgs pa;            // pass arguments (tiled tasks)
+    TileArgs pa;            // pass arguments (tiled tasks)
     void *state;            // the circuit's state in the batch arena
     long long tile_begin;   // first global item of this task
     int32_t ntiles;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
     __shared__ int s_skip;
     // the item's pass arguments, copied once per item into shared memory (the
     // tile code reads them many times; chained kernel, kernels.cu)
-    __shared__ __align__(16) PassArgs s_pa;
+    __shared__ __align__(16) TileArgs s_ta;
     for (;;) {
         if (threadIdx.x == 0) {
             const long long it = (long long)atomicAdd(next_item, 1ull);
@@ -138,10 +138,12 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
                                  reinterpret_cast<const SmallOp<Real> *>(t.small_ops), t.n_small_ops, sm);
             } else {
                 const uint32_t *src = reinterpret_cast<const uint32_t *>(&t.pa);
-                uint32_t *dst = reinterpret_cast<uint32_t *>(&s_pa);
-                for (int w = threadIdx.x; w < (int)(sizeof(PassArgs) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
+                uint32_t *dst = reinterpret_cast<uint32_t *>(&s_ta);
+                for (int w = threadIdx.x; w < (int)(sizeof(TileArgs) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
                 __syncthreads();
-                run_tile<Real, R, W>(reinterpret_cast<A2 *>(t.state), s_pa, (uint64_t)(it - t.tile_begin), sm);
+                fetch_stream(smem_raw + tile_smem_bytes<Real, R, W>(), s_ta);
+                run_tile<Real, R, W, false>(reinterpret_cast<A2 *>(t.state), s_ta, (uint64_t)(it - t.tile_begin),
+                                            smem_raw, 0, nullptr, nullptr);
             }
         }
         __syncthreads();
@@ -225,7 +227,7 @@ namespace {
 
 template <typename Real, int R, int W>
 int batch_setup(Batch *b) {
-    const int smem = tile_smem_elems<R, W>() * (int)sizeof(typename V2<Real>::T);
+    const int smem = cta_smem_bytes<Real, R, W>();
     cudaError_t e = cudaFuncSetAttribute(batch_kernel<Real, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(HGM_ERR_CUDA, "batch kernel attribute: %s", cudaGetErrorString(e));
     int per_sm = 0, dev = 0, sms = 0;
@@ -311,8 +313,7 @@ int batch_finalize(Batch *b) {
                 }
             } else {
                 if (wave >= j.plan->passes.size()) continue;
-                t.pa = j.plan->passes[wave];
-                t.pa.flags = 0;
+                t.pa = j.plan->tiles[wave];
                 t.ntiles = 1 << (j.n - t.pa.k);
             }
             t.dep_need = t.dep >= 0 ? (uint32_t)b->tasks[t.dep].ntiles : 0u;
@@ -340,6 +341,8 @@ int batch_finalize(Batch *b) {
         (rc = cuda_err(cudaMemcpy(b->d_offsets, offs.data(), offs.size() * 8, cudaMemcpyHostToDevice), "offsets")) ||
         (rc = cuda_err(cudaMemcpy(b->d_init, inits.data(), inits.size() * 8, cudaMemcpyHostToDevice), "inits")))
         return rc;
+    // the graph runs on streams that do not wait for these copies' tails
+    if ((rc = cuda_err(cudaStreamSynchronize(cudaStreamLegacy), "batch upload"))) return rc;
     rc = b->precision == HGM_F64 ? batch_dispatch<double>(b, true, nullptr) : batch_dispatch<float>(b, true, nullptr);
     if (rc) return rc;
     // capture: reset counters and states, run the persistent kernel

@@ -41,7 +41,7 @@ std::mutex g_lease_mu;
 
 void free_plan_now(Plan *pl) {
     // launches are asynchronous: the plan's device records may still be in use
-    if (pl->d_ops || pl->d_phases) cudaDeviceSynchronize();
+    if (pl->d_ops || pl->d_norm) cudaDeviceSynchronize();
     delete pl;
 }
 }  // namespace
@@ -193,6 +193,15 @@ int hgm_plan_export(const hgm_plan *p, const void **passes, int64_t *n_passes, c
     if (ops_bytes) *ops_bytes = (int64_t)pl->ops_bytes.size();
     if (warp_bits) *warp_bits = pl->warp_bits;
     if (small) *small = pl->small ? 1 : 0;
+    return HGM_OK;
+}
+
+int hgm_plan_stream(const hgm_plan *p, const void **units, int64_t *bytes) {
+    if (!p) return fail(HGM_ERR_INVALID, "null plan");
+    const Plan *pl = reinterpret_cast<const Plan *>(p);
+    const bool small = pl->small;
+    if (units) *units = small ? (const void *)pl->ops_bytes.data() : (const void *)pl->stream.data();
+    if (bytes) *bytes = small ? (int64_t)pl->ops_bytes.size() : (int64_t)(pl->stream.size() * sizeof(uint32_t));
     return HGM_OK;
 }
 

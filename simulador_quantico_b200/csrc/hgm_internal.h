@@ -230,6 +230,61 @@ struct PassArgs {
 constexpr int32_t PASS_NORM = 1;
 constexpr int32_t PASS_SCALE = 2;
 
+// ---- device stream -----------------------------------------------------------
+// What the kernels run.  Each pass's phases and op records (the plan above)
+// are lowered (lower.cpp) to one stream of 16-byte units: every op is a
+// header unit (word 0: kind in bits 0..7, units of the op in bits 8..) and
+// its data, transposes among them.  A pass's stream is cut into windows of at
+// most STREAM_WINDOW_UNITS, which a CTA copies into shared memory, one window
+// ahead of the one it runs: an op read from global memory cost an L2 round
+// trip each in states of one or a few tiles, where no other warp hides it
+// (12 qubits, 20 layers, one tile: 199 -> 109 us), and in large states the
+// addresses and the waits of those loads (26 qubits, 20 layers, FP32: 16.4 ->
+// 13.3 ms, same arithmetic; the kernels' spills went with them).
+// Two windows of 176 units leave four CTAs an SM within the 164 KB carveout.
+constexpr int STREAM_WINDOW_UNITS = 176;
+enum StreamKind : uint32_t {
+    S_END = 0,    // store the tile
+    S_NEXT = 1,   // go on in the next window; w1: units of the window after it (0: none)
+    S_TRANS = 2,  // transpose; w1: STREAM_SYNC_*; w2, w3: byte steps of register bit 4 in
+                  // the old and the new layout; then old steps 0..3, new steps 0..3, and the
+                  // new layout's byte steps of thread bits 0..3 and 4..7
+    S_ROT = 3,    // FP64: rotations with a phase, on the register bits of w1 (bits 0..7), then X on
+                  // those of w1 bits 8..15; (t, u, p re, p im) per bit (lower.cpp make_rot)
+    S_HAD = 4,    // FP64: sqrt(2) H on the register bits of w1
+    S_REAL = 5,   // real 2x2s on the register bits of w1: m00, m01, m10, m11 per bit
+    S_DENSE = 6,  // complex 2x2s on the register bits of w1: 8 values per bit
+    S_XSET = 7,   // w1 relabeling X gates (K_XSET entries), the first two in w2, w3
+    S_CSWAP = 8,  // X on register bit w1 where (label & w2) == w3
+    S_SCALE = 9,  // FP64: every amplitude times the factor in w2, w3
+    S_PHASES = 10,  // phase block of compact terms; w1: K_PHASE_BLOCK flags (cm_reg), w2: active
+                    // categories (cv_reg), w3: units from the head to the table (0: none); then
+                    // the 16 counts, the thread bits' index bits, the terms and the table
+    S_TERMS = 11,   // phase block of product terms, same head
+    S_GATE = 12,    // any other record; w1: kind | tpos << 8, w2, w3: cm_reg, cv_reg; then thread
+                    // controls, non-tile controls and (not for K_SWAP) the matrix
+    S_SPLIT = 13,   // FP32: a phase, then a real 2x2, on the register bits of w1; m00, m01, m10,
+                    // m11, p re, p im, 0, 0 per bit (K_LAYER_SPLIT)
+};
+constexpr uint32_t STREAM_SYNC_BEFORE = 1, STREAM_SYNC_CROSS = 2;
+
+// A pass as the kernels take it.
+struct TileArgs {
+    const void *stream;     // first window, then the others back to back
+    int32_t units0, units1; // units of the first two windows
+    int32_t n, k;
+    int32_t flags;          // PASS_*
+    int32_t nruns;
+    double *norm_out;
+    const double *scale_in;
+    int8_t run_pos[MAX_FREE_RUNS];
+    int8_t run_len[MAX_FREE_RUNS];
+    int8_t ld_gbit[MAX_LAYOUT_ROLES];
+    int8_t st_gbit[MAX_LAYOUT_ROLES];
+    uint32_t ld_tstep[8];   // load layout: byte step of each thread bit in the transpose buffer
+};
+static_assert(sizeof(TileArgs) % 4 == 0, "copied as words");
+
 // Small-state path (n < 5 + R): whole state in one CTA's shared memory, ops
 // applied one at a time.
 template <typename Real>
@@ -259,13 +314,14 @@ struct Plan {
     std::vector<DevPhase> phases;
     std::vector<Lay> layouts;         // every layout the phases use
     std::vector<unsigned char> ops_bytes;   // DevOp<Real>[] or SmallOp<Real>[]
+    // The passes as the kernels run them (lower.cpp).
+    std::vector<uint32_t> stream;     // units, four words each
+    std::vector<TileArgs> tiles;      // stream holds the offset until upload_plan patches it
     int64_t n_small_ops = 0;
     int64_t n_ops = 0, n_transposes = 0;
     // device copies, and their sizes as allocated
     DevAllocator *allocator = nullptr;
-    size_t d_bytes[6] = {0, 0, 0, 0, 0, 0};  // ops, phases, layouts, norm, chain scratch, chain passes
-    void *d_phases = nullptr;
-    void *d_layouts = nullptr;
+    size_t d_bytes[4] = {0, 0, 0, 0};  // stream (or small ops), norm, chain scratch, chain passes
     void *d_ops = nullptr;
     int renorm_every = 0;
     double *d_norm = nullptr;         // renormalisation scratch (FP32 plans)
@@ -302,6 +358,9 @@ int copy_state(void *dst, const void *src, size_t bytes, bool to_device, void *s
 int build_plan(const std::vector<Op> &ops, int qubits, const hgm_plan_opts &opts, Plan *plan,
                bool force_small = false);
 int upload_plan(Plan *plan);
+// Lowers a tiled plan's passes to the device stream (lower.cpp).  global: the
+// scalar the plan's last record applies (1: there is no such record).
+void lower_plan(Plan *plan, cplx global);
 void plan_lease(const Plan *plan);
 void plan_unlease(const Plan *plan);
 

@@ -87,9 +87,10 @@ static inline int check(const char *what) {
 
 template <typename Real, int R, int W, bool LEAN>
 __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()))
-    pass_kernel(typename V2<Real>::T *__restrict__ state, const PassArgs pa) {
+    pass_kernel(typename V2<Real>::T *__restrict__ state, const __grid_constant__ TileArgs ta) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    run_tile<Real, R, W, LEAN>(state, pa, blockIdx.x, reinterpret_cast<typename V2<Real>::T *>(smem_raw));
+    fetch_stream(smem_raw + tile_smem_bytes<Real, R, W>(), ta);
+    run_tile<Real, R, W, LEAN>(state, ta, blockIdx.x, smem_raw, ta.flags, ta.norm_out, ta.scale_in);
 }
 
 template <typename Real>
@@ -132,7 +133,7 @@ template <typename Real, int R, int W, bool LEAN>
 static int setup_pass_kernel() {
     static bool done = false;
     if (done) return HGM_OK;
-    const int smem = tile_smem_elems<R, W>() * (int)sizeof(typename V2<Real>::T);
+    const int smem = cta_smem_bytes<Real, R, W>();
     cudaError_t e =
         cudaFuncSetAttribute(pass_kernel<Real, R, W, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess && HGM_SMEM_CARVEOUT >= 0)
@@ -144,12 +145,12 @@ static int setup_pass_kernel() {
 }
 
 template <typename Real, int R, int W, bool LEAN>
-static int launch_pass(void *state, const PassArgs &pa, cudaStream_t st) {
+static int launch_pass(void *state, const TileArgs &pa, cudaStream_t st) {
     using A2 = typename V2<Real>::T;
     int rc = setup_pass_kernel<Real, R, W, LEAN>();
     if (rc) return rc;
     const uint64_t tiles = 1ull << (pa.n - pa.k);
-    const int smem = tile_smem_elems<R, W>() * (int)sizeof(A2);
+    const int smem = cta_smem_bytes<Real, R, W>();
     pass_kernel<Real, R, W, LEAN><<<(unsigned)tiles, 32 << W, smem, st>>>(reinterpret_cast<A2 *>(state), pa);
     count_launch();
     return HGM_OK;
@@ -158,7 +159,7 @@ static int launch_pass(void *state, const PassArgs &pa, cudaStream_t st) {
 // FP64 tiles hold 16 amplitudes a thread (R = 4), FP32 tiles 32 (R = 5) or,
 // on request, 16 (plan_reg_bits).
 template <typename Real, int R, bool LEAN>
-static int launch_pass_w(int W, void *state, const PassArgs &pa, cudaStream_t st) {
+static int launch_pass_w(int W, void *state, const TileArgs &pa, cudaStream_t st) {
     switch (W) {
         case 0: return launch_pass<Real, R, 0, LEAN>(state, pa, st);
         case 1: return launch_pass<Real, R, 1, LEAN>(state, pa, st);
@@ -167,7 +168,7 @@ static int launch_pass_w(int W, void *state, const PassArgs &pa, cudaStream_t st
     }
 }
 template <typename Real, int R>
-static int launch_pass_lw(bool lean, int W, void *state, const PassArgs &pa, cudaStream_t st) {
+static int launch_pass_lw(bool lean, int W, void *state, const TileArgs &pa, cudaStream_t st) {
     return lean ? launch_pass_w<Real, R, true>(W, state, pa, st) : launch_pass_w<Real, R, false>(W, state, pa, st);
 }
 
@@ -186,9 +187,7 @@ int launch_plan_steps(State *s, const Plan *p, int iterations, PlanCursor *c, in
     if (s->precision != p->precision) return fail(HGM_ERR_INVALID, "plan and state precision differ");
     // every device pointer a launch passes must exist: an op list that was
     // never uploaded is refused here, not read through a null pointer
-    if ((!p->ops_bytes.empty() && !p->d_ops) || (!p->phases.empty() && !p->d_phases) ||
-        (!p->layouts.empty() && !p->d_layouts) ||
-        (p->renorm_every > 0 && !p->small && !p->d_norm))
+    if (((!p->ops_bytes.empty() || !p->stream.empty()) && !p->d_ops) || (p->renorm_every > 0 && !p->small && !p->d_norm))
         return fail(HGM_ERR_INVALID, "plan used before upload_plan");
     cudaStream_t st = pick(stream);
     if (!st) return HGM_ERR_CUDA;
@@ -204,8 +203,7 @@ int launch_plan_steps(State *s, const Plan *p, int iterations, PlanCursor *c, in
     const int64_t total = np * iterations;
     for (int64_t k = 0; k < max_launches && c->next < total; k++, c->next++) {
         const int64_t g = c->next;
-        PassArgs pa = p->passes[g % np];
-        pa.flags = 0;
+        TileArgs pa = p->tiles[g % np];
         if (c->scale_next) {
             pa.flags |= PASS_SCALE;
             pa.scale_in = p->d_norm + c->scale_slot;
@@ -272,18 +270,15 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 
 template <typename Real, int R, int W, bool LEAN>
 __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()))
-    chain_kernel(typename V2<Real>::T *__restrict__ state, const PassArgs *__restrict__ passes, int npasses,
+    chain_kernel(typename V2<Real>::T *__restrict__ state, const TileArgs *__restrict__ passes, int npasses,
                  int tile_bits, long long total, int renorm, unsigned long long *ctr, double *norms) {
-    using A2 = typename V2<Real>::T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    A2 *sm = reinterpret_cast<A2 *>(smem_raw);
     __shared__ long long s_item;
     __shared__ int s_skip;
     // the item's pass arguments, copied once per item: the tile code reads
     // them many times (the tile-bit map byte by byte), from shared memory
     // rather than through L1
-    __shared__ __align__(16) PassArgs s_pa;
-    static_assert(sizeof(PassArgs) % 4 == 0, "PassArgs copies as words");
+    __shared__ __align__(16) TileArgs s_ta;
     const long long seq = total >> tile_bits;  // passes in the sequence
     for (;;) {
         if (threadIdx.x == 0) {
@@ -325,11 +320,12 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
             }
             {
                 const uint32_t *src = reinterpret_cast<const uint32_t *>(passes + g % npasses);
-                uint32_t *dst = reinterpret_cast<uint32_t *>(&s_pa);
-                for (int w = threadIdx.x; w < (int)(sizeof(PassArgs) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
+                uint32_t *dst = reinterpret_cast<uint32_t *>(&s_ta);
+                for (int w = threadIdx.x; w < (int)(sizeof(TileArgs) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
             }
             __syncthreads();
-            run_tile<Real, R, W, LEAN>(state, s_pa, (uint64_t)(it & ((1ll << tile_bits) - 1)), sm, flags, norm_out,
+            fetch_stream(smem_raw + tile_smem_bytes<Real, R, W>(), s_ta);
+            run_tile<Real, R, W, LEAN>(state, s_ta, (uint64_t)(it & ((1ll << tile_bits) - 1)), smem_raw, flags, norm_out,
                                        scale_in);
         }
         __syncthreads();
@@ -348,7 +344,7 @@ template <typename Real, int R, int W, bool LEAN>
 static int launch_chain_rw(State *s, const Plan *p, int iterations, cudaStream_t st) {
     using A2 = typename V2<Real>::T;
     static int grid_cap = 0;
-    const int smem = tile_smem_elems<R, W>() * (int)sizeof(A2);
+    const int smem = cta_smem_bytes<Real, R, W>();
     if (!grid_cap) {
         cudaError_t e = cudaFuncSetAttribute(chain_kernel<Real, R, W, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int per_sm = 0, dev = 0, sms = 0;
@@ -364,10 +360,10 @@ static int launch_chain_rw(State *s, const Plan *p, int iterations, cudaStream_t
     const unsigned grid = (unsigned)(ntiles < grid_cap ? ntiles : grid_cap);
     unsigned long long *ctr = reinterpret_cast<unsigned long long *>(p->d_chain);
     double *norms = reinterpret_cast<double *>(ctr + 4);
-    cudaError_t e = cudaMemsetAsync(p->d_chain, 0, p->d_bytes[4], st);
+    cudaError_t e = cudaMemsetAsync(p->d_chain, 0, p->d_bytes[2], st);
     if (e != cudaSuccess) return fail(HGM_ERR_CUDA, "chain scratch reset: %s", cudaGetErrorString(e));
     chain_kernel<Real, R, W, LEAN><<<grid, 32 << W, smem, st>>>(reinterpret_cast<A2 *>(s->d),
-                                                          reinterpret_cast<const PassArgs *>(p->d_chain_passes),
+                                                          reinterpret_cast<const TileArgs *>(p->d_chain_passes),
                                                           (int)p->passes.size(), tile_bits, total, p->renorm_every,
                                                           ctr, norms);
     count_launch();
@@ -428,8 +424,8 @@ static cudaError_t plan_alloc(Plan *p, int k, void **out, size_t bytes) {
 }
 
 Plan::~Plan() {
-    void *ptrs[6] = {d_ops, d_phases, d_layouts, d_norm, d_chain, d_chain_passes};
-    for (int k = 0; k < 6; k++) {
+    void *ptrs[4] = {d_ops, d_norm, d_chain, d_chain_passes};
+    for (int k = 0; k < 4; k++) {
         if (!ptrs[k]) continue;
         if (allocator) allocator->free(ptrs[k], d_bytes[k]);
         else cudaFree(ptrs[k]);
@@ -437,71 +433,33 @@ Plan::~Plan() {
 }
 
 int upload_plan(Plan *p) {
-    if (p->d_ops || (p->ops_bytes.empty() && p->phases.empty() && !p->renorm_every)) return HGM_OK;
+    const void *src = p->small ? (const void *)p->ops_bytes.data() : (const void *)p->stream.data();
+    const size_t bytes = p->small ? p->ops_bytes.size() : p->stream.size() * sizeof(uint32_t);
+    if (p->d_ops || p->d_norm || (!bytes && !p->renorm_every)) return HGM_OK;
     if (ensure_ctx()) return HGM_ERR_CUDA;
     cudaError_t e;
-    if (!p->ops_bytes.empty()) {
-        if ((e = plan_alloc(p, 0, &p->d_ops, p->ops_bytes.size())) != cudaSuccess)
+    if (bytes) {
+        if ((e = plan_alloc(p, 0, &p->d_ops, bytes)) != cudaSuccess)
             return fail(HGM_ERR_NOMEM, "plan ops: %s", cudaGetErrorString(e));
-        if ((e = cudaMemcpy(p->d_ops, p->ops_bytes.data(), p->ops_bytes.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+        if ((e = cudaMemcpy(p->d_ops, src, bytes, cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(HGM_ERR_CUDA, "plan ops copy: %s", cudaGetErrorString(e));
     }
-    if (!p->phases.empty()) {
-        size_t b = p->phases.size() * sizeof(DevPhase);
-        if ((e = plan_alloc(p, 1, &p->d_phases, b)) != cudaSuccess) return fail(HGM_ERR_NOMEM, "plan phases: %s", cudaGetErrorString(e));
-        if ((e = cudaMemcpy(p->d_phases, p->phases.data(), b, cudaMemcpyHostToDevice)) != cudaSuccess)
-            return fail(HGM_ERR_CUDA, "plan phases copy: %s", cudaGetErrorString(e));
-    }
-    if (!p->layouts.empty()) {
-        // per layout: the byte step of each register bit, then each thread's
-        // register-0 offset, in the padded transpose buffer (kernels.cuh)
-        const int R = p->reg_bits, W = p->warp_bits, nt = 32 << W;
-        const uint32_t esz = p->precision == HGM_F64 ? 16 : 8;
-        auto pad = [&](uint32_t j) { return (j + (j >> R)) * esz; };
-        std::vector<uint32_t> tab(p->layouts.size() * (LAYOUT_HDR + nt), 0u);
-        for (size_t l = 0; l < p->layouts.size(); l++) {
-            const Lay &lay = p->layouts[l];
-            uint32_t *e0 = tab.data() + l * (LAYOUT_HDR + nt);
-            for (int q = 0; q < R; q++) e0[q] = pad(1u << lay.pos[5 + W + q]);
-            for (int t = 0; t < nt; t++) {
-                uint32_t o = 0;
-                for (int b = 0; b < 5 + W; b++)
-                    if ((t >> b) & 1) o += pad(1u << lay.pos[b]);
-                e0[LAYOUT_HDR + t] = o;
-            }
-        }
-        const size_t b = tab.size() * sizeof(uint32_t);
-        if ((e = plan_alloc(p, 2, &p->d_layouts, b)) != cudaSuccess)
-            return fail(HGM_ERR_NOMEM, "plan layouts: %s", cudaGetErrorString(e));
-        if ((e = cudaMemcpy(p->d_layouts, tab.data(), b, cudaMemcpyHostToDevice)) != cudaSuccess)
-            return fail(HGM_ERR_CUDA, "plan layouts copy: %s", cudaGetErrorString(e));
-    }
     if (p->renorm_every > 0) {
-        if ((e = plan_alloc(p, 3, (void **)&p->d_norm, 64 * sizeof(double))) != cudaSuccess)
+        if ((e = plan_alloc(p, 1, (void **)&p->d_norm, 64 * sizeof(double))) != cudaSuccess)
             return fail(HGM_ERR_NOMEM, "plan norm slots: %s", cudaGetErrorString(e));
     }
-    for (PassArgs &pa : p->passes) {
-        pa.phases = reinterpret_cast<const DevPhase *>(p->d_phases);
-        pa.layouts = reinterpret_cast<const uint32_t *>(p->d_layouts);
-        pa.ops = p->d_ops;
-    }
+    for (TileArgs &t : p->tiles) t.stream = (const unsigned char *)p->d_ops + reinterpret_cast<size_t>(t.stream);
     const int64_t state_bytes = (int64_t(1) << p->qubits) * (p->precision == HGM_F64 ? 16 : 8);
-    if (p->chained && !p->small && p->passes.size() >= 2 && state_bytes <= CHAIN_MAX_BYTES) {
+    if (p->chained && !p->small && p->tiles.size() >= 2 && state_bytes <= CHAIN_MAX_BYTES) {
         // chained execution: the pass records (pointers patched) and the scratch
         p->chain_slots = p->renorm_every > 0 ? CHAIN_NORM_SLOTS : 0;
         const size_t sb = (4 + (size_t)p->chain_slots) * sizeof(double);
-        const size_t pb = p->passes.size() * sizeof(PassArgs);
-        if ((e = plan_alloc(p, 4, &p->d_chain, sb)) != cudaSuccess)
+        const size_t pb = p->tiles.size() * sizeof(TileArgs);
+        if ((e = plan_alloc(p, 2, &p->d_chain, sb)) != cudaSuccess)
             return fail(HGM_ERR_NOMEM, "plan chain scratch: %s", cudaGetErrorString(e));
-        if ((e = plan_alloc(p, 5, &p->d_chain_passes, pb)) != cudaSuccess)
+        if ((e = plan_alloc(p, 3, &p->d_chain_passes, pb)) != cudaSuccess)
             return fail(HGM_ERR_NOMEM, "plan chain passes: %s", cudaGetErrorString(e));
-        std::vector<PassArgs> dev(p->passes);
-        for (PassArgs &pa : dev) {
-            pa.flags = 0;
-            pa.norm_out = nullptr;
-            pa.scale_in = nullptr;
-        }
-        if ((e = cudaMemcpy(p->d_chain_passes, dev.data(), pb, cudaMemcpyHostToDevice)) != cudaSuccess)
+        if ((e = cudaMemcpy(p->d_chain_passes, p->tiles.data(), pb, cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(HGM_ERR_CUDA, "plan chain passes copy: %s", cudaGetErrorString(e));
     }
     // a copy from pageable memory may return before its last piece has

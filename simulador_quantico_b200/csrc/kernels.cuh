@@ -201,6 +201,22 @@ __device__ __forceinline__ void ip_cmul2(A2 &a, A2 f) {
     ip_cmul(a.x, a.y, f.x, f.y, -f.y);
 }
 
+// y already scaled (lower.cpp make_rot): x <- x + u y, then y <- y + t x.  Two
+// multiply-adds a component, in place: no temporary to copy back, and half of
+// a general real 2x2's four operations.
+__device__ __forceinline__ void ip_rot(double &xr, double &xi, double &yr, double &yi, double u, double t) {
+    asm("fma.rn.f64 %0, %4, %2, %0;\n\tfma.rn.f64 %1, %4, %3, %1;\n\t"
+        "fma.rn.f64 %2, %5, %0, %2;\n\tfma.rn.f64 %3, %5, %1, %3;"
+        : "+d"(xr), "+d"(xi), "+d"(yr), "+d"(yi)
+        : "d"(u), "d"(t));
+}
+// sqrt(2) H: x <- x + y, then y <- x - 2 y.
+__device__ __forceinline__ void ip_had(double &xr, double &xi, double &yr, double &yi) {
+    xr += yr;
+    xi += yi;
+    yr = fma(-2.0, yr, xr);
+    yi = fma(-2.0, yi, xi);
+}
 // ---- gate application on register bits -----------------------------------
 
 template <typename Real, typename A2>
@@ -407,14 +423,14 @@ struct RegTarget<Real, A2, R, R, LEAN> {
                                                uint32_t, uint32_t, bool) {}
 };
 
-template <typename Real>
-__device__ __forceinline__ void load_matrix(const Real *__restrict__ src, Real (&m)[8]);
+// Gate data sits in the stream window in shared memory: 16-byte loads of the
+// same address by every lane.
 template <>
 __device__ __forceinline__ void load_matrix<double>(const double *__restrict__ src, double (&m)[8]) {
     const double2 *p = reinterpret_cast<const double2 *>(src);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const double2 v = __ldg(p + k);
+        const double2 v = p[k];
         m[2 * k] = v.x;
         m[2 * k + 1] = v.y;
     }
@@ -424,7 +440,7 @@ __device__ __forceinline__ void load_matrix<float>(const float *__restrict__ src
     const float4 *p = reinterpret_cast<const float4 *>(src);
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-        const float4 v = __ldg(p + k);
+        const float4 v = p[k];
         m[4 * k] = v.x;
         m[4 * k + 1] = v.y;
         m[4 * k + 2] = v.z;
@@ -447,117 +463,78 @@ __device__ __forceinline__ void load_matrix_flip(const Real *__restrict__ src, R
     }
 }
 
-// A layer: uncontrolled dense gates on a set of register bits (mask),
-// applied bit 0 first, one straight-line block per active bit (a uniform
-// branch skips inactive bits).  Its matrices follow in popcount(mask) records.
-template <typename Real, typename A2, int R, int T, bool REAL>
-struct LayerStep {
-    __device__ __forceinline__ static void run(A2 (&a)[1 << R], const DevOp<Real> *__restrict__ mats, uint32_t mask,
-                                               uint32_t xr) {
+// A layer: uncontrolled gates on a set of register bits (mask), lowest bit
+// first, one straight-line block per active bit (a uniform branch skips
+// inactive bits); the gates' data follow the header in the stream.
+
+// Complex 2x2s (S_DENSE) and real ones (S_REAL).
+template <typename Real, typename A2, int R, int T>
+struct DenseStep {
+    __device__ __forceinline__ static void run(A2 (&a)[1 << R], const Real *__restrict__ d, uint32_t mask, uint32_t xr) {
         if (mask & (1u << T)) {
             Real m[8];
-            load_matrix_flip<Real>(mats->m, m, (xr >> T) & 1u);
-            if (REAL) reg_real<Real, A2, R, T, false>(a, m, 0u, 0u);
-            else reg_dense<Real, A2, R, T, false>(a, m, 0u, 0u);
-            mats++;
+            load_matrix_flip<Real>(d, m, (xr >> T) & 1u);
+            reg_dense<Real, A2, R, T, false>(a, m, 0u, 0u);
+            d += 8;
         }
-        LayerStep<Real, A2, R, T + 1, REAL>::run(a, mats, mask, xr);
+        DenseStep<Real, A2, R, T + 1>::run(a, d, mask, xr);
     }
 };
-template <typename Real, typename A2, int R, bool REAL>
-struct LayerStep<Real, A2, R, R, REAL> {
-    __device__ __forceinline__ static void run(A2 (&)[1 << R], const DevOp<Real> *__restrict__, uint32_t,
-                                               uint32_t) {}
+template <typename Real, typename A2, int R>
+struct DenseStep<Real, A2, R, R> {
+    __device__ __forceinline__ static void run(A2 (&)[1 << R], const Real *__restrict__, uint32_t, uint32_t) {}
 };
 
-// A layer gate's matrix as loaded: the four complex entries (dense) or their
-// real parts (REAL); `get` writes the m[8] form, bit-swapped with `flip`.
-template <typename Real, bool REAL>
-struct LayerRec;
-template <>
-struct LayerRec<float, false> {
-    float4 a, b;
-    __device__ __forceinline__ void load(const DevOp<float> *__restrict__ d) {
-        a = __ldg(reinterpret_cast<const float4 *>(d->m));
-        b = __ldg(reinterpret_cast<const float4 *>(d->m) + 1);
-    }
-    __device__ __forceinline__ void get(bool f, float (&m)[8]) const {
-        m[0] = f ? b.z : a.x; m[1] = f ? b.w : a.y; m[2] = f ? b.x : a.z; m[3] = f ? b.y : a.w;
-        m[4] = f ? a.z : b.x; m[5] = f ? a.w : b.y; m[6] = f ? a.x : b.z; m[7] = f ? a.y : b.w;
-    }
-};
-template <>
-struct LayerRec<float, true> {
-    float r0, r1, r2, r3;
-    __device__ __forceinline__ void load(const DevOp<float> *__restrict__ d) {
-        const float4 a = __ldg(reinterpret_cast<const float4 *>(d->m));
-        const float4 b = __ldg(reinterpret_cast<const float4 *>(d->m) + 1);
-        r0 = a.x; r1 = a.z; r2 = b.x; r3 = b.z;
-    }
-    __device__ __forceinline__ void get(bool f, float (&m)[8]) const {
-        m[0] = f ? r3 : r0; m[2] = f ? r2 : r1; m[4] = f ? r1 : r2; m[6] = f ? r0 : r3;
-        m[1] = m[3] = m[5] = m[7] = 0.0f;
-    }
-};
-template <>
-struct LayerRec<double, false> {
-    double2 e0, e1, e2, e3;
-    __device__ __forceinline__ void load(const DevOp<double> *__restrict__ d) {
-        const double2 *p = reinterpret_cast<const double2 *>(d->m);
-        e0 = __ldg(p); e1 = __ldg(p + 1); e2 = __ldg(p + 2); e3 = __ldg(p + 3);
-    }
-    __device__ __forceinline__ void get(bool f, double (&m)[8]) const {
-        m[0] = f ? e3.x : e0.x; m[1] = f ? e3.y : e0.y; m[2] = f ? e2.x : e1.x; m[3] = f ? e2.y : e1.y;
-        m[4] = f ? e1.x : e2.x; m[5] = f ? e1.y : e2.y; m[6] = f ? e0.x : e3.x; m[7] = f ? e0.y : e3.y;
-    }
-};
-template <>
-struct LayerRec<double, true> {
-    double r0, r1, r2, r3;
-    __device__ __forceinline__ void load(const DevOp<double> *__restrict__ d) {
-        r0 = __ldg(d->m); r1 = __ldg(d->m + 2); r2 = __ldg(d->m + 4); r3 = __ldg(d->m + 6);
-    }
-    __device__ __forceinline__ void get(bool f, double (&m)[8]) const {
-        m[0] = f ? r3 : r0; m[2] = f ? r2 : r1; m[4] = f ? r1 : r2; m[6] = f ? r0 : r3;
-        m[1] = m[3] = m[5] = m[7] = 0.0;
-    }
-};
-
-template <typename Real, typename A2, int R, int T, bool REAL>
-struct LayerStepPre {
-    __device__ __forceinline__ static void run(A2 (&a)[1 << R], const DevOp<Real> *__restrict__ mats, uint32_t mask,
-                                               uint32_t xr, LayerRec<Real, REAL> &cur) {
-        if (mask & (1u << T)) {
-            Real m[8];
-            cur.get((xr >> T) & 1u, m);
-            if (mask >> (T + 1)) cur.load(mats + 1);
-            if (REAL) reg_real<Real, A2, R, T, false>(a, m, 0u, 0u);
-            else reg_dense<Real, A2, R, T, false>(a, m, 0u, 0u);
-            mats++;
-        }
-        LayerStepPre<Real, A2, R, T + 1, REAL>::run(a, mats, mask, xr, cur);
-    }
-};
-template <typename Real, typename A2, int R, bool REAL>
-struct LayerStepPre<Real, A2, R, R, REAL> {
-    __device__ __forceinline__ static void run(A2 (&)[1 << R], const DevOp<Real> *__restrict__, uint32_t, uint32_t,
-                                               LayerRec<Real, REAL> &) {}
-};
-// A layer; each active bit's matrix is loaded while the previous bit's
-// arithmetic runs, except in FP64 complex layers, where the 16 registers it
-// holds cost more in spills than the overlap saves (26-qubit FP64 layered 5%
-// slower; FP64 H layers and Grover 5-10% faster, FP32 QFT 2.5% and Grover 9%).
-template <typename Real, typename A2, int R, bool REAL>
-__device__ __forceinline__ void apply_layer(A2 (&a)[1 << R], const DevOp<Real> *__restrict__ mats, uint32_t mask,
-                                            uint32_t xr) {
-    if constexpr (sizeof(Real) == 8 && !REAL) {
-        LayerStep<Real, A2, R, 0, false>::run(a, mats, mask, xr);
-        return;
-    }
-    LayerRec<Real, REAL> cur;
-    cur.load(mats);
-    LayerStepPre<Real, A2, R, 0, REAL>::run(a, mats, mask, xr, cur);
+// four values from the stream
+__device__ __forceinline__ void load4(const float *__restrict__ p, float (&v)[4]) {
+    const float4 x = *reinterpret_cast<const float4 *>(p);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
 }
+__device__ __forceinline__ void load4(const double *__restrict__ p, double (&v)[4]) {
+    const double2 x = reinterpret_cast<const double2 *>(p)[0], y = reinterpret_cast<const double2 *>(p)[1];
+    v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+}
+
+// HAD: the matrix [[1, 1], [1, -1]], no data (a Hadamard layer in a warp with
+// relabeled registers, which the in-place form below does not take).
+template <typename Real, typename A2, int R, int T>
+struct RealStep {
+    __device__ __forceinline__ static void run(A2 (&a)[1 << R], const Real *__restrict__ d, uint32_t mask, uint32_t xr,
+                                               bool had) {
+        if (mask & (1u << T)) {
+            Real v[4] = {1, 1, 1, -1}, m[8];
+            if (!had) load4(d, v);
+            const bool f = (xr >> T) & 1u;
+            m[0] = f ? v[3] : v[0];
+            m[2] = f ? v[2] : v[1];
+            m[4] = f ? v[1] : v[2];
+            m[6] = f ? v[0] : v[3];
+            reg_real<Real, A2, R, T, false>(a, m, 0u, 0u);
+            d += 4;
+        }
+        RealStep<Real, A2, R, T + 1>::run(a, d, mask, xr, had);
+    }
+};
+template <typename Real, typename A2, int R>
+struct RealStep<Real, A2, R, R> {
+    __device__ __forceinline__ static void run(A2 (&)[1 << R], const Real *__restrict__, uint32_t, uint32_t, bool) {}
+};
+
+template <typename Real, typename A2, int R, int T>
+struct HadStep {
+    __device__ __forceinline__ static void run(A2 (&a)[1 << R], uint32_t mask) {
+        if (mask & (1u << T)) {
+#pragma unroll
+            for (int r = 0; r < (1 << R); r++)
+                if (!(r & (1 << T))) ip_had(a[r].x, a[r].y, a[r | (1 << T)].x, a[r | (1 << T)].y);
+        }
+        HadStep<Real, A2, R, T + 1>::run(a, mask);
+    }
+};
+template <typename Real, typename A2, int R>
+struct HadStep<Real, A2, R, R> {
+    __device__ __forceinline__ static void run(A2 (&)[1 << R], uint32_t) {}
+};
 
 template <typename Real, typename A2>
 __device__ __forceinline__ A2 cmul2(A2 a, A2 b);
@@ -571,104 +548,81 @@ __device__ __forceinline__ void reg_half_phase(A2 (&a)[1 << R], A2 f) {
         if (r & (1 << T)) ip_cmul(a[r].x, a[r].y, f.x, f.y, nfi);
 }
 
-// A split layer (K_LAYER_SPLIT): on each active register bit T the gate
-// Rm diag(1, p), Rm real, as a phase on the registers whose bit T is 1 and the
-// real gate (2 packed FP32 instructions per amplitude): 4 instructions per
-// amplitude against the complex matrix's 8.  (A phase after the real part,
-// diag(1, q), follows the layer as a phase record: its code inside every
-// bit's body, never run by Rz.Ry gates, made layered passes 7% slower.)
+// Gates Rm diag(1, p), Rm real: on each active register bit T the phase on the
+// registers whose bit T is 1, then the real part.
+//   FP32 (S_SPLIT): the real 2x2, 2 packed operations an amplitude; 4 with the
+//     phase, against the complex matrix's 8.
+//   FP64 (S_ROT, lower.cpp make_rot): a rotation in place, its factor left
+//     out; 4 + 4 operations a pair against 16 of a complex 2x2 and 12 of the
+//     phase and a real 2x2.
 // Seen through a swapped label (xr bit T set) the gate is
 //   X Rm diag(1, p) X = p (X Rm X) diag(1, p*),
 // so the phase stays on the same registers, conjugated, the real matrix is
-// read bit-swapped and p joins the thread's factor `pend`, which the layer
-// multiplies into all registers at its end.  Each active bit's record is
-// loaded while the previous bit's arithmetic runs (22-26 qubit FP32 layered
-// circuits: 7% faster than loading it where it is used).
-// one split-gate record: (m00, m01, m10, m11) and p
-template <typename Real>
-struct SplitRec;
-template <>
-struct SplitRec<float> {
-    float4 r, pq;
-    __device__ __forceinline__ void load(const DevOp<float> *__restrict__ d) {
-        r = __ldg(reinterpret_cast<const float4 *>(d->m));
-        pq = __ldg(reinterpret_cast<const float4 *>(d->m) + 1);
-    }
-    __device__ __forceinline__ float2 p() const { return make_float2(pq.x, pq.y); }
-};
-template <>
-struct SplitRec<double> {
-    double2 r01, r23, pp;
-    __device__ __forceinline__ void load(const DevOp<double> *__restrict__ d) {
-        const double2 *m = reinterpret_cast<const double2 *>(d->m);
-        r01 = __ldg(m);
-        r23 = __ldg(m + 1);
-        pp = __ldg(m + 2);
-    }
-    __device__ __forceinline__ double2 p() const { return pp; }
-};
-template <typename Real>
-__device__ __forceinline__ void split_real(const SplitRec<Real> &c, bool flip, Real (&mm)[8]);
-template <>
-__device__ __forceinline__ void split_real<float>(const SplitRec<float> &c, bool flip, float (&mm)[8]) {
-    mm[0] = flip ? c.r.w : c.r.x;
-    mm[2] = flip ? c.r.z : c.r.y;
-    mm[4] = flip ? c.r.y : c.r.z;
-    mm[6] = flip ? c.r.x : c.r.w;
-}
-template <>
-__device__ __forceinline__ void split_real<double>(const SplitRec<double> &c, bool flip, double (&mm)[8]) {
-    mm[0] = flip ? c.r23.y : c.r01.x;
-    mm[2] = flip ? c.r23.x : c.r01.y;
-    mm[4] = flip ? c.r01.y : c.r23.x;
-    mm[6] = flip ? c.r01.x : c.r23.y;
-}
-
+// read bit-swapped (a rotation by the opposite angle) and p joins the thread's
+// factor `pend`, which the layer multiplies into all registers at its end.
 template <typename Real, typename A2, int R, int T>
 struct SplitStep {
-    __device__ __forceinline__ static void run(A2 (&a)[1 << R], const DevOp<Real> *__restrict__ mats,
-                                               uint32_t mask, uint32_t phases, uint32_t xr, A2 &pend,
-                                               SplitRec<Real> &cur) {
+    __device__ __forceinline__ static void run(A2 (&a)[1 << R], const Real *__restrict__ d, uint32_t mask, uint32_t xr,
+                                               A2 &pend) {
         if (mask & (1u << T)) {
             const bool flip = (xr >> T) & 1u;
-            const SplitRec<Real> c = cur;
-            // the next active bit's record, while this one's arithmetic runs
-            if (mask >> (T + 1)) cur.load(mats + 1);
-            if (phases & (1u << T)) {
-                A2 p = c.p();
-                const A2 pf = cmul2<Real>(pend, p);
-                pend.x = flip ? pf.x : pend.x;
-                pend.y = flip ? pf.y : pend.y;
+            Real v[4];
+            load4(d, v);
+            A2 p;
+            if constexpr (sizeof(Real) == 4) {
+                p = load_c<Real, A2>(d + 4);
+                d += 8;
+                // one rounding order whatever the compiler makes of the
+                // surrounding code
+                const Real px = __fmaf_rn(pend.x, p.x, -__fmul_rn(pend.y, p.y));
+                const Real py = __fmaf_rn(pend.x, p.y, __fmul_rn(pend.y, p.x));
+                pend.x = flip ? px : pend.x;
+                pend.y = flip ? py : pend.y;
                 p.y = flip ? -p.y : p.y;
+                Real m[8];
+                m[0] = flip ? v[3] : v[0];
+                m[2] = flip ? v[2] : v[1];
+                m[4] = flip ? v[1] : v[2];
+                m[6] = flip ? v[0] : v[3];
                 reg_half_phase<Real, A2, R, T>(a, p);
+                reg_real<Real, A2, R, T, false>(a, m, 0u, 0u);
+            } else {
+                d += 4;
+                if (flip) {
+                    // p itself: the stored phase carries 1 + t^2 = 1 / (1 + u t)
+                    const Real k = v[0] * v[1] + (Real)1;
+                    p.x = v[2] * k;
+                    p.y = v[3] * k;
+                    pend = cmul2<Real>(pend, p);
+                    v[0] = -v[0];
+                    v[1] = -v[1];
+                    v[3] = -v[3];
+                }
+                p.x = v[2];
+                p.y = v[3];
+                reg_half_phase<Real, A2, R, T>(a, p);
+#pragma unroll
+                for (int r = 0; r < (1 << R); r++)
+                    if (!(r & (1 << T))) ip_rot(a[r].x, a[r].y, a[r | (1 << T)].x, a[r | (1 << T)].y, v[1], v[0]);
             }
-            {
-                Real mm[8];
-                split_real<Real>(c, flip, mm);
-                reg_real<Real, A2, R, T, false>(a, mm, 0u, 0u);
-            }
-            mats++;
         }
-        SplitStep<Real, A2, R, T + 1>::run(a, mats, mask, phases, xr, pend, cur);
+        SplitStep<Real, A2, R, T + 1>::run(a, d, mask, xr, pend);
     }
 };
 template <typename Real, typename A2, int R>
 struct SplitStep<Real, A2, R, R> {
-    __device__ __forceinline__ static void run(A2 (&)[1 << R], const DevOp<Real> *__restrict__, uint32_t, uint32_t,
-                                               uint32_t, A2 &, SplitRec<Real> &) {}
+    __device__ __forceinline__ static void run(A2 (&)[1 << R], const Real *__restrict__, uint32_t, uint32_t, A2 &) {}
 };
 
 template <typename Real, typename A2, int R>
-__device__ __forceinline__ void apply_split_layer(A2 (&a)[1 << R], const DevOp<Real> *__restrict__ mats,
-                                                  uint32_t mask, uint32_t phases, uint32_t xr) {
+__device__ __forceinline__ void apply_split_layer(A2 (&a)[1 << R], const Real *__restrict__ d, uint32_t mask,
+                                                  uint32_t xr) {
     A2 pend;
     pend.x = 1;
     pend.y = 0;
-    SplitRec<Real> cur;
-    cur.load(mats);
-    SplitStep<Real, A2, R, 0>::run(a, mats, mask, phases, xr, pend, cur);
+    SplitStep<Real, A2, R, 0>::run(a, d, mask, xr, pend);
     // every thread of the warp reaches this point (ops are uniform)
-    if (__any_sync(0xffffffffu, pend.x != (Real)1 || pend.y != (Real)0)) {
+    if (__any_sync(0xffffffffu, (xr & mask) != 0u)) {
 #pragma unroll
         for (int r = 0; r < (1 << R); r++) ip_cmul2(a[r], pend);
     }
@@ -685,30 +639,48 @@ template <typename Real, typename A2>
 __device__ __forceinline__ A2 load_c(const Real *__restrict__ p);
 template <>
 __device__ __forceinline__ double2 load_c<double, double2>(const double *__restrict__ p) {
-    return __ldg(reinterpret_cast<const double2 *>(p));
+    return *reinterpret_cast<const double2 *>(p);
 }
 template <>
 __device__ __forceinline__ float2 load_c<float, float2>(const float *__restrict__ p) {
-    return __ldg(reinterpret_cast<const float2 *>(p));
+    return *reinterpret_cast<const float2 *>(p);
 }
 
-// Factor of one phase-block term for this thread: d0 or d1 of its diagonal
-// gate by the value of its target (a thread or non-tile bit), or 1 when its
-// controls on thread and non-tile bits do not hold.  Branch-free: the
-// conditions differ between threads of a warp.
+// A product term of a phase block (S_TERMS): thread controls and target,
+// non-tile controls, the diagonal's two entries.
+template <typename Real>
+constexpr int product_term_bytes() {
+    return 32 + 4 * (int)sizeof(Real);
+}
 template <typename Real, typename A2>
-__device__ __forceinline__ A2 term_factor(const DevOp<Real> *__restrict__ t, uint64_t base, uint32_t thr) {
-    const uint4 th = __ldg(reinterpret_cast<const uint4 *>(t) + 1);  // cm_thr, cv_thr, tpos2
-    const ulonglong2 gl = __ldg(reinterpret_cast<const ulonglong2 *>(t) + 2);
-    const A2 f0 = load_c<Real, A2>(t->m), f1 = load_c<Real, A2>(t->m + 6);
-    const bool ok = ((base & gl.x) == gl.y) && ((thr & th.x) == th.y);
-    const int tp = (int)th.z;
-    const uint32_t bv = tp >= TPOS_GLOBAL   ? (uint32_t)(base >> (tp - TPOS_GLOBAL)) & 1u
-                        : tp >= TPOS_THREAD ? (thr >> (tp - TPOS_THREAD)) & 1u
-                                            : 0u;
-    A2 f = bv ? f1 : f0;
-    f.x = ok ? f.x : (Real)1;
-    f.y = ok ? f.y : (Real)0;
+struct ProductTerm {
+    A2 f0, f1;
+    bool ok;
+    int tp;
+    __device__ __forceinline__ ProductTerm(const unsigned char *__restrict__ t, uint64_t base, uint32_t thr) {
+        const uint4 th = *reinterpret_cast<const uint4 *>(t);
+        const ulonglong2 gl = reinterpret_cast<const ulonglong2 *>(t)[1];
+        const Real *m = reinterpret_cast<const Real *>(t + 32);
+        f0 = load_c<Real, A2>(m);
+        f1 = load_c<Real, A2>(m + 2);
+        ok = ((base & gl.x) == gl.y) && ((thr & th.x) == th.y);
+        tp = (int)th.z;
+    }
+};
+
+// Factor of one term for this thread: d0 or d1 of its diagonal gate by the
+// value of its target (a thread or non-tile bit), or 1 when its controls on
+// thread and non-tile bits do not hold.  Branch-free: the conditions differ
+// between threads of a warp.
+template <typename Real, typename A2>
+__device__ __forceinline__ A2 term_factor(const unsigned char *__restrict__ t, uint64_t base, uint32_t thr) {
+    const ProductTerm<Real, A2> q(t, base, thr);
+    const uint32_t bv = q.tp >= TPOS_GLOBAL   ? (uint32_t)(base >> (q.tp - TPOS_GLOBAL)) & 1u
+                        : q.tp >= TPOS_THREAD ? (thr >> (q.tp - TPOS_THREAD)) & 1u
+                                              : 0u;
+    A2 f = bv ? q.f1 : q.f0;
+    f.x = q.ok ? f.x : (Real)1;
+    f.y = q.ok ? f.y : (Real)0;
     return f;
 }
 
@@ -723,71 +695,63 @@ __device__ __forceinline__ A2 cmul2(A2 a, A2 b) {
 // acc times the factors of terms t[0..n), two terms per step (two chains, so
 // that one term's loads overlap the other's arithmetic).
 template <typename Real, typename A2>
-__device__ __forceinline__ A2 term_product(const DevOp<Real> *__restrict__ t, int n, uint64_t base, uint32_t thr,
+__device__ __forceinline__ A2 term_product(const unsigned char *__restrict__ t, int n, uint64_t base, uint32_t thr,
                                            A2 acc) {
+    constexpr int B = product_term_bytes<Real>();
     A2 acc2;
     acc2.x = 1;
     acc2.y = 0;
     int i = 0;
 #pragma unroll 1
     for (; i + 1 < n; i += 2) {
-        const A2 fa = term_factor<Real, A2>(t + i, base, thr), fb = term_factor<Real, A2>(t + i + 1, base, thr);
+        const A2 fa = term_factor<Real, A2>(t + i * B, base, thr), fb = term_factor<Real, A2>(t + (i + 1) * B, base, thr);
         acc = cmul2<Real>(acc, fa);
         acc2 = cmul2<Real>(acc2, fb);
     }
-    if (i < n) acc = cmul2<Real>(acc, term_factor<Real, A2>(t + i, base, thr));
+    if (i < n) acc = cmul2<Real>(acc, term_factor<Real, A2>(t + i * B, base, thr));
     return cmul2<Real>(acc, acc2);
 }
 
 // D terms (a diagonal gate on register bit b, controls elsewhere): h takes
 // d0, g takes d1, where the controls hold.
 template <typename Real, typename A2>
-__device__ __forceinline__ void term_diag_product(const DevOp<Real> *__restrict__ t, int n, uint64_t base,
+__device__ __forceinline__ void term_diag_product(const unsigned char *__restrict__ t, int n, uint64_t base,
                                                   uint32_t thr, A2 &h, A2 &g) {
 #pragma unroll 1
     for (int i = 0; i < n; i++) {
-        const uint4 th = __ldg(reinterpret_cast<const uint4 *>(t + i) + 1);
-        const ulonglong2 gl = __ldg(reinterpret_cast<const ulonglong2 *>(t + i) + 2);
-        A2 f0 = load_c<Real, A2>(t[i].m), f1 = load_c<Real, A2>(t[i].m + 6);
-        const bool ok = ((base & gl.x) == gl.y) && ((thr & th.x) == th.y);
-        f0.x = ok ? f0.x : (Real)1;
-        f0.y = ok ? f0.y : (Real)0;
-        f1.x = ok ? f1.x : (Real)1;
-        f1.y = ok ? f1.y : (Real)0;
-        h = cmul2<Real>(h, f0);
-        g = cmul2<Real>(g, f1);
+        ProductTerm<Real, A2> q(t + i * product_term_bytes<Real>(), base, thr);
+        q.f0.x = q.ok ? q.f0.x : (Real)1;
+        q.f0.y = q.ok ? q.f0.y : (Real)0;
+        q.f1.x = q.ok ? q.f1.x : (Real)1;
+        q.f1.y = q.ok ? q.f1.y : (Real)0;
+        h = cmul2<Real>(h, q.f0);
+        g = cmul2<Real>(g, q.f1);
     }
 }
 
-// A phase block's 2^R table: complex factors by register label, four per
-// record (the m[] of consecutive records from z), register r holding label
-// r ^ xr.  When no lane of the warp has a relabeled register (xr == 0, as in
-// the QFT's phase passes), the labels are the register numbers and every
-// entry sits at a constant offset: two entries per 16-byte load in FP32 and
-// no address arithmetic, which was most of the integer work of a QFT pass
-// (six instructions per register and table).
+// A phase block's 2^R table: complex factors by register label, register r
+// holding label r ^ xr.  When no lane of the warp has a relabeled register
+// (xr == 0, as in the QFT's phase passes), the labels are the register numbers
+// and every entry sits at a constant offset: two entries per 16-byte load in
+// FP32 and no address arithmetic.
 template <typename Real, typename A2, int R>
 __device__ __forceinline__ void apply_table(A2 (&a)[1 << R], const Real *__restrict__ z, uint32_t xr) {
-    constexpr int stride = (int)(sizeof(DevOp<Real>) / sizeof(Real));
     if (__all_sync(0xffffffffu, xr == 0u)) {
         if constexpr (sizeof(Real) == 4) {
 #pragma unroll
             for (int r = 0; r < (1 << R); r += 2) {
-                const float4 f = __ldg(reinterpret_cast<const float4 *>(z + (r >> 2) * stride + 2 * (r & 3)));
+                const float4 f = *reinterpret_cast<const float4 *>(z + 2 * r);
                 ip_cmul2(a[r], make_float2(f.x, f.y));
                 ip_cmul2(a[r + 1], make_float2(f.z, f.w));
             }
         } else {
 #pragma unroll
-            for (int r = 0; r < (1 << R); r++) ip_cmul2(a[r], load_c<Real, A2>(z + (r >> 2) * stride + 2 * (r & 3)));
+            for (int r = 0; r < (1 << R); r++) ip_cmul2(a[r], load_c<Real, A2>(z + 2 * r));
         }
         return;
     }
 #pragma unroll
-    for (int r = 0; r < (1 << R); r++) {
-        const uint32_t l = r ^ xr;
-        ip_cmul2(a[r], load_c<Real, A2>(z + (l >> 2) * stride + 2 * (l & 3)));
-    }
+    for (int r = 0; r < (1 << R); r++) ip_cmul2(a[r], load_c<Real, A2>(z + 2 * (r ^ xr)));
 }
 
 // Byte K of the 16 phase-block term counts, kept packed in four words.
@@ -804,28 +768,29 @@ __device__ __forceinline__ int count_byte(const uint4 &c) {
 // with one sweep.  Inactive bits cost nothing but the pointer step.
 template <typename Real, typename A2, int R, int B>
 struct PhaseBits {
-    __device__ __forceinline__ static void run(A2 (&a)[1 << R], const DevOp<Real> *__restrict__ t,
+    __device__ __forceinline__ static void run(A2 (&a)[1 << R], const unsigned char *__restrict__ t,
                                                const uint4 &cnt, uint32_t act, A2 &carry, uint64_t base,
                                                uint32_t thr, uint32_t xr) {
+        constexpr int TB = product_term_bytes<Real>();
         const int ng = count_byte<1 + B>(cnt), nh = count_byte<1 + R + B>(cnt), nd = count_byte<1 + 2 * R + B>(cnt);
         if (act & (1u << B)) {
             A2 g = term_product<Real, A2>(t, ng, base, thr, carry);
-            A2 h = term_product<Real, A2>(t + ng, nh, base, thr, carry);
+            A2 h = term_product<Real, A2>(t + ng * TB, nh, base, thr, carry);
             carry.x = 1;
             carry.y = 0;
-            term_diag_product<Real, A2>(t + ng + nh, nd, base, thr, h, g);
+            term_diag_product<Real, A2>(t + (ng + nh) * TB, nd, base, thr, h, g);
             // g belongs to the registers whose label has bit B set
             const bool flip = (xr >> B) & 1u;
             const A2 g1 = flip ? h : g, h1 = flip ? g : h;
 #pragma unroll
             for (int r = 0; r < (1 << R); r++) ip_cmul2(a[r], ((r >> B) & 1) ? g1 : h1);
         }
-        PhaseBits<Real, A2, R, B + 1>::run(a, t + ng + nh + nd, cnt, act, carry, base, thr, xr);
+        PhaseBits<Real, A2, R, B + 1>::run(a, t + (ng + nh + nd) * TB, cnt, act, carry, base, thr, xr);
     }
 };
 template <typename Real, typename A2, int R>
 struct PhaseBits<Real, A2, R, R> {
-    __device__ __forceinline__ static void run(A2 (&)[1 << R], const DevOp<Real> *__restrict__, const uint4 &,
+    __device__ __forceinline__ static void run(A2 (&)[1 << R], const unsigned char *__restrict__, const uint4 &,
                                                uint32_t, A2 &, uint64_t, uint32_t, uint32_t) {}
 };
 
@@ -846,7 +811,7 @@ struct TermWords<float> {
     float a0, a1, scale;
     uint64_t mask;
     __device__ __forceinline__ TermWords(const unsigned char *p) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
+        const uint4 v = *reinterpret_cast<const uint4 *>(p);
         head = v.x;
         a0 = __uint_as_float(v.y);
         a1 = __uint_as_float(v.z);
@@ -860,8 +825,8 @@ struct TermWords<double> {
     double a0, a1, scale;
     uint64_t mask;
     __device__ __forceinline__ TermWords(const unsigned char *p) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
-        const double2 w = __ldg(reinterpret_cast<const double2 *>(p) + 1);
+        const uint4 v = *reinterpret_cast<const uint4 *>(p);
+        const double2 w = reinterpret_cast<const double2 *>(p)[1];
         head = v.x;
         a0 = __hiloint2double((int)v.w, (int)v.z);
         a1 = w.x;
@@ -884,8 +849,7 @@ __device__ __forceinline__ Real linear_turns(const TermWords<Real> &t, uint64_t 
 // (0 where its control does not hold).
 template <typename Real>
 __device__ __forceinline__ Real term_turns(const unsigned char *__restrict__ rec0, int k, uint64_t ix) {
-    constexpr int per = pb_terms_per_record<Real>();
-    const TermWords<Real> t(rec0 + (k / per) * sizeof(DevOp<Real>) + (k % per) * sizeof(PhaseTerm<Real>));
+    const TermWords<Real> t(rec0 + k * sizeof(PhaseTerm<Real>));
     const int cbit = (int)(int8_t)(t.head & 0xffu), cval = (int)((t.head >> 8) & 0xffu);
     const int tbit = (int)(int8_t)((t.head >> 16) & 0xffu);
     const uint32_t tv = tbit < 0 ? 0u : (uint32_t)((ix >> (tbit & 63)) & 1u);
@@ -899,8 +863,7 @@ __device__ __forceinline__ Real term_turns(const unsigned char *__restrict__ rec
 template <typename Real>
 __device__ __forceinline__ void dterm_turns(const unsigned char *__restrict__ rec0, int k, uint64_t ix, Real &h,
                                             Real &g) {
-    constexpr int per = pb_terms_per_record<Real>();
-    const TermWords<Real> t(rec0 + (k / per) * sizeof(DevOp<Real>) + (k % per) * sizeof(PhaseTerm<Real>));
+    const TermWords<Real> t(rec0 + k * sizeof(PhaseTerm<Real>));
     const int cbit = (int)(int8_t)(t.head & 0xffu), cval = (int)((t.head >> 8) & 0xffu);
     if (cbit == PB_LINEAR) {
         const int tbit = (int)(int8_t)((t.head >> 16) & 0xffu);
@@ -976,11 +939,10 @@ template <typename Real, typename A2, int R, int B>
 struct GatedSweep {
     __device__ __forceinline__ static void run(int b, A2 (&a)[1 << R], A2 c, const Real *__restrict__ z) {
         if (b == B) {
-            constexpr int stride = (int)(sizeof(DevOp<Real>) / sizeof(Real));
 #pragma unroll
             for (int r = 0; r < (1 << R); r++)
                 if (r & (1 << B)) {
-                    ip_cmul2(a[r], load_c<Real, A2>(z + (r >> 2) * stride + 2 * (r & 3)));
+                    ip_cmul2(a[r], load_c<Real, A2>(z + 2 * r));
                     ip_cmul2(a[r], c);
                 }
             return;
@@ -993,31 +955,30 @@ struct GatedSweep<Real, A2, R, R> {
     __device__ __forceinline__ static void run(int, A2 (&)[1 << R], A2, const Real *__restrict__) {}
 };
 
+// S_PHASES: `op` is the op's head in the stream window, hdr its first unit.
 template <typename Real, typename A2, int R>
-__device__ __forceinline__ void apply_phase_block_angles(A2 (&a)[1 << R], const DevOp<Real> *__restrict__ op,
-                                                         uint64_t base, uint32_t thr, uint32_t xr) {
-    const uint4 hdr = __ldg(reinterpret_cast<const uint4 *>(op));
-    const int nrec = (int)hdr.y;
-    const bool has_table = hdr.z & PB_HAS_TABLE;
-    const uint32_t act = hdr.w;
-    const uint4 cnt = __ldg(reinterpret_cast<const uint4 *>(op->m));
-    const uint2 tg = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const unsigned char *>(op->m) + 16));
+__device__ __forceinline__ void apply_phase_block_angles(A2 (&a)[1 << R], const unsigned char *__restrict__ op,
+                                                         const uint4 hdr, uint64_t base, uint32_t thr, uint32_t xr) {
+    const uint32_t flags = hdr.y, act = hdr.z;
+    const Real *__restrict__ table = reinterpret_cast<const Real *>(op + 16 * hdr.w);
+    const uint4 cnt = reinterpret_cast<const uint4 *>(op)[1];
+    const uint2 tg = reinterpret_cast<const uint2 *>(op)[4];
     uint64_t ix = base;
 #pragma unroll
     for (int t = 0; t < 8; t++) {
         const uint32_t g = ((t < 4 ? tg.x : tg.y) >> (8 * (t & 3))) & 63u;
         ix |= (uint64_t)((thr >> t) & 1u) << g;
     }
-    const unsigned char *rec0 = reinterpret_cast<const unsigned char *>(op + 1);
-    if ((hdr.z & PB_GATED) && __all_sync(0xffffffffu, xr == 0u)) {
+    const unsigned char *rec0 = op + 48;
+    if ((flags & PB_GATED) && __all_sync(0xffffffffu, xr == 0u)) {
         // only G[b] terms, then D[b] terms (the walk order with every other
         // category empty); one factor for the registers whose bit b is 1
-        const int b = (int)((hdr.z >> PB_GATE_SHIFT) & 7u);
+        const int b = (int)((flags >> PB_GATE_SHIFT) & 7u);
         const int ng = count_byte_at(cnt, 1 + b), nd = count_byte_at(cnt, 1 + 2 * R + b);
         Real g = turns_sum<Real>(rec0, 0, ng, ix, (Real)0), h = 0;
 #pragma unroll 1
         for (int i = 0; i < nd; i++) dterm_turns<Real>(rec0, ng + i, ix, h, g);
-        GatedSweep<Real, A2, R, 0>::run(b, a, cis_turns<A2>(g), (op + 1 + nrec - (1 << R) / 4)->m);
+        GatedSweep<Real, A2, R, 0>::run(b, a, cis_turns<A2>(g), table);
         return;
     }
     const int nf = count_byte<0>(cnt);
@@ -1028,46 +989,214 @@ __device__ __forceinline__ void apply_phase_block_angles(A2 (&a)[1 << R], const 
 #pragma unroll
         for (int r = 0; r < (1 << R); r++) ip_cmul2(a[r], f);
     }
-    if (has_table) apply_table<Real, A2, R>(a, (op + 1 + nrec - (1 << R) / 4)->m, xr);
+    if (flags & PB_HAS_TABLE) apply_table<Real, A2, R>(a, table, xr);
 }
 
-// K_PHASE_BLOCK: the F terms fold into one per-thread factor; each active
-// register bit costs one sweep of the registers (PhaseBits); the F factor
-// rides on the first active bit's sweep, or gets a sweep of its own when no
-// bit is active; the thread-independent 2^R table, if any, is one more sweep.
+// S_TERMS: the F terms fold into one per-thread factor; each active register
+// bit costs one sweep of the registers (PhaseBits); the F factor rides on the
+// first active bit's sweep, or gets a sweep of its own when no bit is active;
+// the thread-independent 2^R table, if any, is one more sweep.
 template <typename Real, typename A2, int R>
-__device__ __forceinline__ int apply_phase_block(A2 (&a)[1 << R], const DevOp<Real> *__restrict__ op, uint64_t base,
-                                                 uint32_t thr, uint32_t xr) {
-    const uint4 hdr = __ldg(reinterpret_cast<const uint4 *>(op));
-    const int nrec = (int)hdr.y;  // records after the head
-    const bool has_table = hdr.z & 1u;
-    const uint32_t act = hdr.w;   // active register bits, PB_F_ACTIVE: F terms
-    const uint4 cnt = __ldg(reinterpret_cast<const uint4 *>(op->m));  // 16 count bytes
-    const DevOp<Real> *__restrict__ t = op + 1;
+__device__ __forceinline__ void apply_phase_block(A2 (&a)[1 << R], const unsigned char *__restrict__ op, const uint4 hdr,
+                                                  uint64_t base, uint32_t thr, uint32_t xr) {
+    const uint32_t act = hdr.z;   // active register bits, PB_F_ACTIVE: F terms
+    const uint4 cnt = reinterpret_cast<const uint4 *>(op)[1];  // 16 count bytes
+    const unsigned char *__restrict__ t = op + 48;
     A2 carry;
     carry.x = 1;
     carry.y = 0;
     const int nf = count_byte<0>(cnt);
     carry = term_product<Real, A2>(t, nf, base, thr, carry);
-    PhaseBits<Real, A2, R, 0>::run(a, t + nf, cnt, act, carry, base, thr, xr);
+    PhaseBits<Real, A2, R, 0>::run(a, t + nf * product_term_bytes<Real>(), cnt, act, carry, base, thr, xr);
     if ((act & PB_F_ACTIVE) && !(act & ((1u << R) - 1u))) {
 #pragma unroll
         for (int r = 0; r < (1 << R); r++) ip_cmul2(a[r], carry);
     }
-    if (has_table) apply_table<Real, A2, R>(a, (t + nrec - (1 << R) / 4)->m, xr);
-    return 1 + nrec;
+    if (hdr.y & PB_HAS_TABLE) apply_table<Real, A2, R>(a, reinterpret_cast<const Real *>(op + 16 * hdr.w), xr);
 }
 
-// Records taken by the op whose head record is `hdr`: a phase block's terms
-// and table, a layer's matrices, or the record alone.
-__device__ __forceinline__ int op_records(const uint4 &hdr) {
-    if ((int)hdr.x == K_PHASE_BLOCK) return 1 + (int)hdr.y;
-    if ((int)hdr.x == K_LAYER || (int)hdr.x == K_LAYER_REAL || (int)hdr.x == K_LAYER_SPLIT) return 1 + __popc(hdr.z);
-    return 1;
+// One relabeling X gate (a K_XSET entry): flips the thread's label bit where
+// its control holds.
+__device__ __forceinline__ uint32_t xset_flip(uint32_t w, uint64_t base, uint32_t thr) {
+    const uint32_t t = w & 0xffu, ck = (w >> 8) & 0xffu, cb = (w >> 16) & 0xffu, cv = w >> 24;
+    const uint32_t v = ck == XSET_CTRL_THREAD   ? (thr >> cb) & 1u
+                       : ck == XSET_CTRL_GLOBAL ? (uint32_t)(base >> cb) & 1u
+                                                : cv;
+    return (uint32_t)(v == cv) << t;
 }
 
-// Applies record `op` (and, for a layer or phase block, the records that
-// follow it); its head record `hdr` is already loaded.
+// X on register bit T under register-bit controls (S_CSWAP).
+template <typename A2, int R, int T>
+struct CSwap {
+    __device__ __forceinline__ static void run(uint32_t t, A2 (&a)[1 << R], uint32_t cm, uint32_t cv) {
+        if (t == T) reg_swap<A2, R, T, true>(a, cm, cv);
+        CSwap<A2, R, T + 1>::run(t, a, cm, cv);
+    }
+};
+template <typename A2, int R>
+struct CSwap<A2, R, R> {
+    __device__ __forceinline__ static void run(uint32_t, A2 (&)[1 << R], uint32_t, uint32_t) {}
+};
+
+// Any other record (S_GATE).
+template <typename Real, typename A2, int R, bool LEAN>
+__device__ __forceinline__ void apply_gate(A2 (&a)[1 << R], const unsigned char *__restrict__ op, const uint4 hdr,
+                                           uint64_t base, uint32_t thr, uint32_t &xr) {
+    const int kind = (int)(hdr.y & 0xffu), tpos = (int)(hdr.y >> 8);
+    const uint2 th = reinterpret_cast<const uint2 *>(op)[2];             // cm_thr, cv_thr
+    const ulonglong2 gl = reinterpret_cast<const ulonglong2 *>(op)[2];   // cm_glob, cv_glob
+    if ((base & gl.x) != gl.y) return;
+    if ((thr & th.x) != th.y) return;
+    const Real *m = reinterpret_cast<const Real *>(op + 48);
+    const uint32_t cm = hdr.z, cv = hdr.w ^ (xr & hdr.z);
+    if (tpos < R) {
+        if (kind == K_SWAP && cm == 0) {
+            xr ^= 1u << tpos;
+            return;
+        }
+        // a phase gate seen through a swapped label is diag(d1, 1): run it as
+        // a diagonal gate on the bit-swapped matrix
+        const bool flip = (xr >> tpos) & 1u;
+        const int k = (kind == K_PHASE && flip) ? K_DIAG : kind;
+        RegTarget<Real, A2, R, 0, LEAN>::run(1u << tpos, 1u << k, a, m, cm, cv, flip);
+        return;
+    }
+    // diagonal gate on a thread bit or a non-tile index bit
+    const int bv = tpos >= TPOS_GLOBAL ? (int)((base >> (tpos - TPOS_GLOBAL)) & 1)
+                                       : (int)((thr >> (tpos - TPOS_THREAD)) & 1);
+    if (kind == K_PHASE && !bv) return;
+    const A2 f = load_c<Real, A2>(m + (bv ? 6 : 0));
+    reg_scale<Real, A2, R, true>(a, f.x, f.y, cm, cv);
+}
+
+// ---- the stream in shared memory ---------------------------------------------
+
+constexpr int STREAM_WINDOW_BYTES = STREAM_WINDOW_UNITS * 16;
+
+// Shared memory of a CTA: the transpose buffer, then two stream windows.
+template <typename Real, int R, int W>
+__host__ __device__ constexpr int tile_smem_bytes() {
+    return tile_smem_elems<R, W>() * (int)sizeof(typename V2<Real>::T);
+}
+template <typename Real, int R, int W>
+__host__ __device__ constexpr int cta_smem_bytes() {
+    return tile_smem_bytes<Real, R, W>() + 2 * STREAM_WINDOW_BYTES;
+}
+
+// Starts the CTA's copy of `units` units into shared memory (cached in L1: the
+// SM's other CTAs run the same pass).
+__device__ __forceinline__ void fetch_units(unsigned char *dst, const uint4 *__restrict__ src, int units) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    for (int i = threadIdx.x; i < units; i += blockDim.x)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d + 16u * i), "l"(src + i) : "memory");
+}
+__device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Starts copying a pass's first two windows; every earlier reader of the
+// windows must be done.
+__device__ __forceinline__ void fetch_stream(unsigned char *win, const TileArgs &ta) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(ta.stream);
+    fetch_units(win, src, ta.units0);
+    if (ta.units1) fetch_units(win + STREAM_WINDOW_BYTES, src + ta.units0, ta.units1);
+}
+
+// ---- layout transposes through shared memory --------------------------------
+
+// Moves the registers from the current layout (thread base `tb`, byte steps in
+// the op) to the next.  Register r holds label r ^ xr (register relabeling,
+// below): its slot is the thread's base plus the steps of the bits of r ^ xr,
+// i.e. the base moved by the steps of xr plus the steps of r with those bits
+// negated.
+template <typename A2, int R, int W>
+__device__ __forceinline__ void transpose(A2 (&a)[1 << R], unsigned char *sm, const unsigned char *__restrict__ op,
+                                          const uint4 hdr, uint32_t thr, uint32_t &tb, uint32_t xr) {
+    {
+        const uint4 f = reinterpret_cast<const uint4 *>(op)[1];
+        const uint32_t all[5] = {f.x, f.y, f.z, f.w, hdr.z};
+        uint32_t wb = tb, s[R];
+        if (hdr.y & STREAM_SYNC_BEFORE) __syncthreads();
+        else __syncwarp();
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+            const bool fl = (xr >> q) & 1u;
+            wb += fl ? all[q] : 0u;
+            s[q] = fl ? 0u - all[q] : all[q];
+        }
+#pragma unroll
+        for (int r = 0; r < (1 << R); r++) {
+            uint32_t o = wb;
+#pragma unroll
+            for (int q = 0; q < R; q++)
+                if (r & (1 << q)) o += s[q];
+            *reinterpret_cast<A2 *>(sm + o) = a[r];
+        }
+    }
+    const uint4 t = reinterpret_cast<const uint4 *>(op)[2], b0 = reinterpret_cast<const uint4 *>(op)[3],
+                b1 = reinterpret_cast<const uint4 *>(op)[4];
+    const uint32_t u[5] = {t.x, t.y, t.z, t.w, hdr.w};
+    const uint32_t bs[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    tb = 0;
+#pragma unroll
+    for (int b = 0; b < 5 + W; b++) tb += ((thr >> b) & 1u) * bs[b];
+    if (hdr.y & STREAM_SYNC_CROSS) __syncthreads();
+    else __syncwarp();
+#pragma unroll
+    for (int r = 0; r < (1 << R); r++) {
+        uint32_t o = tb;
+#pragma unroll
+        for (int q = 0; q < R; q++)
+            if (r & (1 << q)) o += u[q];
+        a[r] = *reinterpret_cast<const A2 *>(sm + o);
+    }
+}
+
+// Index of tile `t`: deposit the bits of t into the non-tile index bits, one
+// run of consecutive non-tile bits at a time (uniform across the CTA).
+__device__ __forceinline__ uint64_t tile_base(uint64_t t, const TileArgs &ta) {
+    uint64_t base = 0;
+#pragma unroll
+    for (int i = 0; i < MAX_FREE_RUNS; i++) {
+        if (i >= ta.nruns) break;
+        const int len = ta.run_len[i];
+        base |= (t & ((1ull << len) - 1ull)) << ta.run_pos[i];
+        t >>= len;
+    }
+    return base;
+}
+
+template <typename Real, int R, int W>
+__device__ __forceinline__ void load_tile(typename V2<Real>::T (&a)[1 << R],
+                                          const typename V2<Real>::T *__restrict__ state, const TileArgs &ta,
+                                          uint64_t base, uint32_t thr) {
+    using A2 = typename V2<Real>::T;
+    uint64_t off, rs[R];
+    thread_geometry<R, W>(ta.ld_gbit, thr, off, rs);
+    LoadF<A2, R> f{a, state + (base | off), rs};
+    Unroll<1 << R>::run(f);
+}
+
+template <typename Real, int R, int W>
+__device__ __forceinline__ void store_tile(const typename V2<Real>::T (&a)[1 << R],
+                                           typename V2<Real>::T *__restrict__ state, const TileArgs &ta,
+                                           uint64_t base, uint32_t xr) {
+    using A2 = typename V2<Real>::T;
+    // The thread index is re-read so the store geometry is recomputed here
+    // instead of being held in registers through every phase.
+    uint32_t thr;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thr));
+    uint64_t off, rs[R];
+    thread_geometry<R, W>(ta.st_gbit, thr, off, rs);
+    uint64_t xo = 0;
+#pragma unroll
+    for (int q = 0; q < R; q++)
+        if ((xr >> q) & 1u) xo |= rs[q];
+    StoreF<A2, R> f{a, state, base | off | xo, rs};
+    Unroll<1 << R>::run(f);
+}
+
+// Applies a pass's stream to a tile already in registers (loaded in the
+// pass's load layout) and stores it.  The first windows' copy (fetch_stream)
+// has been started.
 //
 // Register relabeling: a thread keeps `xr`, and register r holds the
 // amplitude whose register label is r ^ xr.  An X on a register bit whose
@@ -1083,185 +1212,19 @@ __device__ __forceinline__ int op_records(const uint4 &hdr) {
 // -- code the benchmark circuits never run -- made 26-qubit FP32 layered
 // passes 5% and QFT passes 9% faster (fewer instruction-fetch stalls), so
 // each plan runs the smallest build it can.
-template <typename Real, typename A2, int R, bool LEAN>
-__device__ __forceinline__ void apply_op(A2 (&a)[1 << R], const DevOp<Real> *__restrict__ op, const uint4 hdr,
-                                         uint64_t base, uint32_t thr, uint32_t &xr) {
-    const int kind = (int)hdr.x, tpos = (int)hdr.y;  // hdr: kind, tpos, cm_reg, cv_reg of `op`
-    if (kind == K_PHASE_BLOCK) {
-        if (LEAN || (hdr.z & PB_ANGLES)) apply_phase_block_angles<Real, A2, R>(a, op, base, thr, xr);
-        else apply_phase_block<Real, A2, R>(a, op, base, thr, xr);
-        return;
-    }
-    if (kind == K_XSET) {
-        // up to 8 (FP32) or 16 (FP64) relabeling X gates, 4 bytes each
-        const uint4 *e = reinterpret_cast<const uint4 *>(op->m);
-        const int n = tpos;
-#pragma unroll
-        for (int q = 0; q < xset_entries<Real>() / 4; q++) {
-            if (4 * q >= n) break;
-            const uint4 w4 = __ldg(e + q);
-            const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if (4 * q + j >= n) break;
-                const uint32_t t = w[j] & 0xffu, ck = (w[j] >> 8) & 0xffu, cb = (w[j] >> 16) & 0xffu,
-                               cv = w[j] >> 24;
-                const uint32_t v = ck == XSET_CTRL_THREAD   ? (thr >> cb) & 1u
-                                   : ck == XSET_CTRL_GLOBAL ? (uint32_t)(base >> cb) & 1u
-                                                            : cv;
-                xr ^= (uint32_t)(v == cv) << t;
-            }
-        }
-        return;
-    }
-    if (kind == K_LAYER_SPLIT) {
-        apply_split_layer<Real, A2, R>(a, op + 1, hdr.z, hdr.w, xr);
-        return;
-    }
-    if (kind == K_LAYER || kind == K_LAYER_REAL) {
-        const uint32_t mask = hdr.z;  // active register bits
-        if (kind == K_LAYER) {
-            if constexpr (!LEAN) apply_layer<Real, A2, R, false>(a, op + 1, mask, xr);
-        } else {
-            apply_layer<Real, A2, R, true>(a, op + 1, mask, xr);
-        }
-        return;
-    }
-    const uint4 th = __ldg(reinterpret_cast<const uint4 *>(op) + 1);                 // cm_thr, cv_thr
-    const ulonglong2 gl = __ldg(reinterpret_cast<const ulonglong2 *>(op) + 2);       // cm_glob, cv_glob
-    if ((base & gl.x) != gl.y) return;
-    if ((thr & th.x) != th.y) return;
-    const uint32_t cm = hdr.z, cv = hdr.w ^ (xr & hdr.z);
-    if (tpos < R) {
-        if (kind == K_SWAP && cm == 0) {
-            xr ^= 1u << tpos;
-            return;
-        }
-        // a phase gate seen through a swapped label is diag(d1, 1): run it as
-        // a diagonal gate on the bit-swapped matrix
-        const bool flip = (xr >> tpos) & 1u;
-        const int k = (kind == K_PHASE && flip) ? K_DIAG : kind;
-        RegTarget<Real, A2, R, 0, LEAN>::run(1u << tpos, 1u << k, a, op->m, cm, cv, flip);
-        return;
-    }
-    // diagonal gate on a thread bit or a non-tile index bit
-    const int bv = tpos >= TPOS_GLOBAL ? (int)((base >> (tpos - TPOS_GLOBAL)) & 1)
-                                       : (int)((thr >> (tpos - TPOS_THREAD)) & 1);
-    if (kind == K_PHASE && !bv) return;
-    const A2 f = load_c<Real, A2>(op->m + (bv ? 6 : 0));
-    const Real fr = f.x, fi = f.y;
-    reg_scale<Real, A2, R, true>(a, fr, fi, cm, cv);
-    return;
-}
-
-// ---- layout transposes through shared memory --------------------------------
-
-// Moves the registers from layout `from` to layout `to` (layout tables: the
-// byte offset of each register bit's unit step, then each thread's register-0
-// offset).  Register r holds label r ^ xr (apply_op): its slot is the
-// thread's base plus the steps of the bits of r ^ xr, i.e. the base moved by
-// the steps of xr plus the steps of r with those bits negated.
-template <typename A2, int R>
-__device__ __forceinline__ void transpose(A2 (&a)[1 << R], unsigned char *sm, uint32_t thr,
-                                          const uint32_t *__restrict__ from, const uint32_t *__restrict__ to,
-                                          bool sync_cta_before, bool cross, uint32_t xr) {
-    uint32_t wb = __ldg(from + LAYOUT_HDR + thr), s[R];
-#pragma unroll
-    for (int q = 0; q < R; q++) s[q] = __ldg(from + q);
-    if (sync_cta_before) __syncthreads();
-    else __syncwarp();
-#pragma unroll
-    for (int q = 0; q < R; q++) {
-        const bool f = (xr >> q) & 1u;
-        wb += f ? s[q] : 0u;
-        s[q] = f ? 0u - s[q] : s[q];
-    }
-#pragma unroll
-    for (int r = 0; r < (1 << R); r++) {
-        uint32_t o = wb;
-#pragma unroll
-        for (int q = 0; q < R; q++)
-            if (r & (1 << q)) o += s[q];
-        *reinterpret_cast<A2 *>(sm + o) = a[r];
-    }
-    uint32_t rb = __ldg(to + LAYOUT_HDR + thr), u[R];
-#pragma unroll
-    for (int q = 0; q < R; q++) u[q] = __ldg(to + q);
-    if (cross) __syncthreads();
-    else __syncwarp();
-#pragma unroll
-    for (int r = 0; r < (1 << R); r++) {
-        uint32_t o = rb;
-#pragma unroll
-        for (int q = 0; q < R; q++)
-            if (r & (1 << q)) o += u[q];
-        a[r] = *reinterpret_cast<const A2 *>(sm + o);
-    }
-}
-
-// Index of tile `t`: deposit the bits of t into the non-tile index bits, one
-// run of consecutive non-tile bits at a time (uniform across the CTA).
-__device__ __forceinline__ uint64_t tile_base(uint64_t t, const PassArgs &pa) {
-    uint64_t base = 0;
-#pragma unroll
-    for (int i = 0; i < MAX_FREE_RUNS; i++) {
-        if (i >= pa.nruns) break;
-        const int len = pa.run_len[i];
-        base |= (t & ((1ull << len) - 1ull)) << pa.run_pos[i];
-        t >>= len;
-    }
-    return base;
-}
-
-template <typename Real, int R, int W>
-__device__ __forceinline__ void load_tile(typename V2<Real>::T (&a)[1 << R],
-                                          const typename V2<Real>::T *__restrict__ state, const PassArgs &pa,
-                                          uint64_t base, uint32_t thr) {
-    using A2 = typename V2<Real>::T;
-    uint64_t off, rs[R];
-    thread_geometry<R, W>(pa.ld_gbit, thr, off, rs);
-    LoadF<A2, R> f{a, state + (base | off), rs};
-    Unroll<1 << R>::run(f);
-}
-
-template <typename Real, int R, int W>
-__device__ __forceinline__ void store_tile(const typename V2<Real>::T (&a)[1 << R],
-                                           typename V2<Real>::T *__restrict__ state, const PassArgs &pa,
-                                           uint64_t base, uint32_t xr) {
-    using A2 = typename V2<Real>::T;
-    // The thread index is re-read so the store geometry is recomputed here
-    // instead of being held in registers through every phase.
-    uint32_t thr;
-    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thr));
-    uint64_t off, rs[R];
-    thread_geometry<R, W>(pa.st_gbit, thr, off, rs);
-    uint64_t xo = 0;
-#pragma unroll
-    for (int q = 0; q < R; q++)
-        if ((xr >> q) & 1u) xo |= rs[q];
-    StoreF<A2, R> f{a, state, base | off | xo, rs};
-    Unroll<1 << R>::run(f);
-}
-
-// Applies a pass's phases to a tile already in registers (loaded in the
-// pass's load layout) and stores it.  `prev_cross`: the CTA's previous use
-// of `sm` may still be read by other warps, so the first transpose must
-// synchronise the CTA before writing.
+//
 // flags, norm_out, scale_in: the pass's PASS_* flags and renormalisation
-// slots (the plain pass kernel passes pa's own; the chained kernel computes
+// slots (the plain pass kernel passes ta's own; the chained kernel computes
 // them per position in the pass sequence).  The scale is read through L2:
 // in a chained run it was accumulated by other CTAs of the same launch.
-template <typename Real, int R, int W, bool LEAN = false>
+template <typename Real, int R, int W, bool LEAN>
 __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], typename V2<Real>::T *__restrict__ state,
-                                            const PassArgs &pa, uint64_t base, typename V2<Real>::T *sm,
-                                            bool prev_cross, int32_t flags, double *norm_out,
-                                            const double *scale_in) {
+                                            const TileArgs &ta, uint64_t base, unsigned char *sm, int32_t flags,
+                                            double *norm_out, const double *scale_in) {
     using A2 = typename V2<Real>::T;
-    constexpr uint32_t LS = LAYOUT_HDR + (32u << W);  // words per layout table
+    constexpr bool F64 = sizeof(Real) == 8;
     const uint32_t thr = threadIdx.x, lane = thr & 31;
-    const DevOp<Real> *__restrict__ ops = reinterpret_cast<const DevOp<Real> *>(pa.ops);
-    unsigned char *smb = reinterpret_cast<unsigned char *>(sm);
-    int cur = pa.load_layout;
+    unsigned char *win = sm + tile_smem_bytes<Real, R, W>();
     if (flags & PASS_SCALE) {
         const Real s = (Real)rsqrt(__ldcg(scale_in));
 #pragma unroll
@@ -1270,30 +1233,73 @@ __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], t
             a[r].y *= s;
         }
     }
-    uint32_t xr = 0;  // register relabeling (apply_op)
-    for (int p = pa.phase_begin; p < pa.phase_end; p++) {
-        const DevPhase ph = pa.phases[p];
-        if (ph.layout != cur) {
-            transpose<A2, R>(a, smb, thr, pa.layouts + cur * LS, pa.layouts + ph.layout * LS, prev_cross || ph.xwarp,
-                             ph.xwarp != 0, xr);
+    uint32_t tb = 0;
+#pragma unroll
+    for (int b = 0; b < 5 + W; b++) tb += ((thr >> b) & 1u) * ta.ld_tstep[b];
+    uint32_t xr = 0;            // register relabeling
+    uint32_t pc = 0;            // byte offset in the two windows
+    uint32_t next = ta.units0 + ta.units1;  // first unit not fetched yet
+    fetch_wait();
+    __syncthreads();
+    for (;;) {
+        const unsigned char *op = win + pc;
+        const uint4 hdr = *reinterpret_cast<const uint4 *>(op);
+        const uint32_t kind = hdr.x & 0xffu;
+        const Real *data = reinterpret_cast<const Real *>(op + 16);
+        pc += (hdr.x >> 8) << 4;
+        if (kind == (F64 ? S_ROT : S_SPLIT)) {
+            const uint32_t mask = hdr.y & 0xffu;
+            apply_split_layer<Real, A2, R>(a, data, mask, xr);
+            if (F64) xr ^= hdr.y >> 8;
+        } else if (kind == S_REAL || (F64 && kind == S_HAD)) {
+            const bool had = F64 && kind == S_HAD;
+            if (had && !__any_sync(0xffffffffu, (xr & hdr.y) != 0u)) {
+                if constexpr (F64) HadStep<Real, A2, R, 0>::run(a, hdr.y);
+            } else {
+                RealStep<Real, A2, R, 0>::run(a, data, hdr.y, xr, had);
+            }
+        } else if (kind == S_TRANS) {
+            transpose<A2, R, W>(a, sm, op, hdr, thr, tb, xr);
             xr = 0;
-            prev_cross = ph.xwarp != 0;
-            cur = ph.layout;
-        }
-        // (loading the next op's head record while this op runs costs more
-        // in registers than it saves in load latency)
-        for (int i = ph.op_begin; i < ph.op_end;) {
-            const uint4 hdr = __ldg(reinterpret_cast<const uint4 *>(ops + i));
-            apply_op<Real, A2, R, LEAN>(a, ops + i, hdr, base, thr, xr);
-            i += op_records(hdr);
+        } else if (kind == S_XSET) {
+            const int n = (int)hdr.y;
+            xr ^= xset_flip(hdr.z, base, thr);
+            if (n > 1) xr ^= xset_flip(hdr.w, base, thr);
+#pragma unroll 1
+            for (int j = 2; j < n; j++) xr ^= xset_flip(reinterpret_cast<const uint32_t *>(op)[2 + j], base, thr);
+        } else if (kind == S_CSWAP) {
+            CSwap<A2, R, 0>::run(hdr.y, a, hdr.z, hdr.w ^ (xr & hdr.z));
+        } else if (kind == S_PHASES) {
+            apply_phase_block_angles<Real, A2, R>(a, op, hdr, base, thr, xr);
+        } else if (F64 && kind == S_SCALE) {
+            const Real f = (Real)__hiloint2double((int)hdr.w, (int)hdr.z);
+#pragma unroll
+            for (int r = 0; r < (1 << R); r++) {
+                a[r].x *= f;
+                a[r].y *= f;
+            }
+        } else if (kind == S_GATE) {
+            apply_gate<Real, A2, R, LEAN>(a, op, hdr, base, thr, xr);
+        } else if (kind == S_NEXT) {
+            // the next window has been fetched; this one makes room for the
+            // window after it
+            fetch_wait();
+            __syncthreads();
+            const bool first = pc <= STREAM_WINDOW_BYTES;
+            if (hdr.y)
+                fetch_units(win + (first ? 0 : STREAM_WINDOW_BYTES), reinterpret_cast<const uint4 *>(ta.stream) + next,
+                            (int)hdr.y);
+            next += hdr.y;
+            pc = first ? STREAM_WINDOW_BYTES : 0;
+        } else if (!LEAN && kind == S_DENSE) {
+            DenseStep<Real, A2, R, 0>::run(a, data, hdr.y, xr);
+        } else if (!LEAN && kind == S_TERMS) {
+            apply_phase_block<Real, A2, R>(a, op, hdr, base, thr, xr);
+        } else {
+            break;  // S_END
         }
     }
-    if (cur != pa.store_layout) {
-        transpose<A2, R>(a, smb, thr, pa.layouts + cur * LS, pa.layouts + pa.store_layout * LS,
-                         prev_cross || pa.store_xwarp, pa.store_xwarp != 0, xr);
-        xr = 0;
-    }
-    store_tile<Real, R, W>(a, state, pa, base, xr);
+    store_tile<Real, R, W>(a, state, ta, base, xr);
     if (flags & PASS_NORM) {
         double acc = 0.0;
 #pragma unroll
@@ -1305,21 +1311,16 @@ __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], t
 }
 
 // Runs one pass over tile `tile`.  Shared by the plain pass kernel and the
-// batched persistent kernel.
-template <typename Real, int R, int W, bool LEAN = false>
-__device__ __forceinline__ void run_tile(typename V2<Real>::T *__restrict__ state, const PassArgs &pa, uint64_t tile,
-                                         typename V2<Real>::T *sm, int32_t flags, double *norm_out,
-                                         const double *scale_in) {
+// chained and batched persistent kernels; the first windows' copy has been
+// started.
+template <typename Real, int R, int W, bool LEAN>
+__device__ __forceinline__ void run_tile(typename V2<Real>::T *__restrict__ state, const TileArgs &ta, uint64_t tile,
+                                         unsigned char *sm, int32_t flags, double *norm_out, const double *scale_in) {
     using A2 = typename V2<Real>::T;
-    const uint64_t base = tile_base(tile, pa);
+    const uint64_t base = tile_base(tile, ta);
     A2 a[1 << R];
-    load_tile<Real, R, W>(a, state, pa, base, threadIdx.x);
-    finish_tile<Real, R, W, LEAN>(a, state, pa, base, sm, false, flags, norm_out, scale_in);
-}
-template <typename Real, int R, int W, bool LEAN = false>
-__device__ __forceinline__ void run_tile(typename V2<Real>::T *__restrict__ state, const PassArgs &pa, uint64_t tile,
-                                         typename V2<Real>::T *sm) {
-    run_tile<Real, R, W, LEAN>(state, pa, tile, sm, pa.flags, pa.norm_out, pa.scale_in);
+    load_tile<Real, R, W>(a, state, ta, base, threadIdx.x);
+    finish_tile<Real, R, W, LEAN>(a, state, ta, base, sm, flags, norm_out, scale_in);
 }
 
 }  // namespace hgm

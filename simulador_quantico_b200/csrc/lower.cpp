@@ -1,0 +1,379 @@
+// Lowering: a plan's passes -> the device stream the kernels run.
+//
+// The planner's records (hgm_internal.h DevOp) say what a pass does; this
+// file writes it in the form that costs the pass kernel least:
+//   * one linear stream per pass, ops and transposes in the order they run,
+//     16 to 32 bytes a gate instead of 80 to 112, so that a window of it fits
+//     beside the transpose buffer in shared memory;
+//   * FP64 rotations and Hadamards without their common factor (cos or
+//     1/sqrt 2), which leaves half the operations of the real 2x2 out; the
+//     factors multiply into one S_SCALE at the plan's end (or when they leave
+//     [2^-200, 2^200]).  28 qubits, 10 layers, FP64: 67.0 -> 50.1 ms with the
+//     stream; 26-qubit search, 32 iterations: 78.7 -> 60.2 ms.  FP32 keeps the plain form: its results stay, bit by
+//     bit, those of the records.
+#include <cmath>
+#include <cstring>
+
+#include "hgm_internal.h"
+
+namespace hgm {
+
+namespace {
+
+struct Rot {
+    double kappa;   // factor left out
+    double t, u, pr, pi;
+    bool x;         // an X follows
+};
+
+// Writes a real orthogonal matrix (up to a factor) with a phase before it,
+//   M = Rm diag(1, p),   Rm = h [[c, -d s], [s, d c]],  d = +-1,
+// as kappa X^x R(t) diag(1, e p) with |t| <= 1, e = +-1 and
+// R(t) = [[1, -t], [t, 1]]: t = s / c, or (with an X behind) c / s.  The
+// kernel runs R(t) diag(1, e p) in place with two multiply-adds a component,
+//   y' = ((1 + t^2) e p) y,   x1 = x + u y',   y1 = y' + t x1,
+//   u = -t / (1 + t^2),
+// the factor 1 + t^2 riding on the phase.  m: Rm row-major.  False when Rm is
+// not of that form (a gate that is not unitary up to a factor).
+bool make_rot(const double *m, double p_re, double p_im, Rot &r) {
+    double big = 0.0;
+    for (int k = 0; k < 4; k++) big = std::max(big, std::abs(m[k]));
+    const double d = m[0] * m[3] - m[1] * m[2] >= 0.0 ? 1.0 : -1.0;
+    const double tol = 4e-15 * big;
+    if (!(std::abs(m[3] - d * m[0]) <= tol && std::abs(m[2] + d * m[1]) <= tol)) return false;
+    const double c = 0.5 * (m[0] + d * m[3]), s = 0.5 * (m[2] - d * m[1]);
+    if (!std::isfinite(c) || !std::isfinite(s) || (c == 0.0 && s == 0.0)) return false;
+    r.x = std::abs(s) > std::abs(c);
+    const double num = r.x ? c : s, den = r.x ? s : c, e = r.x ? -d : d;
+    r.t = num / den;
+    const double sq = 1.0 + r.t * r.t;
+    r.kappa = den;
+    r.u = -r.t / sq;
+    r.pr = e * p_re * sq;
+    r.pi = e * p_im * sq;
+    return true;
+}
+
+// The factor a of a [[1, 1], [1, -1]], or 0.
+double hadamard_factor(const double *m) {
+    const double a = 0.25 * (m[0] + m[1] + m[2] - m[3]), tol = 4e-16 * std::abs(a);
+    const bool ok = std::isfinite(a) && std::abs(m[0] - a) <= tol && std::abs(m[1] - a) <= tol &&
+                    std::abs(m[2] - a) <= tol && std::abs(m[3] + a) <= tol;
+    return ok ? a : 0.0;
+}
+
+template <typename Real>
+struct Lowering {
+    Plan *plan;
+    const cplx global;
+    const int R, W;
+    double scale = 1.0;      // factors left out and not yet applied
+    // the current pass: its windows' units
+    std::vector<uint32_t> out;
+    std::vector<uint32_t> window;
+    std::vector<size_t> windows;   // units of each finished window
+    static constexpr size_t CAP = STREAM_WINDOW_UNITS - 1;  // one unit for S_NEXT or S_END
+
+    Lowering(Plan *p, cplx gl) : plan(p), global(gl), R(p->reg_bits), W(p->warp_bits) {}
+
+    static void put_real(std::vector<uint32_t> &v, Real x) {
+        uint32_t w[2] = {0, 0};
+        memcpy(w, &x, sizeof(Real));
+        v.push_back(w[0]);
+        if (sizeof(Real) == 8) v.push_back(w[1]);
+    }
+    static void put_u64(std::vector<uint32_t> &v, uint64_t x) {
+        v.push_back((uint32_t)x);
+        v.push_back((uint32_t)(x >> 32));
+    }
+
+    // Ends the current window with S_NEXT (its w1 is set when the windows are known).
+    void flush(uint32_t kind) {
+        window.insert(window.end(), {kind | (1u << 8), 0u, 0u, 0u});
+        windows.push_back(window.size() / 4);
+        out.insert(out.end(), window.begin(), window.end());
+        window.clear();
+    }
+    // Adds one op (whole units; word 0's unit count is set here).
+    void add(uint32_t kind, std::vector<uint32_t> op) {
+        while (op.size() % 4) op.push_back(0);
+        const size_t units = op.size() / 4;
+        op[0] = kind | (uint32_t)(units << 8);
+        if (window.size() / 4 + units > CAP) flush(S_NEXT);
+        window.insert(window.end(), op.begin(), op.end());
+    }
+    void add_scale() {
+        if (scale == 1.0) return;  // FP32: always
+        std::vector<uint32_t> op = {0u, 0u};
+        put_real(op, (Real)scale);
+        add(S_SCALE, op);
+        scale = 1.0;
+    }
+    void left_out(double kappa) {
+        scale *= kappa;
+        const double a = std::abs(scale);
+        if (!(a < 0x1p200 && a > 0x1p-200)) add_scale();
+    }
+
+    uint32_t slot(uint32_t j) const { return (j + (j >> R)) * (uint32_t)(2 * sizeof(Real)); }
+    uint32_t reg_step(const Lay &l, int q) const { return q < R ? slot(1u << l.pos[5 + W + q]) : 0u; }
+    uint32_t thread_step(const Lay &l, int b) const { return b < 5 + W ? slot(1u << l.pos[b]) : 0u; }
+
+    void transpose(int from, int to, bool before, bool cross) {
+        const Lay &f = plan->layouts[from], &t = plan->layouts[to];
+        std::vector<uint32_t> op = {0u, (before ? STREAM_SYNC_BEFORE : 0u) | (cross ? STREAM_SYNC_CROSS : 0u),
+                                    reg_step(f, 4), reg_step(t, 4)};
+        for (int q = 0; q < 4; q++) op.push_back(reg_step(f, q));
+        for (int q = 0; q < 4; q++) op.push_back(reg_step(t, q));
+        for (int b = 0; b < 8; b++) op.push_back(thread_step(t, b));
+        add(S_TRANS, op);
+    }
+
+    void gate(const DevOp<Real> &d) {
+        if (d.kind == K_SWAP && d.tpos < R && !d.cm_thr && !d.cm_glob && d.cm_reg) {
+            add(S_CSWAP, {0u, (uint32_t)d.tpos, d.cm_reg, d.cv_reg});
+            return;
+        }
+        std::vector<uint32_t> op = {0u, (uint32_t)d.kind | ((uint32_t)d.tpos << 8), d.cm_reg, d.cv_reg,
+                                    d.cm_thr, d.cv_thr, 0u, 0u};
+        put_u64(op, d.cm_glob);
+        put_u64(op, d.cv_glob);
+        if (d.kind != K_SWAP)
+            for (int k = 0; k < 8; k++) put_real(op, d.m[k]);
+        add(S_GATE, op);
+    }
+
+    // A layer of real or split gates: mats[k] is the record of the k-th bit of the mask.
+    void layer(const DevOp<Real> &head, const DevOp<Real> *mats) {
+        const uint32_t mask = head.cm_reg;
+        const int n = __builtin_popcount(mask);
+        const bool split = head.kind == K_LAYER_SPLIT;
+        if (sizeof(Real) == 4) {
+            std::vector<uint32_t> op = {0u, mask, 0u, 0u};
+            for (int i = 0; i < n; i++) {
+                for (int j = 0; j < 4; j++) put_real(op, mats[i].m[split ? j : 2 * j]);
+                if (split)
+                    for (Real v : {mats[i].m[4], mats[i].m[5], (Real)0, (Real)0}) put_real(op, v);
+            }
+            add(split ? S_SPLIT : S_REAL, op);
+            return;
+        }
+        std::vector<int> bit;
+        for (int b = 0; b < R; b++)
+            if ((mask >> b) & 1u) bit.push_back(b);
+        std::vector<uint32_t> rot = {0u, mask, 0u, 0u}, had = {0u, 0u, 0u, 0u}, real = {0u, 0u, 0u, 0u};
+        double factor = 1.0;
+        bool all_rot = split;
+        for (int i = 0; i < n && all_rot; i++) {
+            const Real *m = mats[i].m;
+            const double rm[4] = {(double)m[0], (double)m[1], (double)m[2], (double)m[3]};
+            Rot r;
+            all_rot = make_rot(rm, (double)m[4], (double)m[5], r);
+            if (!all_rot) break;
+            if (r.x) rot[1] |= 1u << (8 + bit[i]);
+            for (double v : {r.t, r.u, r.pr, r.pi}) put_real(rot, (Real)v);
+            factor *= r.kappa;
+        }
+        if (all_rot) {
+            add(S_ROT, rot);
+            left_out(factor);
+            return;
+        }
+        factor = 1.0;
+        for (int i = 0; i < n; i++) {
+            const Real *m = mats[i].m;
+            const double rm[4] = {(double)m[0], (double)m[split ? 1 : 2], (double)m[split ? 2 : 4], (double)m[split ? 3 : 6]};
+            if (split && (m[4] != (Real)1 || m[5] != (Real)0)) {  // the phase, then the real matrix
+                DevOp<Real> d;
+                memset(&d, 0, sizeof d);
+                d.kind = K_PHASE;
+                d.tpos = bit[i];
+                d.m[0] = (Real)1;
+                d.m[6] = m[4];
+                d.m[7] = m[5];
+                gate(d);
+            }
+            const double a = hadamard_factor(rm);
+            if (a != 0.0) {
+                had[1] |= 1u << bit[i];
+                factor *= a;
+            } else {
+                real[1] |= 1u << bit[i];
+                for (double v : rm) put_real(real, (Real)v);
+            }
+        }
+        if (had[1]) {
+            add(S_HAD, had);
+            left_out(factor);
+        }
+        if (real[1]) add(S_REAL, real);
+    }
+
+    // The parts of a phase block: its terms by category in the kernel's walk
+    // order (F, then G, H, D of each register bit), `per` units each, and its
+    // table.  A block too large for a window goes out as several (each a
+    // block of its own: factors multiply), the table with the last.
+    int phase_block(const DevOp<Real> *rec) {
+        const DevOp<Real> &head = rec[0];
+        const bool angles = head.cm_reg & PB_ANGLES;
+        uint8_t counts[16];
+        memcpy(counts, head.m, 16);
+        std::vector<int> order = {0};
+        for (int b = 0; b < R; b++)
+            for (int c : {1 + b, 1 + R + b, 1 + 2 * R + b}) order.push_back(c);
+        const int total_terms = [&] {
+            int t = 0;
+            for (int c : order) t += counts[c];
+            return t;
+        }();
+        // the terms' words, in walk order
+        constexpr int per = pb_terms_per_record<Real>();
+        const int tu = angles ? (int)sizeof(PhaseTerm<Real>) / 16 : 2 + (sizeof(Real) == 8 ? 2 : 1);
+        std::vector<std::vector<uint32_t>> terms;
+        for (int k = 0; k < total_terms; k++) {
+            std::vector<uint32_t> t;
+            if (angles) {
+                t.resize(sizeof(PhaseTerm<Real>) / 4);
+                memcpy(t.data(), reinterpret_cast<const unsigned char *>(rec + 1 + k / per) + (k % per) * sizeof(PhaseTerm<Real>),
+                       sizeof(PhaseTerm<Real>));
+            } else {
+                const DevOp<Real> &d = rec[1 + k];
+                t = {d.cm_thr, d.cv_thr, (uint32_t)d.tpos2, 0u};
+                put_u64(t, d.cm_glob);
+                put_u64(t, d.cv_glob);
+                for (int j : {0, 1, 6, 7}) put_real(t, d.m[j]);
+            }
+            terms.push_back(t);
+        }
+        const int nrec = head.tpos;
+        const bool table = head.cm_reg & PB_HAS_TABLE;
+        const int tab_units = table ? (int)((size_t(1) << R) * 2 * sizeof(Real) / 16) : 0;
+        const int fit = ((int)CAP - 3 - tab_units) / tu;
+        int done = 0;
+        do {
+            const int take = std::min(fit, total_terms - done);
+            const bool last = done + take == total_terms;
+            uint8_t cnt[16] = {0};
+            uint32_t act = 0;
+            int at = 0;
+            for (int c : order) {
+                for (int j = 0; j < counts[c]; j++, at++) {
+                    if (at < done || at >= done + take) continue;
+                    cnt[c]++;
+                    act |= c == 0 ? PB_F_ACTIVE : 1u << ((c - 1) % R);
+                }
+            }
+            uint32_t flags = head.cm_reg;
+            if (!(last && done == 0)) flags &= ~PB_GATED;
+            if (!last) flags &= ~PB_HAS_TABLE;
+            const bool tab = last && table;
+            std::vector<uint32_t> op = {0u, flags, act, tab ? (uint32_t)(3 + take * tu) : 0u};
+            op.resize(12);
+            memcpy(&op[4], cnt, 16);
+            memcpy(&op[8], reinterpret_cast<const unsigned char *>(head.m) + 16, 8);
+            for (int k = done; k < done + take; k++) op.insert(op.end(), terms[k].begin(), terms[k].end());
+            if (tab)
+                for (int r = 0; r < (1 << R); r++) {
+                    const DevOp<Real> &z = rec[1 + nrec - (1 << R) / 4 + r / 4];
+                    put_real(op, z.m[2 * (r & 3)]);
+                    put_real(op, z.m[2 * (r & 3) + 1]);
+                }
+            add(angles ? S_PHASES : S_TERMS, op);
+            done += take;
+        } while (done < total_terms);
+        return 1 + nrec;
+    }
+
+    void pass(const PassArgs &pa, const DevOp<Real> *ops, size_t n_ops, bool last_pass) {
+        out.clear();
+        window.clear();
+        windows.clear();
+        int cur = pa.load_layout;
+        bool prev_cross = false;
+        for (int p = pa.phase_begin; p < pa.phase_end; p++) {
+            const DevPhase &ph = plan->phases[p];
+            if (ph.layout != cur) {
+                transpose(cur, ph.layout, prev_cross || ph.xwarp, ph.xwarp != 0);
+                prev_cross = ph.xwarp != 0;
+                cur = ph.layout;
+            }
+            for (int i = ph.op_begin; i < ph.op_end;) {
+                const DevOp<Real> &d = ops[i];
+                if (d.kind == K_PHASE_BLOCK) {
+                    i += phase_block(ops + i);
+                } else if (d.kind == K_LAYER_REAL || d.kind == K_LAYER_SPLIT) {
+                    layer(d, ops + i + 1);
+                    i += 1 + __builtin_popcount(d.cm_reg);
+                } else if (d.kind == K_LAYER) {
+                    const int k = __builtin_popcount(d.cm_reg);
+                    std::vector<uint32_t> op = {0u, d.cm_reg, 0u, 0u};
+                    for (int j = 0; j < k; j++)
+                        for (int e = 0; e < 8; e++) put_real(op, ops[i + 1 + j].m[e]);
+                    add(S_DENSE, op);
+                    i += 1 + k;
+                } else if (d.kind == K_XSET) {
+                    std::vector<uint32_t> op = {0u, (uint32_t)d.tpos};
+                    op.resize(2 + d.tpos);
+                    memcpy(&op[2], d.m, 4 * (size_t)d.tpos);
+                    add(S_XSET, op);
+                    i++;
+                } else if (last_pass && i + 1 == (int)n_ops && global != 1.0) {
+                    // the plan's scalar takes the factors left out with it
+                    DevOp<Real> e = d;
+                    const cplx z = global * scale;
+                    e.m[0] = e.m[6] = (Real)z.real();
+                    e.m[1] = e.m[7] = (Real)z.imag();
+                    scale = 1.0;
+                    gate(e);
+                    i++;
+                } else {
+                    gate(d);
+                    i++;
+                }
+            }
+        }
+        if (last_pass) add_scale();
+        if (cur != pa.store_layout)
+            transpose(cur, pa.store_layout, prev_cross || pa.store_xwarp, pa.store_xwarp != 0);
+        flush(S_END);
+
+        TileArgs t;
+        memset(&t, 0, sizeof t);
+        t.stream = reinterpret_cast<const void *>(plan->stream.size() * 4);
+        t.units0 = (int32_t)windows[0];
+        t.units1 = windows.size() > 1 ? (int32_t)windows[1] : 0;
+        // every S_NEXT names the units of the window after the one it enters
+        size_t end = 0;
+        for (size_t w = 0; w < windows.size(); w++) {
+            end += windows[w];
+            if (w + 2 < windows.size()) out[4 * (end - 1) + 1] = (uint32_t)windows[w + 2];
+        }
+        plan->stream.insert(plan->stream.end(), out.begin(), out.end());
+        t.n = pa.n;
+        t.k = pa.k;
+        t.nruns = pa.nruns;
+        memcpy(t.run_pos, pa.run_pos, sizeof t.run_pos);
+        memcpy(t.run_len, pa.run_len, sizeof t.run_len);
+        memcpy(t.ld_gbit, pa.ld_gbit, sizeof t.ld_gbit);
+        memcpy(t.st_gbit, pa.st_gbit, sizeof t.st_gbit);
+        for (int b = 0; b < 8; b++) t.ld_tstep[b] = thread_step(plan->layouts[pa.load_layout], b);
+        plan->tiles.push_back(t);
+    }
+
+    void run() {
+        const DevOp<Real> *ops = reinterpret_cast<const DevOp<Real> *>(plan->ops_bytes.data());
+        const size_t n_ops = plan->ops_bytes.size() / sizeof(DevOp<Real>);
+        for (size_t p = 0; p < plan->passes.size(); p++) pass(plan->passes[p], ops, n_ops, p + 1 == plan->passes.size());
+    }
+};
+
+}  // namespace
+
+void lower_plan(Plan *plan, cplx global) {
+    plan->stream.clear();
+    plan->tiles.clear();
+    if (plan->precision == HGM_F64) Lowering<double>(plan, global).run();
+    else Lowering<float>(plan, global).run();
+}
+
+}  // namespace hgm

@@ -1015,6 +1015,7 @@ int build_tiled(const std::vector<SOp> &ops, int n, const hgm_plan_opts &o, Plan
     plan->lean = lean_ops<Real>(dev_ops, R);
     plan->ops_bytes.resize(dev_ops.size() * sizeof(DevOp<Real>));
     if (!dev_ops.empty()) memcpy(plan->ops_bytes.data(), dev_ops.data(), plan->ops_bytes.size());
+    lower_plan(plan, global);
     return HGM_OK;
 }
 

@@ -135,8 +135,9 @@ class Plan:
         passes = C.c_void_p()
         check(lib.hgm_plan_export(self.h, C.byref(passes), C.byref(npa), None, C.byref(nph), None, C.byref(nb),
                                   C.byref(wb), C.byref(small)))
-        # bytes copied to the device when the plan is created: op records and phase table
-        upload = nb.value + 16 * nph.value
+        # bytes copied to the device when the plan is uploaded: the passes' streams
+        check(lib.hgm_plan_stream(self.h, None, C.byref(nb)))
+        upload = nb.value
         # register bits from the first pass's tile bits (struct PassArgs: n, k, ...): k = 5 + R + W
         reg_bits = 4 if self.precision == HGM_F64 else 5
         if npa.value and passes.value:
