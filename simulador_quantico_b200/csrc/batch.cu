@@ -26,7 +26,7 @@
 
 namespace hgm {
 
-struct BatchTask {
+struct alignas(16) BatchTask {
     TileArgs pa;            // pass arguments (tiled tasks)
     void *state;            // the circuit's state in the batch arena
     long long tile_begin;   // first global item of this task
@@ -54,103 +54,127 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
     return v;
 }
 
+// A whole small circuit in shared memory.  Its gates come through the stream
+// windows (`win`), as many at a time as fit: a gate read from global memory
+// costs an L2 round trip, more than its arithmetic.
 template <typename Real>
 __device__ __forceinline__ void small_task(typename V2<Real>::T *__restrict__ state, int n,
                                            const SmallOp<Real> *__restrict__ ops, long long n_ops,
-                                           typename V2<Real>::T *sm) {
+                                           typename V2<Real>::T *sm, unsigned char *win) {
     using A2 = typename V2<Real>::T;
+    static_assert(sizeof(SmallOp<Real>) % 16 == 0, "fetched as units");
+    constexpr int CHUNK = 2 * STREAM_WINDOW_BYTES / (int)sizeof(SmallOp<Real>);
     const int N = 1 << n, half = N >> 1;
     for (int i = threadIdx.x; i < N; i += blockDim.x) sm[i] = __ldcg(state + i);
-    __syncthreads();
-    for (long long k = 0; k < n_ops; k++) {
-        const SmallOp<Real> &o = ops[k];
-        const int t = o.target;
-        const uint32_t cm = o.cmask, cv = o.cval;
-        const Real m0r = o.m[0], m0i = o.m[1], m1r = o.m[2], m1i = o.m[3];
-        const Real m2r = o.m[4], m2i = o.m[5], m3r = o.m[6], m3i = o.m[7];
-        for (int p = threadIdx.x; p < half; p += blockDim.x) {
-            const int i0 = ((p >> t) << (t + 1)) | (p & ((1 << t) - 1));
-            const int i1 = i0 | (1 << t);
-            if (((uint32_t)i0 & cm) != cv) continue;
-            const A2 x = sm[i0], y = sm[i1];
-            A2 o0, o1;
-            o0.x = m0r * x.x - m0i * x.y + m1r * y.x - m1i * y.y;
-            o0.y = m0r * x.y + m0i * x.x + m1r * y.y + m1i * y.x;
-            o1.x = m2r * x.x - m2i * x.y + m3r * y.x - m3i * y.y;
-            o1.y = m2r * x.y + m2i * x.x + m3r * y.y + m3i * y.x;
-            sm[i0] = o0;
-            sm[i1] = o1;
-        }
+    for (long long k0 = 0; k0 < n_ops; k0 += CHUNK) {
+        const int count = (int)(n_ops - k0 < CHUNK ? n_ops - k0 : CHUNK);
+        fetch_units(win, reinterpret_cast<const uint4 *>(ops + k0), count * (int)(sizeof(SmallOp<Real>) / 16));
+        fetch_wait();
         __syncthreads();
+        for (int k = 0; k < count; k++) {
+            const SmallOp<Real> &o = reinterpret_cast<const SmallOp<Real> *>(win)[k];
+            const int t = o.target;
+            const uint32_t cm = o.cmask, cv = o.cval;
+            const Real m0r = o.m[0], m0i = o.m[1], m1r = o.m[2], m1i = o.m[3];
+            const Real m2r = o.m[4], m2i = o.m[5], m3r = o.m[6], m3i = o.m[7];
+            for (int p = threadIdx.x; p < half; p += blockDim.x) {
+                const int i0 = ((p >> t) << (t + 1)) | (p & ((1 << t) - 1));
+                const int i1 = i0 | (1 << t);
+                if (((uint32_t)i0 & cm) != cv) continue;
+                const A2 x = sm[i0], y = sm[i1];
+                A2 o0, o1;
+                o0.x = m0r * x.x - m0i * x.y + m1r * y.x - m1i * y.y;
+                o0.y = m0r * x.y + m0i * x.x + m1r * y.y + m1i * y.x;
+                o1.x = m2r * x.x - m2i * x.y + m3r * y.x - m3i * y.y;
+                o1.y = m2r * x.y + m2i * x.x + m3r * y.y + m3i * y.x;
+                sm[i0] = o0;
+                sm[i1] = o1;
+            }
+            __syncthreads();
+        }
     }
     for (int i = threadIdx.x; i < N; i += blockDim.x) __stcg(state + i, sm[i]);
 }
 
-template <typename Real, int R, int W>
+// LEAN: every plan of the batch runs on the lean build (kernels.cuh finish_tile).
+template <typename Real, int R, int W, bool LEAN>
 __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()))
     batch_kernel(const BatchTask *__restrict__ tasks, int ntasks, long long total_items,
                  unsigned long long *next_item, unsigned int *done, int *error) {
     using A2 = typename V2<Real>::T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     A2 *sm = reinterpret_cast<A2 *>(smem_raw);
-    __shared__ long long s_item;
-    __shared__ int s_task;
+    unsigned char *win = smem_raw + tile_smem_bytes<Real, R, W>();
+    __shared__ long long s_next;
+    __shared__ int s_next_task;
     __shared__ int s_skip;
-    // the item's pass arguments, copied once per item into shared memory (the
-    // tile code reads them many times; chained kernel, kernels.cu)
+    // the item's pass arguments: the tile code reads them many times
     __shared__ __align__(16) TileArgs s_ta;
-    for (;;) {
+    // Claims an item and finds its task.
+    auto claim = [&]() {
+        const long long it = (long long)atomicAdd(next_item, 1ull);
+        int lo = 0, hi = ntasks - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(&tasks[mid].tile_begin) <= it) lo = mid;
+            else hi = mid - 1;
+        }
+        s_next = it;
+        s_next_task = lo;
+    };
+    auto fetch_args = [&](TileArgs *dst, int task) {
+        fetch_units(reinterpret_cast<unsigned char *>(dst), reinterpret_cast<const uint4 *>(&tasks[task].pa),
+                    (int)(sizeof(TileArgs) / 16));
+    };
+    // one thread claims the next item and finds its task while another
+    // publishes this one
+    if (threadIdx.x == 0) claim();
+    __syncthreads();
+    long long it = s_next;
+    int task = s_next_task;
+    while (it < total_items) {
+        const BatchTask &t = tasks[task];
+        const bool tiled = !t.small;
+        if (tiled) fetch_args(&s_ta, task);
         if (threadIdx.x == 0) {
-            const long long it = (long long)atomicAdd(next_item, 1ull);
-            s_item = it;
-            s_skip = 0;
-            if (it < total_items) {
-                int lo = 0, hi = ntasks - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (tasks[mid].tile_begin <= it) lo = mid;
-                    else hi = mid - 1;
-                }
-                s_task = lo;
-                const int dep = tasks[lo].dep;
-                if (dep >= 0) {
-                    const unsigned int need = tasks[lo].dep_need;
-                    const unsigned long long limit = tasks[lo].wait_ns;
-                    const unsigned long long t0 = global_ns();
-                    while (ld_acquire(&done[dep]) < need) {
+            int skip = 0;
+            if (t.dep >= 0) {
+                const unsigned int need = t.dep_need;
+                if (ld_acquire(&done[t.dep]) < need) {
+                    const unsigned long long limit = t.wait_ns, t0 = global_ns();
+                    while (ld_acquire(&done[t.dep]) < need) {
                         if (global_ns() - t0 > limit) {
                             atomicExch(error, 1);
-                            s_skip = 1;
+                            skip = 1;
                             break;
                         }
-                        __nanosleep(128);
+                        __nanosleep(64);
                     }
                 }
             }
+            s_skip = skip;
         }
+        fetch_wait();
         __syncthreads();
-        const long long it = s_item;
-        if (it >= total_items) break;
-        const BatchTask &t = tasks[s_task];
         if (!s_skip) {
-            if (t.small) {
-                small_task<Real>(reinterpret_cast<A2 *>(t.state), t.n,
-                                 reinterpret_cast<const SmallOp<Real> *>(t.small_ops), t.n_small_ops, sm);
+            if (tiled) {
+                fetch_stream(win, s_ta);
+                run_tile<Real, R, W, LEAN>(reinterpret_cast<A2 *>(t.state), s_ta, (uint64_t)(it - t.tile_begin),
+                                           smem_raw, 0, nullptr, nullptr);
             } else {
-                const uint32_t *src = reinterpret_cast<const uint32_t *>(&t.pa);
-                uint32_t *dst = reinterpret_cast<uint32_t *>(&s_ta);
-                for (int w = threadIdx.x; w < (int)(sizeof(TileArgs) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
-                __syncthreads();
-                fetch_stream(smem_raw + tile_smem_bytes<Real, R, W>(), s_ta);
-                run_tile<Real, R, W, false>(reinterpret_cast<A2 *>(t.state), s_ta, (uint64_t)(it - t.tile_begin),
-                                            smem_raw, 0, nullptr, nullptr);
+                small_task<Real>(reinterpret_cast<A2 *>(t.state), t.n,
+                                 reinterpret_cast<const SmallOp<Real> *>(t.small_ops), t.n_small_ops, sm, win);
             }
         }
         __syncthreads();
+        if (threadIdx.x == blockDim.x - 1) claim();
         if (threadIdx.x == 0) {
             __threadfence();
-            atomicAdd(&done[s_task], 1u);
+            atomicAdd(&done[task], 1u);
         }
+        __syncthreads();
+        it = s_next;
+        task = s_next_task;
     }
 }
 
@@ -195,6 +219,7 @@ struct Batch {
     long long *d_offsets = nullptr, *d_init = nullptr;
     int grid = 0;
     int smem = 0;
+    bool lean = false;      // every tiled plan runs on the lean build
     cudaGraphExec_t graph = nullptr;
     cudaStream_t stream = nullptr;
     std::vector<State> views;
@@ -225,36 +250,40 @@ struct Batch {
 
 namespace {
 
-template <typename Real, int R, int W>
+template <typename Real, int R, int W, bool LEAN>
 int batch_setup(Batch *b) {
     const int smem = cta_smem_bytes<Real, R, W>();
-    cudaError_t e = cudaFuncSetAttribute(batch_kernel<Real, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(batch_kernel<Real, R, W, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(HGM_ERR_CUDA, "batch kernel attribute: %s", cudaGetErrorString(e));
     int per_sm = 0, dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<Real, R, W>, 32 << W, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<Real, R, W, LEAN>, 32 << W, smem);
     if (e != cudaSuccess || per_sm < 1) return fail(HGM_ERR_CUDA, "batch kernel occupancy: %s", cudaGetErrorString(e));
     b->grid = sms * per_sm;
     b->smem = smem;
     return HGM_OK;
 }
 
-template <typename Real, int R, int W>
+template <typename Real, int R, int W, bool LEAN>
 void batch_launch(Batch *b, cudaStream_t st) {
-    batch_kernel<Real, R, W><<<b->grid, 32 << W, b->smem, st>>>(b->d_tasks, (int)b->tasks.size(), b->total_items,
+    batch_kernel<Real, R, W, LEAN><<<b->grid, 32 << W, b->smem, st>>>(b->d_tasks, (int)b->tasks.size(), b->total_items,
                                                                  b->d_next, b->d_done, b->d_error);
 }
 
-template <typename Real>
-int batch_dispatch(Batch *b, bool setup, cudaStream_t st) {
+template <typename Real, bool LEAN>
+int batch_dispatch_w(Batch *b, bool setup, cudaStream_t st) {
     constexpr int R = sizeof(Real) == 8 ? HGM_F64_REG_BITS : HGM_F32_REG_BITS;
     switch (b->warp_bits) {
-        case 0: return setup ? batch_setup<Real, R, 0>(b) : (batch_launch<Real, R, 0>(b, st), HGM_OK);
-        case 1: return setup ? batch_setup<Real, R, 1>(b) : (batch_launch<Real, R, 1>(b, st), HGM_OK);
-        case 2: return setup ? batch_setup<Real, R, 2>(b) : (batch_launch<Real, R, 2>(b, st), HGM_OK);
-        default: return setup ? batch_setup<Real, R, 3>(b) : (batch_launch<Real, R, 3>(b, st), HGM_OK);
+        case 0: return setup ? batch_setup<Real, R, 0, LEAN>(b) : (batch_launch<Real, R, 0, LEAN>(b, st), HGM_OK);
+        case 1: return setup ? batch_setup<Real, R, 1, LEAN>(b) : (batch_launch<Real, R, 1, LEAN>(b, st), HGM_OK);
+        case 2: return setup ? batch_setup<Real, R, 2, LEAN>(b) : (batch_launch<Real, R, 2, LEAN>(b, st), HGM_OK);
+        default: return setup ? batch_setup<Real, R, 3, LEAN>(b) : (batch_launch<Real, R, 3, LEAN>(b, st), HGM_OK);
     }
+}
+template <typename Real>
+int batch_dispatch(Batch *b, bool setup, cudaStream_t st) {
+    return b->lean ? batch_dispatch_w<Real, true>(b, setup, st) : batch_dispatch_w<Real, false>(b, setup, st);
 }
 
 int cuda_err(cudaError_t e, const char *what) {
@@ -270,6 +299,7 @@ int batch_finalize(Batch *b) {
     const size_t amp = b->precision == HGM_F64 ? 16 : 8;
     // plans and arena layout
     long long off = 0;
+    bool lean = true;
     for (BatchJob &j : b->jobs) {
         hgm_plan_opts o;
         hgm_plan_default_opts(&o, b->precision);
@@ -286,7 +316,9 @@ int batch_finalize(Batch *b) {
         if (rc) return rc;
         j.offset = off;
         off += 1ll << j.n;
+        lean = lean && (j.plan->small || j.plan->lean);
     }
+    b->lean = lean;
     b->arena_bytes = (size_t)off * amp;
     int rc = cuda_err(cudaMalloc(&b->arena, b->arena_bytes), "batch arena");
     if (rc) return rc;

@@ -268,8 +268,14 @@ enum StreamKind : uint32_t {
 };
 constexpr uint32_t STREAM_SYNC_BEFORE = 1, STREAM_SYNC_CROSS = 2;
 
-// A pass as the kernels take it.
-struct TileArgs {
+// A pass as the kernels take it.  The byte arrays are read 16 bytes at a time.
+constexpr int TILE_RUNS = 16;  // a tile of at most 13 bits leaves at most 14 runs
+struct alignas(16) TileArgs {
+    int8_t ld_gbit[MAX_LAYOUT_ROLES];  // global index bit of every role of the load and store layouts
+    int8_t st_gbit[MAX_LAYOUT_ROLES];
+    int8_t run_pos[TILE_RUNS];         // the non-tile index bits as runs (PassArgs)
+    int8_t run_len[TILE_RUNS];
+    uint32_t ld_tstep[8];   // load layout: byte step of each thread bit in the transpose buffer
     const void *stream;     // first window, then the others back to back
     int32_t units0, units1; // units of the first two windows
     int32_t n, k;
@@ -277,13 +283,8 @@ struct TileArgs {
     int32_t nruns;
     double *norm_out;
     const double *scale_in;
-    int8_t run_pos[MAX_FREE_RUNS];
-    int8_t run_len[MAX_FREE_RUNS];
-    int8_t ld_gbit[MAX_LAYOUT_ROLES];
-    int8_t st_gbit[MAX_LAYOUT_ROLES];
-    uint32_t ld_tstep[8];   // load layout: byte step of each thread bit in the transpose buffer
 };
-static_assert(sizeof(TileArgs) % 4 == 0, "copied as words");
+static_assert(sizeof(TileArgs) % 16 == 0, "copied as 16-byte units");
 
 // Small-state path (n < 5 + R): whole state in one CTA's shared memory, ops
 // applied one at a time.

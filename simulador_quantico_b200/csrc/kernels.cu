@@ -239,14 +239,24 @@ int64_t plan_launches(const Plan *p, int iterations) {
 // one launch.  Its CTAs claim work items (pass g, tile t) in sequence order
 // from a counter, and the CTA that claimed an item of pass g waits until
 // every item of passes 0..g-1 is done (a second counter) before it loads.
+//
+// Between two passes a CTA only waits for what the next pass needs: one thread
+// claims the next item while another publishes this one, and the arguments and
+// the stream of the pass the CTA will probably run next (it takes every
+// stride-th item when no other kernel is in the way) are fetched before its
+// item is known.  (Claiming an item ahead does the same, but holds it back
+// from idle CTAs: the serving mix, whose launches share the SMs, lost 5%.)
 // An item only waits for items claimed before it, and a claimed item is held
 // by a running CTA, so the sequence always progresses whether or not all of
-// the grid is resident.  The wait is bounded (2 s of %globaltimer); a CTA
-// that gives up sets the error word and skips its tile.
+// the grid is resident.  The wait is bounded (2 s of %globaltimer); a CTA that
+// gives up sets the error word and skips its tile.
 //
-// Scratch (Plan::d_chain): claim counter, done counter, error word, one
-// unused word, then CHAIN_NORM_SLOTS FP64 norm slots used in turn, so that a
+// Scratch (Plan::d_chain): claim counter, done counter, error word, exit
+// counter, then CHAIN_NORM_SLOTS FP64 norm slots used in turn, so that a
 // sequence of any length (many iterations of a short FP32 plan) runs chained.
+// The last CTA to leave zeroes all but the error word for the next launch (no
+// memset in front of it: 2 us a call); the holder of item 0 clears the error
+// word, which nothing can set before a wait of 2 s has run out.
 // Renormalisation k accumulates into slot k % CHAIN_NORM_SLOTS during pass
 // (k + 1) * renorm - 1 and is read during the next pass; tile 0 of the pass
 // before an accumulating pass zeroes its slot before counting itself done, so
@@ -273,69 +283,127 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
     chain_kernel(typename V2<Real>::T *__restrict__ state, const TileArgs *__restrict__ passes, int npasses,
                  int tile_bits, long long total, int renorm, unsigned long long *ctr, double *norms) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ long long s_item;
+    unsigned char *win = smem_raw + tile_smem_bytes<Real, R, W>();
+    __shared__ long long s_next;
     __shared__ int s_skip;
-    // the item's pass arguments, copied once per item: the tile code reads
-    // them many times (the tile-bit map byte by byte), from shared memory
-    // rather than through L1
-    __shared__ __align__(16) TileArgs s_ta;
+    // the pass arguments of this item and of the next: the tile code reads
+    // them many times (the tile-bit map byte by byte)
+    __shared__ __align__(16) TileArgs s_ta[2];
     const long long seq = total >> tile_bits;  // passes in the sequence
-    for (;;) {
+    auto fetch_args = [&](TileArgs *dst, int pass) {
+        fetch_units(reinterpret_cast<unsigned char *>(dst), reinterpret_cast<const uint4 *>(passes + pass),
+                    (int)(sizeof(TileArgs) / 16));
+    };
+    // g modulo the plan's passes and the renormalisation period, stepped along
+    // with g: 64-bit divisions for each item took a microsecond
+    struct Place {
+        long long g;
+        int pass, phase, slot;
+    };
+    auto step_to = [&](Place p, long long g) {
+        for (; p.g < g; p.g++) {
+            if (++p.pass == npasses) p.pass = 0;
+            if (renorm > 0 && ++p.phase == renorm) {
+                p.phase = 0;
+                if (++p.slot == CHAIN_NORM_SLOTS) p.slot = 0;
+            }
+        }
+        return p;
+    };
+    if (threadIdx.x == 0) s_next = (long long)atomicAdd(&ctr[0], 1ull);
+    __syncthreads();
+    long long it = s_next;
+    Place at;
+    at.g = it >> tile_bits;
+    at.pass = (int)(at.g % npasses);
+    at.phase = renorm > 0 ? (int)(at.g % renorm) : 0;
+    at.slot = renorm > 0 ? (int)(at.g / renorm % CHAIN_NORM_SLOTS) : 0;
+    const long long stride = gridDim.x;
+    int cur = 0;
+    if (it < total) {
+        fetch_args(&s_ta[0], at.pass);
+        fetch_wait();
+        __syncthreads();
+        fetch_stream(win, s_ta[0]);
+    }
+    while (it < total) {
+        const long long g = at.g;
         if (threadIdx.x == 0) {
-            const long long it = (long long)atomicAdd(&ctr[0], 1ull);
-            s_item = it;
-            s_skip = 0;
-            if (it < total) {
-                const unsigned long long need = (unsigned long long)((it >> tile_bits) << tile_bits);
+            int skip = 0;
+            const unsigned long long need = (unsigned long long)(g << tile_bits);
+            if (it == 0) ctr[2] = 0ull;
+            if (ld_acquire_u64(&ctr[1]) < need) {
                 const unsigned long long t0 = chain_now_ns();
                 while (ld_acquire_u64(&ctr[1]) < need) {
                     if (chain_now_ns() - t0 > CHAIN_WAIT_LIMIT_NS) {
                         atomicExch(&ctr[2], 1ull);
-                        s_skip = 1;
+                        skip = 1;
                         break;
                     }
-                    __nanosleep(64);
+                    __nanosleep(32);
                 }
             }
+            s_skip = skip;
         }
         __syncthreads();
-        const long long it = s_item;
-        if (it >= total) break;
+        // the pass of the item this CTA will probably claim next
+        const Place guess = step_to(at, (it + stride) >> tile_bits);
+        const bool fetched = guess.g < seq && guess.pass != at.pass;
+        if (fetched) fetch_args(&s_ta[cur ^ 1], guess.pass);
         if (!s_skip) {
-            const long long g = it >> tile_bits;
             int32_t flags = 0;
             double *norm_out = nullptr;
             const double *scale_in = nullptr;
             if (renorm > 0) {
                 // the plain launcher's schedule: a norm on every renorm-th
                 // pass but the last, a rescale on the pass after it
-                if ((g + 1) % renorm == 0 && g + 1 < seq) {
+                if (at.phase + 1 == renorm && g + 1 < seq) {
                     flags |= PASS_NORM;
-                    norm_out = norms + ((g + 1) / renorm - 1) % CHAIN_NORM_SLOTS;
+                    norm_out = norms + at.slot;
                 }
-                if (g > 0 && g % renorm == 0) {
+                if (at.phase == 0 && g > 0) {
                     flags |= PASS_SCALE;
-                    scale_in = norms + (g / renorm - 1) % CHAIN_NORM_SLOTS;
+                    scale_in = norms + (at.slot ? at.slot - 1 : CHAIN_NORM_SLOTS - 1);
                 }
             }
-            {
-                const uint32_t *src = reinterpret_cast<const uint32_t *>(passes + g % npasses);
-                uint32_t *dst = reinterpret_cast<uint32_t *>(&s_ta);
-                for (int w = threadIdx.x; w < (int)(sizeof(TileArgs) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
-            }
-            __syncthreads();
-            fetch_stream(smem_raw + tile_smem_bytes<Real, R, W>(), s_ta);
-            run_tile<Real, R, W, LEAN>(state, s_ta, (uint64_t)(it & ((1ll << tile_bits) - 1)), smem_raw, flags, norm_out,
-                                       scale_in);
+            run_tile<Real, R, W, LEAN>(state, s_ta[cur], (uint64_t)(it & ((1ll << tile_bits) - 1)), smem_raw, flags,
+                                       norm_out, scale_in);
         }
+        fetch_wait();  // the guessed pass's arguments
         __syncthreads();
+        if (threadIdx.x == blockDim.x - 1) s_next = (long long)atomicAdd(&ctr[0], 1ull);
+        if (fetched) cur ^= 1;
+        fetch_stream(win, s_ta[cur]);
         if (threadIdx.x == 0) {
-            const long long g = it >> tile_bits;
             // the next pass accumulates a norm: zero its slot first
-            if (renorm > 0 && (it & ((1ll << tile_bits) - 1)) == 0 && (g + 2) % renorm == 0 && g + 2 < seq)
-                norms[((g + 2) / renorm - 1) % CHAIN_NORM_SLOTS] = 0.0;
+            if (renorm > 0 && (it & ((1ll << tile_bits) - 1)) == 0 && g + 2 < seq) {
+                const bool wrap = at.phase + 2 > renorm;  // the next pass is in the next period
+                if (wrap ? renorm == 1 : at.phase + 2 == renorm)
+                    norms[wrap ? (at.slot + 1 == CHAIN_NORM_SLOTS ? 0 : at.slot + 1) : at.slot] = 0.0;
+            }
             __threadfence();
             atomicAdd(&ctr[1], 1ull);
+        }
+        __syncthreads();
+        const int here = fetched ? guess.pass : at.pass;
+        it = s_next;
+        at = step_to(at, it >> tile_bits);
+        if (it < total && at.pass != here) {  // guessed wrong
+            fetch_args(&s_ta[cur], at.pass);
+            fetch_wait();
+            __syncthreads();
+            fetch_stream(win, s_ta[cur]);
+        }
+    }
+    fetch_wait();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&ctr[3], 1ull) + 1 == gridDim.x) {
+            ctr[0] = 0ull;
+            ctr[1] = 0ull;
+            ctr[3] = 0ull;
+            if (renorm > 0)
+                for (int k = 0; k < CHAIN_NORM_SLOTS; k++) norms[k] = 0.0;
         }
     }
 }
@@ -360,8 +428,6 @@ static int launch_chain_rw(State *s, const Plan *p, int iterations, cudaStream_t
     const unsigned grid = (unsigned)(ntiles < grid_cap ? ntiles : grid_cap);
     unsigned long long *ctr = reinterpret_cast<unsigned long long *>(p->d_chain);
     double *norms = reinterpret_cast<double *>(ctr + 4);
-    cudaError_t e = cudaMemsetAsync(p->d_chain, 0, p->d_bytes[2], st);
-    if (e != cudaSuccess) return fail(HGM_ERR_CUDA, "chain scratch reset: %s", cudaGetErrorString(e));
     chain_kernel<Real, R, W, LEAN><<<grid, 32 << W, smem, st>>>(reinterpret_cast<A2 *>(s->d),
                                                           reinterpret_cast<const TileArgs *>(p->d_chain_passes),
                                                           (int)p->passes.size(), tile_bits, total, p->renorm_every,
@@ -457,6 +523,9 @@ int upload_plan(Plan *p) {
         const size_t pb = p->tiles.size() * sizeof(TileArgs);
         if ((e = plan_alloc(p, 2, &p->d_chain, sb)) != cudaSuccess)
             return fail(HGM_ERR_NOMEM, "plan chain scratch: %s", cudaGetErrorString(e));
+        // zero for the first launch; every launch leaves it so
+        if ((e = cudaMemset(p->d_chain, 0, sb)) != cudaSuccess)
+            return fail(HGM_ERR_CUDA, "plan chain scratch: %s", cudaGetErrorString(e));
         if ((e = plan_alloc(p, 3, &p->d_chain_passes, pb)) != cudaSuccess)
             return fail(HGM_ERR_NOMEM, "plan chain passes: %s", cudaGetErrorString(e));
         if ((e = cudaMemcpy(p->d_chain_passes, p->tiles.data(), pb, cudaMemcpyHostToDevice)) != cudaSuccess)

@@ -85,17 +85,22 @@ __host__ __device__ constexpr int tile_smem_elems() {
 
 // Offset (in amplitudes) of a thread's register-0 amplitude and the R
 // register-bit strides in the state, for a layout given by the global index
-// bit of each role (thread bits 0..4+W, then register bits).  Every lookup
-// uses a constant index into the kernel parameters (a runtime index would
-// copy them to local memory).
+// bit of each role (thread bits 0..4+W, then register bits), read as one
+// 16-byte word: byte by byte, the loads alone took several hundred cycles of
+// a small state's pass.
 template <int R, int W>
 __device__ __forceinline__ void thread_geometry(const int8_t (&gb)[MAX_LAYOUT_ROLES], uint32_t thr, uint64_t &off,
                                                 uint64_t (&rs)[R]) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(gb);
+    auto bit = [&](int k) {
+        const uint32_t w = k < 4 ? v.x : k < 8 ? v.y : k < 12 ? v.z : v.w;
+        return (w >> (8 * (k & 3))) & 63u;
+    };
     off = 0;
 #pragma unroll
-    for (int t = 0; t < 5 + W; t++) off |= (uint64_t)((thr >> t) & 1) << gb[t];
+    for (int t = 0; t < 5 + W; t++) off |= (uint64_t)((thr >> t) & 1) << bit(t);
 #pragma unroll
-    for (int q = 0; q < R; q++) rs[q] = (uint64_t)1 << gb[5 + W + q];
+    for (int q = 0; q < R; q++) rs[q] = (uint64_t)1 << bit(5 + W + q);
 }
 
 template <int R, int r>
@@ -131,18 +136,16 @@ struct LoadF {
         a[r] = __ldcg(p + reg_offset<R, r>(rs));
     }
 };
-// Register r goes to element idx ^ offset(r): idx already carries the
-// offset of the relabeling mask (the offsets are disjoint bits, so
-// offset(r ^ xr) = offset(r) ^ offset(xr)).
+// p is register 0's place and rs the steps with the relabeled bits' signs
+// turned (store_tile).
 template <typename A2, int R>
 struct StoreF {
     const A2 (&a)[1 << R];
     A2 *__restrict__ p;
-    uint64_t idx;
     const uint64_t (&rs)[R];
     template <int r>
     __device__ __forceinline__ void go() {
-        __stcg(p + (idx ^ reg_offset<R, r>(rs)), a[r]);
+        __stcg(p + (int64_t)reg_offset<R, r>(rs), a[r]);
     }
 };
 
@@ -1153,13 +1156,19 @@ __device__ __forceinline__ void transpose(A2 (&a)[1 << R], unsigned char *sm, co
 // Index of tile `t`: deposit the bits of t into the non-tile index bits, one
 // run of consecutive non-tile bits at a time (uniform across the CTA).
 __device__ __forceinline__ uint64_t tile_base(uint64_t t, const TileArgs &ta) {
-    uint64_t base = 0;
-#pragma unroll
-    for (int i = 0; i < MAX_FREE_RUNS; i++) {
-        if (i >= ta.nruns) break;
-        const int len = ta.run_len[i];
-        base |= (t & ((1ull << len) - 1ull)) << ta.run_pos[i];
-        t >>= len;
+    const ulonglong2 pos = *reinterpret_cast<const ulonglong2 *>(ta.run_pos),
+                     len = *reinterpret_cast<const ulonglong2 *>(ta.run_len);
+    uint64_t base = 0, p = pos.x, l = len.x;
+    for (int i = 0; i < ta.nruns; i++) {
+        if (i == 8) {
+            p = pos.y;
+            l = len.y;
+        }
+        const int n = (int)(l & 63u);
+        base |= (t & ((1ull << n) - 1ull)) << (p & 63u);
+        t >>= n;
+        p >>= 8;
+        l >>= 8;
     }
     return base;
 }
@@ -1186,11 +1195,16 @@ __device__ __forceinline__ void store_tile(const typename V2<Real>::T (&a)[1 << 
     asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thr));
     uint64_t off, rs[R];
     thread_geometry<R, W>(ta.st_gbit, thr, off, rs);
-    uint64_t xo = 0;
+    // register r goes to the place of label r ^ xr: start at the relabeled
+    // bits' steps and take those steps back where r has the bit
+    uint64_t idx = base | off;
 #pragma unroll
     for (int q = 0; q < R; q++)
-        if ((xr >> q) & 1u) xo |= rs[q];
-    StoreF<A2, R> f{a, state, base | off | xo, rs};
+        if ((xr >> q) & 1u) {
+            idx += rs[q];
+            rs[q] = 0ull - rs[q];
+        }
+    StoreF<A2, R> f{a, state + idx, rs};
     Unroll<1 << R>::run(f);
 }
 

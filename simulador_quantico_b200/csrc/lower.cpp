@@ -352,6 +352,7 @@ struct Lowering {
         t.n = pa.n;
         t.k = pa.k;
         t.nruns = pa.nruns;
+        static_assert(TILE_RUNS <= MAX_FREE_RUNS && 5 + PB_MAX_R + 3 + 1 <= TILE_RUNS, "runs of the largest tile");
         memcpy(t.run_pos, pa.run_pos, sizeof t.run_pos);
         memcpy(t.run_len, pa.run_len, sizeof t.run_len);
         memcpy(t.ld_gbit, pa.ld_gbit, sizeof t.ld_gbit);
