@@ -139,8 +139,8 @@ int hgm_plan_export(const hgm_plan *p, const void **passes, int64_t *n_passes, c
 int hgm_plan_layouts(const hgm_plan *p, const int8_t **pos, int64_t *n_layouts);
 /* What the plan's upload copies to the device: the passes lowered to streams
  * of 16-byte units (csrc/hgm_internal.h, "device stream"), or the small
- * state's records. */
-int hgm_plan_stream(const hgm_plan *p, const void **units, int64_t *bytes);
+ * state's records; and the passes as launched (struct TileArgs). */
+int hgm_plan_stream(const hgm_plan *p, const void **units, int64_t *bytes, const void **tiles, int64_t *n_tiles);
 
 /* ---- device-resident states -------------------------------------------- */
 

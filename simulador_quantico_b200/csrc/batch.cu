@@ -107,7 +107,8 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
     unsigned char *win = smem_raw + tile_smem_bytes<Real, R, W>();
     __shared__ long long s_next;
     __shared__ int s_next_task;
-    __shared__ int s_skip;
+    __shared__ int s_skip, s_task;
+    __shared__ PassCtl s_ctl;  // no renormalisation
     // the item's pass arguments: the tile code reads them many times
     __shared__ __align__(16) TileArgs s_ta;
     // Claims an item and finds its task.
@@ -127,15 +128,17 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
                     (int)(sizeof(TileArgs) / 16));
     };
     // one thread claims the next item and finds its task while another
-    // publishes this one
-    if (threadIdx.x == 0) claim();
-    __syncthreads();
-    long long it = s_next;
-    int task = s_next_task;
-    while (it < total_items) {
-        const BatchTask &t = tasks[task];
+    // publishes this one; nothing but shared memory is live through a tile
+    if (threadIdx.x == 0) {
+        claim();
+        s_ctl.flags = 0;
+    }
+    for (;;) {
+        __syncthreads();
+        if (s_next >= total_items) break;
+        const BatchTask &t = tasks[s_next_task];
         const bool tiled = !t.small;
-        if (tiled) fetch_args(&s_ta, task);
+        if (tiled) fetch_args(&s_ta, s_next_task);
         if (threadIdx.x == 0) {
             int skip = 0;
             if (t.dep >= 0) {
@@ -153,14 +156,15 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
                 }
             }
             s_skip = skip;
+            s_task = s_next_task;
         }
         fetch_wait();
         __syncthreads();
         if (!s_skip) {
             if (tiled) {
                 fetch_stream(win, s_ta);
-                run_tile<Real, R, W, LEAN>(reinterpret_cast<A2 *>(t.state), s_ta, (uint64_t)(it - t.tile_begin),
-                                           smem_raw, 0, nullptr, nullptr);
+                run_tile<Real, R, W, LEAN, true>(reinterpret_cast<A2 *>(t.state), s_ta,
+                                                 (uint64_t)(s_next - t.tile_begin), smem_raw, s_ctl);
             } else {
                 small_task<Real>(reinterpret_cast<A2 *>(t.state), t.n,
                                  reinterpret_cast<const SmallOp<Real> *>(t.small_ops), t.n_small_ops, sm, win);
@@ -170,11 +174,8 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
         if (threadIdx.x == blockDim.x - 1) claim();
         if (threadIdx.x == 0) {
             __threadfence();
-            atomicAdd(&done[task], 1u);
+            atomicAdd(&done[s_task], 1u);
         }
-        __syncthreads();
-        it = s_next;
-        task = s_next_task;
     }
 }
 
@@ -325,7 +326,7 @@ int batch_finalize(Batch *b) {
     // tasks, wave by wave
     std::vector<std::vector<int>> task_of(b->jobs.size());
     size_t max_passes = 0;
-    for (BatchJob &j : b->jobs) max_passes = std::max(max_passes, j.plan->small ? (size_t)1 : j.plan->passes.size());
+    for (BatchJob &j : b->jobs) max_passes = std::max(max_passes, j.plan->small ? (size_t)1 : j.plan->tiles.size());
     for (size_t wave = 0; wave < max_passes; wave++) {
         for (size_t ji = 0; ji < b->jobs.size(); ji++) {
             BatchJob &j = b->jobs[ji];
@@ -344,7 +345,7 @@ int batch_finalize(Batch *b) {
                     t.small_ops = nullptr;
                 }
             } else {
-                if (wave >= j.plan->passes.size()) continue;
+                if (wave >= j.plan->tiles.size()) continue;
                 t.pa = j.plan->tiles[wave];
                 t.ntiles = 1 << (j.n - t.pa.k);
             }

@@ -196,12 +196,14 @@ int hgm_plan_export(const hgm_plan *p, const void **passes, int64_t *n_passes, c
     return HGM_OK;
 }
 
-int hgm_plan_stream(const hgm_plan *p, const void **units, int64_t *bytes) {
+int hgm_plan_stream(const hgm_plan *p, const void **units, int64_t *bytes, const void **tiles, int64_t *n_tiles) {
     if (!p) return fail(HGM_ERR_INVALID, "null plan");
     const Plan *pl = reinterpret_cast<const Plan *>(p);
     const bool small = pl->small;
     if (units) *units = small ? (const void *)pl->ops_bytes.data() : (const void *)pl->stream.data();
     if (bytes) *bytes = small ? (int64_t)pl->ops_bytes.size() : (int64_t)(pl->stream.size() * sizeof(uint32_t));
+    if (tiles) *tiles = pl->tiles.data();
+    if (n_tiles) *n_tiles = (int64_t)pl->tiles.size();
     return HGM_OK;
 }
 

@@ -132,8 +132,9 @@ struct alignas(16) DevOp {
     int32_t kind, tpos;
     uint32_t cm_reg, cv_reg;   // controls on register bits
     uint32_t cm_thr, cv_thr;   // controls on thread bits (lane | warp << 5)
-    int32_t tpos2;             // tpos again, so a phase-block term's thread controls and
-    uint32_t pad1;             // target come in one 16-byte load
+    int32_t tpos2;             // tpos again
+    uint32_t pad1;             // ops of the swaps that end the circuit (planner swap_tail): 1 for a
+                               // record of its own, a bit per entry of a K_XSET
     uint64_t cm_glob, cv_glob; // controls on non-tile index bits
     Real m[8];
 };
@@ -229,6 +230,7 @@ struct PassArgs {
 
 constexpr int32_t PASS_NORM = 1;
 constexpr int32_t PASS_SCALE = 2;
+constexpr int32_t PASS_PERMUTE = 4;  // a permutation pass (below), no stream
 
 // ---- device stream -----------------------------------------------------------
 // What the kernels run.  Each pass's phases and op records (the plan above)
@@ -270,6 +272,24 @@ constexpr uint32_t STREAM_SYNC_BEFORE = 1, STREAM_SYNC_CROSS = 2;
 
 // A pass as the kernels take it.  The byte arrays are read 16 bytes at a time.
 constexpr int TILE_RUNS = 16;  // a tile of at most 13 bits leaves at most 14 runs
+// What renormalisation asks of one run of a pass.
+struct PassCtl {
+    int32_t flags;          // PASS_NORM, PASS_SCALE
+    double *norm_out;
+    const double *scale_in;
+};
+// A permutation pass (PASS_PERMUTE) swaps pairs of index bits of the whole
+// state in place.  It works on sub-tiles of 2^PERM_BITS amplitudes that agree
+// on the other index bits; a pair of bits lies inside the sub-tile or outside
+// it, so sub-tile u, permuted inside, goes to the place of sub-tile v and v to
+// that of u, both held by the same CTA.  Fields: ld_gbit[0..PERM_BITS) index
+// bit of each local bit, st_gbit local bit each local bit goes to, runs of the
+// other bits, ld_tstep as bytes the pairs of other bits, `pairs` of them; no
+// stream (units0 = units1 = 0: nothing is fetched).
+// Only for plans of at least PERM_WARP_BITS warp bits: smaller CTAs' tile code
+// has no permutation branch.
+constexpr int PERM_BITS = 10;
+constexpr int PERM_WARP_BITS = 2;
 struct alignas(16) TileArgs {
     int8_t ld_gbit[MAX_LAYOUT_ROLES];  // global index bit of every role of the load and store layouts
     int8_t st_gbit[MAX_LAYOUT_ROLES];
@@ -279,10 +299,11 @@ struct alignas(16) TileArgs {
     const void *stream;     // first window, then the others back to back
     int32_t units0, units1; // units of the first two windows
     int32_t n, k;
-    int32_t flags;          // PASS_*
+    int32_t flags;          // PASS_PERMUTE
     int32_t nruns;
-    double *norm_out;
-    const double *scale_in;
+    PassCtl ctl;            // (the pass kernel's; the chained kernel has its own)
+    int32_t pass;           // the plan's pass (permutation: -1)
+    int32_t pairs;          // permutation: pairs of other bits
 };
 static_assert(sizeof(TileArgs) % 16 == 0, "copied as 16-byte units");
 
@@ -310,6 +331,7 @@ struct Plan {
     int qubits = 0;
     int warp_bits = 0;
     int reg_bits = 5;                 // amplitudes per thread = 2^reg_bits
+    int low_bits = 0;                 // index bits 0.. that load and store layouts keep on thread bits
     bool small = false;               // n < 5 + reg_bits: single-CTA shared-memory path
     std::vector<PassArgs> passes;     // device pointers patched after upload
     std::vector<DevPhase> phases;
@@ -360,8 +382,10 @@ int build_plan(const std::vector<Op> &ops, int qubits, const hgm_plan_opts &opts
                bool force_small = false);
 int upload_plan(Plan *plan);
 // Lowers a tiled plan's passes to the device stream (lower.cpp).  global: the
-// scalar the plan's last record applies (1: there is no such record).
-void lower_plan(Plan *plan, cplx global);
+// scalar the plan's last record applies (1: there is no such record).  swaps:
+// the pairs of index bits whose swaps end the circuit (their records are
+// marked, DevOp pad1).
+void lower_plan(Plan *plan, cplx global, const std::vector<std::pair<int, int>> &swaps);
 void plan_lease(const Plan *plan);
 void plan_unlease(const Plan *plan);
 

@@ -90,7 +90,16 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
     pass_kernel(typename V2<Real>::T *__restrict__ state, const __grid_constant__ TileArgs ta) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     fetch_stream(smem_raw + tile_smem_bytes<Real, R, W>(), ta);
-    run_tile<Real, R, W, LEAN>(state, ta, blockIdx.x, smem_raw, ta.flags, ta.norm_out, ta.scale_in);
+    run_tile<Real, R, W, LEAN, false>(state, ta, blockIdx.x, smem_raw, ta.ctl);
+}
+
+// A permutation pass over a large state, one sub-tile a block.
+constexpr int PERM_THREADS = 128;
+template <typename Real>
+__global__ void __launch_bounds__(PERM_THREADS) permute_kernel(typename V2<Real>::T *__restrict__ state,
+                                                               const __grid_constant__ TileArgs ta) {
+    __shared__ typename V2<Real>::T sm[2 * PERM_SLOTS];
+    permute_subtile<Real, PERM_THREADS>(state, ta, blockIdx.x, sm, ta.ctl);
 }
 
 template <typename Real>
@@ -198,24 +207,33 @@ int launch_plan_steps(State *s, const Plan *p, int iterations, PlanCursor *c, in
                                                          : launch_small<float>(s, p, iterations, st))
                               : HGM_OK;
     }
-    const int64_t np = (int64_t)p->passes.size();
+    const int64_t np = (int64_t)p->tiles.size();
     const int R = p->renorm_every;
     const int64_t total = np * iterations;
     for (int64_t k = 0; k < max_launches && c->next < total; k++, c->next++) {
         const int64_t g = c->next;
         TileArgs pa = p->tiles[g % np];
         if (c->scale_next) {
-            pa.flags |= PASS_SCALE;
-            pa.scale_in = p->d_norm + c->scale_slot;
+            pa.ctl.flags |= PASS_SCALE;
+            pa.ctl.scale_in = p->d_norm + c->scale_slot;
             c->scale_next = false;
         }
         if (R > 0 && ((g + 1) % R == 0) && g + 1 < total) {
-            pa.flags |= PASS_NORM;
-            pa.norm_out = p->d_norm + c->slot;
-            cudaMemsetAsync(pa.norm_out, 0, sizeof(double), st);
+            pa.ctl.flags |= PASS_NORM;
+            pa.ctl.norm_out = p->d_norm + c->slot;
+            cudaMemsetAsync(pa.ctl.norm_out, 0, sizeof(double), st);
             c->scale_next = true;
             c->scale_slot = c->slot;
             c->slot = (c->slot + 1) % 64;
+        }
+        if (pa.flags & PASS_PERMUTE) {
+            const unsigned grid = 1u << (pa.n - PERM_BITS);
+            if (p->precision == HGM_F64)
+                permute_kernel<double><<<grid, PERM_THREADS, 0, st>>>((double2 *)s->d, pa);
+            else
+                permute_kernel<float><<<grid, PERM_THREADS, 0, st>>>((float2 *)s->d, pa);
+            count_launch();
+            continue;
         }
         int rc = p->precision == HGM_F64
                      ? launch_pass_lw<double, HGM_F64_REG_BITS>(p->lean, p->warp_bits, s->d, pa, st)
@@ -227,7 +245,7 @@ int launch_plan_steps(State *s, const Plan *p, int iterations, PlanCursor *c, in
 }
 
 int64_t plan_launches(const Plan *p, int iterations) {
-    return p->small ? 1 : (int64_t)p->passes.size() * iterations;
+    return p->small ? 1 : (int64_t)p->tiles.size() * iterations;
 }
 
 // ---------------------------------------------------------------------------
@@ -284,21 +302,25 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
                  int tile_bits, long long total, int renorm, unsigned long long *ctr, double *norms) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *win = smem_raw + tile_smem_bytes<Real, R, W>();
-    __shared__ long long s_next;
-    __shared__ int s_skip;
-    // the pass arguments of this item and of the next: the tile code reads
-    // them many times (the tile-bit map byte by byte)
+    // The sequence's state is kept in shared memory by thread 0: in registers
+    // it would be live through every tile.  g modulo the plan's passes and the
+    // renormalisation period are stepped along with g (64-bit divisions for
+    // each item took a microsecond).
+    struct Place {
+        long long g;
+        int pass, phase, slot;
+    };
+    __shared__ Place s_at, s_guess;
+    __shared__ long long s_it, s_next;
+    __shared__ PassCtl s_ctl;
+    __shared__ int s_skip, s_fetched, s_refetch, s_cur;
+    // the arguments of this item's pass and of the guessed next one: the tile
+    // code reads them many times (the tile-bit map byte by byte)
     __shared__ __align__(16) TileArgs s_ta[2];
     const long long seq = total >> tile_bits;  // passes in the sequence
     auto fetch_args = [&](TileArgs *dst, int pass) {
         fetch_units(reinterpret_cast<unsigned char *>(dst), reinterpret_cast<const uint4 *>(passes + pass),
                     (int)(sizeof(TileArgs) / 16));
-    };
-    // g modulo the plan's passes and the renormalisation period, stepped along
-    // with g: 64-bit divisions for each item took a microsecond
-    struct Place {
-        long long g;
-        int pass, phase, slot;
     };
     auto step_to = [&](Place p, long long g) {
         for (; p.g < g; p.g++) {
@@ -310,89 +332,89 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
         }
         return p;
     };
-    if (threadIdx.x == 0) s_next = (long long)atomicAdd(&ctr[0], 1ull);
-    __syncthreads();
-    long long it = s_next;
-    Place at;
-    at.g = it >> tile_bits;
-    at.pass = (int)(at.g % npasses);
-    at.phase = renorm > 0 ? (int)(at.g % renorm) : 0;
-    at.slot = renorm > 0 ? (int)(at.g / renorm % CHAIN_NORM_SLOTS) : 0;
-    const long long stride = gridDim.x;
-    int cur = 0;
-    if (it < total) {
-        fetch_args(&s_ta[0], at.pass);
-        fetch_wait();
-        __syncthreads();
-        fetch_stream(win, s_ta[0]);
+    if (threadIdx.x == 0) {
+        s_next = (long long)atomicAdd(&ctr[0], 1ull);
+        s_at.g = s_next >> tile_bits;
+        s_at.pass = (int)(s_at.g % npasses);
+        s_at.phase = renorm > 0 ? (int)(s_at.g % renorm) : 0;
+        s_at.slot = renorm > 0 ? (int)(s_at.g / renorm % CHAIN_NORM_SLOTS) : 0;
+        s_guess = s_at;
+        s_guess.pass = -1;  // nothing is fetched yet
+        s_fetched = 1;
+        s_cur = 1;
     }
-    while (it < total) {
-        const long long g = at.g;
-        if (threadIdx.x == 0) {
-            int skip = 0;
-            const unsigned long long need = (unsigned long long)(g << tile_bits);
-            if (it == 0) ctr[2] = 0ull;
-            if (ld_acquire_u64(&ctr[1]) < need) {
-                const unsigned long long t0 = chain_now_ns();
-                while (ld_acquire_u64(&ctr[1]) < need) {
-                    if (chain_now_ns() - t0 > CHAIN_WAIT_LIMIT_NS) {
-                        atomicExch(&ctr[2], 1ull);
-                        skip = 1;
-                        break;
-                    }
-                    __nanosleep(32);
-                }
-            }
-            s_skip = skip;
-        }
+    for (;;) {
+        // thread 0: the item claimed below (thread 0 itself before the first turn)
         __syncthreads();
-        // the pass of the item this CTA will probably claim next
-        const Place guess = step_to(at, (it + stride) >> tile_bits);
-        const bool fetched = guess.g < seq && guess.pass != at.pass;
-        if (fetched) fetch_args(&s_ta[cur ^ 1], guess.pass);
-        if (!s_skip) {
-            int32_t flags = 0;
-            double *norm_out = nullptr;
-            const double *scale_in = nullptr;
-            if (renorm > 0) {
+        if (threadIdx.x == 0) {
+            const long long it = s_next;
+            const int here = s_fetched ? s_guess.pass : s_at.pass;  // the pass that is fetched
+            const Place at = step_to(s_at, it >> tile_bits);
+            const long long g = at.g;
+            s_it = it;
+            s_at = at;
+            s_cur ^= s_fetched;
+            s_refetch = at.pass != here;
+            if (it < total) {
+                // the pass of the item this CTA will probably claim next
+                const Place guess = step_to(at, (it + gridDim.x) >> tile_bits);
+                s_guess = guess;
+                s_fetched = guess.g < seq && guess.pass != at.pass;
                 // the plain launcher's schedule: a norm on every renorm-th
                 // pass but the last, a rescale on the pass after it
-                if (at.phase + 1 == renorm && g + 1 < seq) {
-                    flags |= PASS_NORM;
-                    norm_out = norms + at.slot;
+                int32_t flags = 0;
+                if (renorm > 0) {
+                    if (at.phase + 1 == renorm && g + 1 < seq) flags |= PASS_NORM;
+                    if (at.phase == 0 && g > 0) flags |= PASS_SCALE;
+                    s_ctl.norm_out = norms + at.slot;
+                    s_ctl.scale_in = norms + (at.slot ? at.slot - 1 : CHAIN_NORM_SLOTS - 1);
                 }
-                if (at.phase == 0 && g > 0) {
-                    flags |= PASS_SCALE;
-                    scale_in = norms + (at.slot ? at.slot - 1 : CHAIN_NORM_SLOTS - 1);
+                s_ctl.flags = flags;
+                int skip = 0;
+                const unsigned long long need = (unsigned long long)(g << tile_bits);
+                if (it == 0) ctr[2] = 0ull;
+                if (ld_acquire_u64(&ctr[1]) < need) {
+                    const unsigned long long t0 = chain_now_ns();
+                    while (ld_acquire_u64(&ctr[1]) < need) {
+                        if (chain_now_ns() - t0 > CHAIN_WAIT_LIMIT_NS) {
+                            atomicExch(&ctr[2], 1ull);
+                            skip = 1;
+                            break;
+                        }
+                        __nanosleep(32);
+                    }
                 }
+                s_skip = skip;
             }
-            run_tile<Real, R, W, LEAN>(state, s_ta[cur], (uint64_t)(it & ((1ll << tile_bits) - 1)), smem_raw, flags,
-                                       norm_out, scale_in);
         }
+        __syncthreads();
+        if (s_it >= total) break;
+        if (s_refetch) {  // the first item, or guessed wrong
+            fetch_wait();
+            __syncthreads();
+            fetch_args(&s_ta[s_cur], s_at.pass);
+            fetch_wait();
+            __syncthreads();
+            fetch_stream(win, s_ta[s_cur]);
+        }
+        if (s_fetched) fetch_args(&s_ta[s_cur ^ 1], s_guess.pass);
+        if (!s_skip)
+            run_tile<Real, R, W, LEAN, true>(state, s_ta[s_cur], (uint64_t)(s_it & ((1ll << tile_bits) - 1)), smem_raw,
+                                             s_ctl);
         fetch_wait();  // the guessed pass's arguments
         __syncthreads();
         if (threadIdx.x == blockDim.x - 1) s_next = (long long)atomicAdd(&ctr[0], 1ull);
-        if (fetched) cur ^= 1;
-        fetch_stream(win, s_ta[cur]);
+        fetch_stream(win, s_ta[s_cur ^ s_fetched]);
         if (threadIdx.x == 0) {
             // the next pass accumulates a norm: zero its slot first
-            if (renorm > 0 && (it & ((1ll << tile_bits) - 1)) == 0 && g + 2 < seq) {
-                const bool wrap = at.phase + 2 > renorm;  // the next pass is in the next period
-                if (wrap ? renorm == 1 : at.phase + 2 == renorm)
-                    norms[wrap ? (at.slot + 1 == CHAIN_NORM_SLOTS ? 0 : at.slot + 1) : at.slot] = 0.0;
+            if (renorm > 0 && (s_it & ((1ll << tile_bits) - 1)) == 0 && s_at.g + 2 < seq) {
+                const int slot = s_at.slot;
+                const bool wrap = s_at.phase + 2 > renorm;  // the next pass is in the next period
+                if (wrap ? renorm == 1 : s_at.phase + 2 == renorm)
+                    norms[wrap ? (slot + 1 == CHAIN_NORM_SLOTS ? 0 : slot + 1) : slot] = 0.0;
             }
             __threadfence();
             atomicAdd(&ctr[1], 1ull);
-        }
-        __syncthreads();
-        const int here = fetched ? guess.pass : at.pass;
-        it = s_next;
-        at = step_to(at, it >> tile_bits);
-        if (it < total && at.pass != here) {  // guessed wrong
-            fetch_args(&s_ta[cur], at.pass);
-            fetch_wait();
-            __syncthreads();
-            fetch_stream(win, s_ta[cur]);
         }
     }
     fetch_wait();
@@ -422,15 +444,15 @@ static int launch_chain_rw(State *s, const Plan *p, int iterations, cudaStream_t
         if (e != cudaSuccess || per_sm < 1) return fail(HGM_ERR_CUDA, "chain kernel setup: %s", cudaGetErrorString(e));
         grid_cap = sms * per_sm;
     }
-    const int tile_bits = p->qubits - p->passes[0].k;
-    const long long total = ((long long)p->passes.size() * iterations) << tile_bits;
+    const int tile_bits = p->qubits - p->tiles[0].k;
+    const long long total = ((long long)p->tiles.size() * iterations) << tile_bits;
     const long long ntiles = 1ll << tile_bits;
     const unsigned grid = (unsigned)(ntiles < grid_cap ? ntiles : grid_cap);
     unsigned long long *ctr = reinterpret_cast<unsigned long long *>(p->d_chain);
     double *norms = reinterpret_cast<double *>(ctr + 4);
     chain_kernel<Real, R, W, LEAN><<<grid, 32 << W, smem, st>>>(reinterpret_cast<A2 *>(s->d),
                                                           reinterpret_cast<const TileArgs *>(p->d_chain_passes),
-                                                          (int)p->passes.size(), tile_bits, total, p->renorm_every,
+                                                          (int)p->tiles.size(), tile_bits, total, p->renorm_every,
                                                           ctr, norms);
     count_launch();
     return check("chain_kernel launch");
@@ -452,10 +474,7 @@ static int launch_chain_w(State *s, const Plan *p, int iterations, cudaStream_t 
 }
 
 bool chain_eligible(const Plan *p, int iterations) {
-    if (p->small || !p->d_chain || p->passes.size() < 2 || iterations < 1) return false;
-    const int64_t seq = (int64_t)p->passes.size() * iterations;
-    (void)seq;
-    return true;
+    return !p->small && p->d_chain && p->tiles.size() >= 2 && iterations >= 1;
 }
 
 int launch_plan_chain(State *s, const Plan *p, int iterations, void *stream) {
@@ -514,7 +533,8 @@ int upload_plan(Plan *p) {
         if ((e = plan_alloc(p, 1, (void **)&p->d_norm, 64 * sizeof(double))) != cudaSuccess)
             return fail(HGM_ERR_NOMEM, "plan norm slots: %s", cudaGetErrorString(e));
     }
-    for (TileArgs &t : p->tiles) t.stream = (const unsigned char *)p->d_ops + reinterpret_cast<size_t>(t.stream);
+    for (TileArgs &t : p->tiles)
+        if (!(t.flags & PASS_PERMUTE)) t.stream = (const unsigned char *)p->d_ops + reinterpret_cast<size_t>(t.stream);
     const int64_t state_bytes = (int64_t(1) << p->qubits) * (p->precision == HGM_F64 ? 16 : 8);
     if (p->chained && !p->small && p->tiles.size() >= 2 && state_bytes <= CHAIN_MAX_BYTES) {
         // chained execution: the pass records (pointers patched) and the scratch

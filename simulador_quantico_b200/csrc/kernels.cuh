@@ -1227,20 +1227,20 @@ __device__ __forceinline__ void store_tile(const typename V2<Real>::T (&a)[1 << 
 // passes 5% and QFT passes 9% faster (fewer instruction-fetch stalls), so
 // each plan runs the smallest build it can.
 //
-// flags, norm_out, scale_in: the pass's PASS_* flags and renormalisation
-// slots (the plain pass kernel passes ta's own; the chained kernel computes
-// them per position in the pass sequence).  The scale is read through L2:
-// in a chained run it was accumulated by other CTAs of the same launch.
+// ctl: renormalisation (the plain pass kernel passes ta's own; the chained
+// kernel sets it per position in the pass sequence, in shared memory, where it
+// costs the tile no registers).  The scale is read through L2: in a chained
+// run it was accumulated by other CTAs of the same launch.
 template <typename Real, int R, int W, bool LEAN>
 __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], typename V2<Real>::T *__restrict__ state,
-                                            const TileArgs &ta, uint64_t base, unsigned char *sm, int32_t flags,
-                                            double *norm_out, const double *scale_in) {
+                                            const TileArgs &ta, uint64_t base, unsigned char *sm,
+                                            const PassCtl &ctl) {
     using A2 = typename V2<Real>::T;
     constexpr bool F64 = sizeof(Real) == 8;
     const uint32_t thr = threadIdx.x, lane = thr & 31;
     unsigned char *win = sm + tile_smem_bytes<Real, R, W>();
-    if (flags & PASS_SCALE) {
-        const Real s = (Real)rsqrt(__ldcg(scale_in));
+    if (ctl.flags & PASS_SCALE) {
+        const Real s = (Real)rsqrt(__ldcg(ctl.scale_in));
 #pragma unroll
         for (int r = 0; r < (1 << R); r++) {
             a[r].x *= s;
@@ -1314,27 +1314,115 @@ __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], t
         }
     }
     store_tile<Real, R, W>(a, state, ta, base, xr);
-    if (flags & PASS_NORM) {
+    if (ctl.flags & PASS_NORM) {
         double acc = 0.0;
 #pragma unroll
         for (int r = 0; r < (1 << R); r++) acc += (double)a[r].x * a[r].x + (double)a[r].y * a[r].y;
 #pragma unroll
         for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) atomicAdd(norm_out, acc);
+        if (lane == 0) atomicAdd(ctl.norm_out, acc);
+    }
+}
+
+// ---- permutation pass -----------------------------------------------------------
+
+// Sub-tile u of a permutation pass (hgm_internal.h PASS_PERMUTE), NT threads:
+// u, permuted inside, to the place of its partner v and v to that of u; u's
+// holder does both, v's nothing.  Loads and stores are runs of 128 bytes and
+// more; the bits change places in shared memory (slot s + s / 16: lanes that
+// write 2^4 slots apart miss each other's banks), both sub-tiles at once, so
+// that few amplitudes are held in registers: inlined in the chained kernels
+// beside the tile code, sixteen of them cost 190-430 bytes of spills.
+constexpr int PERM_SLOTS = (1 << PERM_BITS) + (1 << (PERM_BITS - 4));  // a sub-tile's slots
+template <typename Real, int NT>
+__device__ __forceinline__ void permute_subtile(typename V2<Real>::T *__restrict__ state, const TileArgs &ta, uint64_t u,
+                                                typename V2<Real>::T *sm, const PassCtl &ctl) {
+    using A2 = typename V2<Real>::T;
+    constexpr int PER = (1 << PERM_BITS) / NT;
+    const uint32_t tid = threadIdx.x;
+    const uint64_t base = tile_base(u, ta);
+    uint64_t other = base;
+    const unsigned char *pair = reinterpret_cast<const unsigned char *>(ta.ld_tstep);
+    for (int k = 0; k < ta.pairs; k++) {
+        const int a = pair[2 * k], b = pair[2 * k + 1];
+        const uint64_t x = ((other >> a) ^ (other >> b)) & 1ull;
+        other ^= (x << a) | (x << b);
+    }
+    if (other < base) return;
+    // place in the state and slot after the permutation of local index j
+    auto place = [&](uint32_t j) {
+        uint64_t o = 0;
+#pragma unroll
+        for (int q = 0; q < PERM_BITS; q++) o |= (uint64_t)((j >> q) & 1u) << ta.ld_gbit[q];
+        return o;
+    };
+    auto slot = [&](uint32_t j) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int q = 0; q < PERM_BITS; q++) v |= ((j >> q) & 1u) << ta.st_gbit[q];
+        return v + (v >> 4);
+    };
+    const uint64_t at = place(tid);
+    const uint32_t to = slot(tid);
+    const Real scale = (ctl.flags & PASS_SCALE) ? (Real)rsqrt(__ldcg(ctl.scale_in)) : (Real)1;
+    double acc = 0.0;
+    const int sides = other != base ? 2 : 1;
+#pragma unroll 1
+    for (int side = 0; side < sides; side++) {
+        const A2 *__restrict__ src = state + ((side ? other : base) | at);
+        A2 v[PER];
+#pragma unroll
+        for (int i = 0; i < PER; i++) v[i] = __ldcg(src + place(i * NT));
+        if (ctl.flags & (PASS_SCALE | PASS_NORM)) {
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                v[i].x *= scale;
+                v[i].y *= scale;
+                acc += (double)v[i].x * v[i].x + (double)v[i].y * v[i].y;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < PER; i++) sm[side * PERM_SLOTS + to + slot(i * NT)] = v[i];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int side = 0; side < sides; side++) {
+        A2 *__restrict__ dst = state + ((side ? base : other) | at);
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const uint32_t j = i * NT + tid;
+            __stcg(dst + place(i * NT), sm[side * PERM_SLOTS + j + (j >> 4)]);
+        }
+    }
+    __syncthreads();
+    if (ctl.flags & PASS_NORM) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if ((tid & 31) == 0) atomicAdd(ctl.norm_out, acc);
     }
 }
 
 // Runs one pass over tile `tile`.  Shared by the plain pass kernel and the
 // chained and batched persistent kernels; the first windows' copy has been
-// started.
-template <typename Real, int R, int W, bool LEAN>
+// started.  PERM: the pass may be a permutation pass (the pass kernel's are
+// launches of their own).
+template <typename Real, int R, int W, bool LEAN, bool PERM>
 __device__ __forceinline__ void run_tile(typename V2<Real>::T *__restrict__ state, const TileArgs &ta, uint64_t tile,
-                                         unsigned char *sm, int32_t flags, double *norm_out, const double *scale_in) {
+                                         unsigned char *sm, const PassCtl &ctl) {
     using A2 = typename V2<Real>::T;
+    if constexpr (W >= PERM_WARP_BITS && PERM) {
+        if (ta.flags & PASS_PERMUTE) {
+            constexpr int SUB = 5 + R + W - PERM_BITS;  // sub-tiles a tile, as a power of two
+            static_assert(2 * PERM_SLOTS <= tile_smem_elems<R, W>(), "two sub-tiles fit the transpose buffer");
+            for (uint64_t k = 0; k < (1ull << SUB); k++)
+                permute_subtile<Real, 32 << W>(state, ta, (tile << SUB) | k, reinterpret_cast<A2 *>(sm), ctl);
+            return;
+        }
+    }
     const uint64_t base = tile_base(tile, ta);
     A2 a[1 << R];
     load_tile<Real, R, W>(a, state, ta, base, threadIdx.x);
-    finish_tile<Real, R, W, LEAN>(a, state, ta, base, sm, flags, norm_out, scale_in);
+    finish_tile<Real, R, W, LEAN>(a, state, ta, base, sm, ctl);
 }
 
 }  // namespace hgm

@@ -10,7 +10,12 @@
 //     factors multiply into one S_SCALE at the plan's end (or when they leave
 //     [2^-200, 2^200]).  28 qubits, 10 layers, FP64: 67.0 -> 50.1 ms with the
 //     stream; 26-qubit search, 32 iterations: 78.7 -> 60.2 ms.  FP32 keeps the plain form: its results stay, bit by
-//     bit, those of the records.
+//     bit, those of the records;
+//   * the swaps that end a circuit (a QFT's qubit reversal), where they fill
+//     passes of their own, as one permutation pass: it reads and writes the
+//     state once at memory speed, whatever the pairs, where CNOTs need the
+//     bits of a pair in one tile (27-qubit FP32 QFT:
+//     4.65 -> 3.31 ms, three passes of CNOTs and some of three others gone).
 #include <cmath>
 #include <cstring>
 
@@ -74,7 +79,40 @@ struct Lowering {
     std::vector<size_t> windows;   // units of each finished window
     static constexpr size_t CAP = STREAM_WINDOW_UNITS - 1;  // one unit for S_NEXT or S_END
 
+    bool drop_swaps = false; // the marked records are left to a permutation pass
+
     Lowering(Plan *p, cplx gl) : plan(p), global(gl), R(p->reg_bits), W(p->warp_bits) {}
+
+    bool same_warps(int a, int b) const {
+        for (int w = 0; w < W; w++)
+            if (plan->layouts[a].pos[5 + w] != plan->layouts[b].pos[5 + w]) return false;
+        return true;
+    }
+    // whether the layout may store the state (planner LayoutMaker::coalesced)
+    bool coalesced(int l) const {
+        for (int i = 0; i < plan->low_bits && i < 5; i++)
+            if (plan->layouts[l].pos[i] != i) return false;
+        return true;
+    }
+    static int records(const DevOp<Real> &d) {
+        if (d.kind == K_PHASE_BLOCK) return 1 + d.tpos;
+        if (d.kind == K_LAYER || d.kind == K_LAYER_REAL || d.kind == K_LAYER_SPLIT) return 1 + __builtin_popcount(d.cm_reg);
+        return 1;
+    }
+    // whether every op of the record belongs to the final swaps
+    static bool swap_record(const DevOp<Real> &d) {
+        return d.kind == K_XSET ? d.pad1 == (1u << d.tpos) - 1u : d.kind == K_SWAP && d.pad1;
+    }
+    bool only_swaps(const DevPhase &ph, const DevOp<Real> *ops) const {
+        for (int i = ph.op_begin; i < ph.op_end; i += records(ops[i]))
+            if (!swap_record(ops[i])) return false;
+        return true;
+    }
+    bool only_swaps(const PassArgs &pa, const DevOp<Real> *ops) const {
+        for (int p = pa.phase_begin; p < pa.phase_end; p++)
+            if (!only_swaps(plan->phases[p], ops)) return false;
+        return true;
+    }
 
     static void put_real(std::vector<uint32_t> &v, Real x) {
         uint32_t w[2] = {0, 0};
@@ -290,16 +328,22 @@ struct Lowering {
         windows.clear();
         int cur = pa.load_layout;
         bool prev_cross = false;
+        auto go_to = [&](int layout) {
+            if (layout == cur) return;
+            const bool cross = !same_warps(cur, layout);
+            transpose(cur, layout, prev_cross || cross, cross);
+            prev_cross = cross;
+            cur = layout;
+        };
         for (int p = pa.phase_begin; p < pa.phase_end; p++) {
             const DevPhase &ph = plan->phases[p];
-            if (ph.layout != cur) {
-                transpose(cur, ph.layout, prev_cross || ph.xwarp, ph.xwarp != 0);
-                prev_cross = ph.xwarp != 0;
-                cur = ph.layout;
-            }
+            if (drop_swaps && only_swaps(ph, ops)) continue;
+            go_to(ph.layout);
             for (int i = ph.op_begin; i < ph.op_end;) {
                 const DevOp<Real> &d = ops[i];
-                if (d.kind == K_PHASE_BLOCK) {
+                if (drop_swaps && swap_record(d)) {
+                    i++;
+                } else if (d.kind == K_PHASE_BLOCK) {
                     i += phase_block(ops + i);
                 } else if (d.kind == K_LAYER_REAL || d.kind == K_LAYER_SPLIT) {
                     layer(d, ops + i + 1);
@@ -312,9 +356,14 @@ struct Lowering {
                     add(S_DENSE, op);
                     i += 1 + k;
                 } else if (d.kind == K_XSET) {
-                    std::vector<uint32_t> op = {0u, (uint32_t)d.tpos};
-                    op.resize(2 + d.tpos);
-                    memcpy(&op[2], d.m, 4 * (size_t)d.tpos);
+                    std::vector<uint32_t> op = {0u, 0u};
+                    for (int k = 0; k < d.tpos; k++) {
+                        if (drop_swaps && ((d.pad1 >> k) & 1u)) continue;
+                        uint32_t w;
+                        memcpy(&w, reinterpret_cast<const unsigned char *>(d.m) + 4 * k, 4);
+                        op.push_back(w);
+                        op[1]++;
+                    }
                     add(S_XSET, op);
                     i++;
                 } else if (last_pass && i + 1 == (int)n_ops && global != 1.0) {
@@ -333,8 +382,7 @@ struct Lowering {
             }
         }
         if (last_pass) add_scale();
-        if (cur != pa.store_layout)
-            transpose(cur, pa.store_layout, prev_cross || pa.store_xwarp, pa.store_xwarp != 0);
+        if (!(drop_swaps && coalesced(cur))) go_to(pa.store_layout);
         flush(S_END);
 
         TileArgs t;
@@ -356,25 +404,91 @@ struct Lowering {
         memcpy(t.run_pos, pa.run_pos, sizeof t.run_pos);
         memcpy(t.run_len, pa.run_len, sizeof t.run_len);
         memcpy(t.ld_gbit, pa.ld_gbit, sizeof t.ld_gbit);
-        memcpy(t.st_gbit, pa.st_gbit, sizeof t.st_gbit);
+        for (int k = 0; k < 5 + W + R; k++) t.st_gbit[k] = pa.tb[plan->layouts[cur].pos[k]];
+        t.pass = (int32_t)(&pa - plan->passes.data());
         for (int b = 0; b < 8; b++) t.ld_tstep[b] = thread_step(plan->layouts[pa.load_layout], b);
         plan->tiles.push_back(t);
     }
 
-    void run() {
+    // The permutation pass for `swaps`; false when its sub-tile cannot be
+    // chosen: the low index bits (128-byte runs) with their partners, then
+    // pairs, then bits that stay, PERM_BITS in all.
+    bool permutation(const std::vector<std::pair<int, int>> &swaps, TileArgs &t) const {
+        const int n = plan->qubits, low = sizeof(Real) == 8 ? 3 : 4;
+        if (n < PERM_BITS || W < PERM_WARP_BITS) return false;
+        int to[64];
+        for (int b = 0; b < n; b++) to[b] = b;
+        for (const auto &p : swaps) {
+            to[p.first] = p.second;
+            to[p.second] = p.first;
+        }
+        uint64_t in = 0;
+        for (int b = 0; b < low; b++) in |= (uint64_t(1) << b) | (uint64_t(1) << to[b]);
+        for (int want_pair = 1; want_pair >= 0; want_pair--)
+            for (int b = 0; b < n; b++) {
+                const uint64_t m = (uint64_t(1) << b) | (uint64_t(1) << to[b]);
+                if ((in & m) || (to[b] != b) != (want_pair == 1)) continue;
+                if (__builtin_popcountll(in | m) <= PERM_BITS) in |= m;
+            }
+        if (__builtin_popcountll(in) != PERM_BITS) return false;
+        memset(&t, 0, sizeof t);
+        int local[64], k = 0;
+        for (int b = 0; b < n; b++)
+            if ((in >> b) & 1) {
+                t.ld_gbit[k] = (int8_t)b;
+                local[b] = k++;
+            }
+        for (int q = 0; q < PERM_BITS; q++) t.st_gbit[q] = (int8_t)local[to[t.ld_gbit[q]]];
+        for (int g = 0; g < n;) {
+            if ((in >> g) & 1) {
+                g++;
+                continue;
+            }
+            int e = g;
+            while (e < n && !((in >> e) & 1)) e++;
+            if (t.nruns == TILE_RUNS) return false;
+            t.run_pos[t.nruns] = (int8_t)g;
+            t.run_len[t.nruns++] = (int8_t)(e - g);
+            g = e;
+        }
+        int8_t *pair = reinterpret_cast<int8_t *>(t.ld_tstep);
+        for (const auto &p : swaps) {
+            if ((in >> p.first) & 1) continue;
+            if (2 * (t.pairs + 1) > (int)sizeof t.ld_tstep) return false;
+            pair[2 * t.pairs] = (int8_t)p.first;
+            pair[2 * t.pairs + 1] = (int8_t)p.second;
+            t.pairs++;
+        }
+        t.n = n;
+        t.k = 5 + R + W;
+        t.flags = PASS_PERMUTE;
+        t.pass = -1;
+        return true;
+    }
+
+    void run(const std::vector<std::pair<int, int>> &swaps) {
         const DevOp<Real> *ops = reinterpret_cast<const DevOp<Real> *>(plan->ops_bytes.data());
         const size_t n_ops = plan->ops_bytes.size() / sizeof(DevOp<Real>);
-        for (size_t p = 0; p < plan->passes.size(); p++) pass(plan->passes[p], ops, n_ops, p + 1 == plan->passes.size());
+        // one permutation pass instead of the swaps when that saves a pass of
+        // theirs: 15 qubits and up for a QFT.  Below, every pass has gates to
+        // run, and the swaps ride along at less than a pass's fixed cost.
+        TileArgs perm;
+        size_t passes = plan->passes.size(), first = passes;
+        while (first > 0 && only_swaps(plan->passes[first - 1], ops)) first--;
+        drop_swaps = first < passes && first > 0 && global == 1.0 && !swaps.empty() && permutation(swaps, perm);
+        if (drop_swaps) passes = first;
+        for (size_t p = 0; p < passes; p++) pass(plan->passes[p], ops, n_ops, p + 1 == passes);
+        if (drop_swaps) plan->tiles.push_back(perm);
     }
 };
 
 }  // namespace
 
-void lower_plan(Plan *plan, cplx global) {
+void lower_plan(Plan *plan, cplx global, const std::vector<std::pair<int, int>> &swaps) {
     plan->stream.clear();
     plan->tiles.clear();
-    if (plan->precision == HGM_F64) Lowering<double>(plan, global).run();
-    else Lowering<float>(plan, global).run();
+    if (plan->precision == HGM_F64) Lowering<double>(plan, global).run(swaps);
+    else Lowering<float>(plan, global).run(swaps);
 }
 
 }  // namespace hgm

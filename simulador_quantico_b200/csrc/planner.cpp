@@ -513,7 +513,7 @@ bool emit_phase_block(const std::vector<SOp> &ops, std::vector<int> &rest, const
 // instead of a record per gate).
 template <typename Real>
 bool emit_xset(const std::vector<SOp> &ops, std::vector<int> &rest, const Roles &ro, const int loc_of[64],
-               uint64_t tmask, std::vector<DevOp<Real>> &out) {
+               uint64_t tmask, int tail, std::vector<DevOp<Real>> &out) {
     constexpr int cap = xset_entries<Real>();
     std::vector<int> members;
     uint8_t ent[cap][4];
@@ -557,6 +557,8 @@ bool emit_xset(const std::vector<SOp> &ops, std::vector<int> &rest, const Roles 
     memset(&d, 0, sizeof d);
     d.kind = K_XSET;
     d.tpos = (int32_t)members.size();
+    for (size_t k = 0; k < members.size(); k++)
+        if (members[k] >= tail) d.pad1 |= 1u << k;
     memcpy(d.m, ent, members.size() * 4);
     out.push_back(d);
     std::vector<int> keep;
@@ -604,10 +606,10 @@ bool split_gate(const cplx m[4], double rm[4], cplx &s, cplx &p, cplx &q) {
 // front (K_XSET); else the first remaining gate on its own record.
 // With `split`, a layer of complex gates that all have the split form
 // (split_gate) goes out as K_LAYER_SPLIT; their scalars s multiply into
-// `global`.
+// `global`.  Records of ops from index `tail` on (swap_tail) are marked in pad1.
 template <typename Real>
 void emit_phase(const std::vector<SOp> &ops, std::vector<int> rest, const Roles &ro, int R, const int loc_of[64],
-                uint64_t tmask, bool split, cplx &global, std::vector<DevOp<Real>> &out) {
+                uint64_t tmask, bool split, int tail, cplx &global, std::vector<DevOp<Real>> &out) {
     std::vector<int> keep;
     while (!rest.empty()) {
         if (emit_phase_block<Real>(ops, rest, ro, R, loc_of, tmask, 3, out)) continue;
@@ -699,12 +701,13 @@ void emit_phase(const std::vector<SOp> &ops, std::vector<int> rest, const Roles 
             }
         } else if (found != 1 && emit_phase_block<Real>(ops, rest, ro, R, loc_of, tmask, 2, out)) {
             continue;
-        } else if (emit_xset<Real>(ops, rest, ro, loc_of, tmask, out)) {
+        } else if (emit_xset<Real>(ops, rest, ro, loc_of, tmask, tail, out)) {
             // relabeling X gates as late as the schedule allows: fewer later
             // gates see a relabeled bit
             continue;
         } else {
             out.push_back(encode<Real>(ops[rest[0]], ro, loc_of, tmask));
+            if (rest[0] >= tail) out.back().pad1 = 1u;
             keep.assign(rest.begin() + 1, rest.end());
         }
         rest.swap(keep);
@@ -776,6 +779,32 @@ bool lean_ops(const std::vector<DevOp<Real>> &d, int R) {
     return true;
 }
 
+// The swaps that end an op list: CNOT triples (c, t), (t, c), (c, t) on
+// disjoint pairs of index bits, as a QFT's qubit reversal.  Returns the index
+// of the first of them and their pairs.
+int swap_tail(const std::vector<SOp> &ops, std::vector<std::pair<int, int>> &pairs) {
+    auto cnot = [](const SOp &o, int &c, int &t) {
+        if (o.mc != MC_ANTI || o.m[1] != 1.0 || o.m[2] != 1.0 || __builtin_popcountll(o.cmask) != 1 || o.cval != o.cmask)
+            return false;
+        c = __builtin_ctzll(o.cmask);
+        t = o.target;
+        return true;
+    };
+    uint64_t used = 0;
+    size_t i = ops.size();
+    for (; i >= 3; i -= 3) {
+        int c[3], t[3];
+        bool ok = true;
+        for (int k = 0; k < 3 && ok; k++) ok = cnot(ops[i - 3 + k], c[k], t[k]);
+        if (!ok || c[1] != t[0] || t[1] != c[0] || c[2] != c[0] || t[2] != t[0]) break;
+        const uint64_t b = (uint64_t(1) << c[0]) | (uint64_t(1) << t[0]);
+        if (used & b) break;
+        used |= b;
+        pairs.push_back({std::min(c[0], t[0]), std::max(c[0], t[0])});
+    }
+    return (int)i;
+}
+
 template <typename Real>
 int build_tiled(const std::vector<SOp> &ops, int n, const hgm_plan_opts &o, Plan *plan) {
     const int W = plan->warp_bits;
@@ -796,6 +825,8 @@ int build_tiled(const std::vector<SOp> &ops, int n, const hgm_plan_opts &o, Plan
 
     // product of the scalars split layers leave out (emit_phase)
     cplx global = 1.0;
+    std::vector<std::pair<int, int>> swaps;
+    const int tail = swap_tail(ops, swaps);
     OpList list((int)ops.size());
     std::vector<int> pass_ops;
     int pass_index = 0;
@@ -961,7 +992,7 @@ int build_tiled(const std::vector<SOp> &ops, int n, const hgm_plan_opts &o, Plan
             ph.op_begin = (int)dev_ops.size();
             Roles ro(plan->layouts[lay], R, W);
             for (int t = 0; t < 5 + W; t++) ro.thr_gbit[t] = pa.tb[plan->layouts[lay].pos[t]];
-            emit_phase<Real>(ops, taken, ro, R, loc_of, tmask, o.split_layers != 0, global, dev_ops);
+            emit_phase<Real>(ops, taken, ro, R, loc_of, tmask, o.split_layers != 0, tail, global, dev_ops);
             ph.op_end = (int)dev_ops.size();
             ph.xwarp = 0;
             if (cur >= 0 && cur != lay) {
@@ -1015,7 +1046,8 @@ int build_tiled(const std::vector<SOp> &ops, int n, const hgm_plan_opts &o, Plan
     plan->lean = lean_ops<Real>(dev_ops, R);
     plan->ops_bytes.resize(dev_ops.size() * sizeof(DevOp<Real>));
     if (!dev_ops.empty()) memcpy(plan->ops_bytes.data(), dev_ops.data(), plan->ops_bytes.size());
-    lower_plan(plan, global);
+    plan->low_bits = L;
+    lower_plan(plan, global, swaps);
     return HGM_OK;
 }
 

@@ -136,7 +136,7 @@ class Plan:
         check(lib.hgm_plan_export(self.h, C.byref(passes), C.byref(npa), None, C.byref(nph), None, C.byref(nb),
                                   C.byref(wb), C.byref(small)))
         # bytes copied to the device when the plan is uploaded: the passes' streams
-        check(lib.hgm_plan_stream(self.h, None, C.byref(nb)))
+        check(lib.hgm_plan_stream(self.h, None, C.byref(nb), None, None))
         upload = nb.value
         # register bits from the first pass's tile bits (struct PassArgs: n, k, ...): k = 5 + R + W
         reg_bits = 4 if self.precision == HGM_F64 else 5

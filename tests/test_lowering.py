@@ -22,20 +22,55 @@ WINDOW = 176
 plan_export = emu.export
 
 
+TILE_DT = np.dtype([("ld_gbit", "i1", 16), ("st_gbit", "i1", 16), ("run_pos", "i1", 16), ("run_len", "i1", 16),
+                    ("ld_tstep", "<u4", 8), ("stream", "<u8"), ("units", "<i4", 2), ("n", "<i4"), ("k", "<i4"),
+                    ("flags", "<i4"), ("nruns", "<i4"), ("ctl", "<u8", 3), ("pass", "<i4"), ("pairs", "<i4")])
+PERMUTE, PERM_BITS = 4, 10
+
+
 def stream_units(plan):
-    p, n = C.c_void_p(), C.c_int64()
-    check(lib.hgm_plan_stream(plan.h, C.byref(p), C.byref(n)))
-    return np.frombuffer(C.string_at(p, n.value), "<u4").reshape(-1, 4)
+    p, n, t, nt = C.c_void_p(), C.c_int64(), C.c_void_p(), C.c_int64()
+    check(lib.hgm_plan_stream(plan.h, C.byref(p), C.byref(n), C.byref(t), C.byref(nt)))
+    return (np.frombuffer(C.string_at(p, n.value), "<u4").reshape(-1, 4),
+            np.frombuffer(C.string_at(t, nt.value * TILE_DT.itemsize), TILE_DT))
+
+
+def permuted(tile, v):
+    """A permutation pass on the state v, as the kernel walks it: sub-tile u to the place of its partner."""
+    n = int(tile["n"])
+    gb, to = [int(x) for x in tile["ld_gbit"][:PERM_BITS]], [int(x) for x in tile["st_gbit"][:PERM_BITS]]
+    pairs = tile["ld_tstep"].view("i1").astype(int)[:2 * int(tile["pairs"])].reshape(-1, 2)
+    assert not tile["units"].any() and not tile["stream"]  # the kernels fetch nothing for it
+    j = np.arange(1 << PERM_BITS)
+    place = sum(((j >> q) & 1) << gb[q] for q in range(PERM_BITS))
+    moved = sum(((j >> q) & 1) << to[q] for q in range(PERM_BITS))
+    assert sorted(moved) == list(range(1 << PERM_BITS))
+    u = np.arange(1 << (n - PERM_BITS))
+    base, shift = np.zeros_like(u), 0
+    for k in range(int(tile["nruns"])):
+        ln = int(tile["run_len"][k])
+        base |= ((u >> shift) & ((1 << ln) - 1)) << int(tile["run_pos"][k])
+        shift += ln
+    assert shift == n - PERM_BITS
+    other = base.copy()
+    for a, b in pairs:
+        x = ((other >> a) ^ (other >> b)) & 1
+        other ^= (x << a) | (x << b)
+    out = np.full_like(v, np.nan)
+    out[other[:, None] | place[moved][None, :]] = v[base[:, None] | place[None, :]]
+    return out
 
 
 def lowered_export(plan, prec):
     """emu.export's form of what the stream says."""
     e = plan_export(plan, prec)
-    units = stream_units(plan)
+    units, tiles = stream_units(plan)
     real, esz = ("<f8", 16) if prec == "f64" else ("<f4", 8)
     odt = e["ops"].dtype
     W = e["W"]
-    recs, phases, passes = [], [], e["passes"].copy()
+    steps = tiles[tiles["flags"] == 0]
+    assert (np.diff(steps["pass"]) > 0).all()
+    recs, phases, passes = [], [], e["passes"][steps["pass"]].copy()
     at = 0
 
     def vals(u0, u1):
@@ -56,11 +91,12 @@ def lowered_export(plan, prec):
     for pi in range(len(passes)):
         R = int(passes[pi]["k"]) - 5 - W
         pad = lambda j: (j + (j >> R)) * esz
-        steps = {}
+        layout_of = {}
         for li, lay in enumerate(e["layouts"]):
-            steps[tuple(pad(1 << int(lay[k])) for k in range(5 + W + R))] = li
+            layout_of[tuple(pad(1 << int(lay[k])) for k in range(5 + W + R))] = li
         passes[pi]["phase_begin"] = len(phases)
         layout, begin, xwarp = int(passes[pi]["load_layout"]), len(recs), 0
+        assert int(steps[pi]["stream"]) == 16 * at and not units[at][0] & 0xFF == S_NEXT
         window, named = at, []
         sizes = []
         while True:
@@ -82,7 +118,7 @@ def lowered_export(plan, prec):
                 thr = [int(x) for x in units[at + 3:at + 5].reshape(-1)]
                 assert tuple(old[:R]) == tuple(pad(1 << int(p)) for p in e["layouts"][layout][5 + W:5 + W + R])
                 phases.append((layout, begin, len(recs), xwarp))
-                layout, begin, xwarp = steps[tuple(thr[:5 + W] + new[:R])], len(recs), int(bool(w[1] & 2))
+                layout, begin, xwarp = layout_of[tuple(thr[:5 + W] + new[:R])], len(recs), int(bool(w[1] & 2))
             elif kind in (S_ROT, S_SPLIT, S_REAL, S_DENSE):
                 per = {S_ROT: 4, S_SPLIT: 8, S_REAL: 4, S_DENSE: 8}[kind]
                 v = vals(body, at + n)
@@ -160,7 +196,9 @@ def lowered_export(plan, prec):
         assert named == [sizes[k + 2] if k + 2 < len(sizes) else 0 for k in range(len(sizes) - 1)] + [0]
         phases.append((layout, begin, len(recs), xwarp))
         passes[pi]["phase_end"] = len(phases)
-        assert layout == int(passes[pi]["store_layout"])
+        assert list(steps[pi]["units"]) == (sizes + [0])[:2]
+        passes[pi]["store_layout"], passes[pi]["store_xwarp"] = layout, 1
+        passes[pi]["st_gbit"] = steps[pi]["st_gbit"]
     assert at == len(units)
     ph = np.array(phases, emu.PHASE_DT) if phases else np.zeros(0, emu.PHASE_DT)
     ops = np.array(recs, odt) if recs else np.zeros(0, odt)
@@ -171,7 +209,10 @@ def both(monkeypatch, plan, prec, n, seed):
     v = random_state(n, seed=seed, dtype=np.complex128)
     want = emu.run(plan, prec, v)
     monkeypatch.setattr(emu, "export", lowered_export)
-    return emu.run(plan, prec, v), want
+    got = emu.run(plan, prec, v)
+    tiles = stream_units(plan)[1]
+    assert not (tiles["flags"][:-1] & PERMUTE).any()
+    return (permuted(tiles[-1], got) if tiles["flags"][-1] & PERMUTE else got), want
 
 
 def chain_of_phases(n, depth):
@@ -224,6 +265,56 @@ def test_stream_is_the_plan(monkeypatch, name, prec):
     # products of both in other ways: at most 300 gates in a row here
     scale = max(1.0, np.abs(want).max())
     assert np.abs(got - want).max() <= 1e-12 * scale
+
+
+def swap_ending(n, pairs, seed):
+    """Gates, then swaps of the given pairs of index bits."""
+    c = random_gate_circuit_spec(n, 40, seed=seed).build(sq.Circuit())
+    for a, b in pairs:
+        for ctl, t in ((a, b), (b, a), (a, b)):
+            c.append_op(t, 1 << ctl, 1 << ctl, [0, 1, 1, 0])
+    return c
+
+
+SWAPS = [(17, [(q, 16 - q) for q in range(8)]), (18, [(q, 17 - q) for q in range(9)]),
+         (19, [(0, 18), (1, 2), (3, 9), (4, 17), (5, 16), (6, 15), (7, 14)]), (20, [(q, 19 - q) for q in range(10)]),
+         (17, [(0, 1), (2, 3), (4, 16), (5, 15), (6, 14), (7, 13), (8, 12), (9, 11)]), (20, [(q + 4, 19 - q) for q in range(8)])]
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("n,pairs", SWAPS)
+def test_final_swaps(monkeypatch, n, pairs, prec):
+    plan = sq.Plan(swap_ending(n, pairs, n), n, prec)
+    got, want = both(monkeypatch, plan, prec, n, seed=n)
+    assert np.abs(got - want).max() <= 1e-12
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_qft_ends_in_one_permutation(prec):
+    """From 15 qubits the reversal's passes become one; below, and where the pairs cannot be split, the CNOTs stay."""
+    for n in range(12, 29):
+        plan = sq.Plan(wl.qft(n).build(sq.Circuit()), n, prec)
+        flags = stream_units(plan)[1]["flags"]
+        assert (flags == PERMUTE).sum() == (1 if n >= (15 if prec == "f32" else 14) else 0)
+        assert len(flags) <= plan.stats()["passes"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("chained", [1, 0])
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("n,pairs", SWAPS)
+def test_final_swaps_on_the_device(n, pairs, prec, chained):
+    sq.init()
+    plan = sq.Plan(swap_ending(n, pairs, n), n, prec, chained=chained, renorm_every=3 if prec == "f32" else 0)
+    v = random_state(n, seed=n, dtype=np.complex128 if prec == "f64" else np.complex64)
+    want = v.astype(np.complex128)
+    for _ in range(2):
+        want = emu.run(plan, prec, want)
+    st = sq.State(n, prec).upload(v)
+    got = st.execute(plan, 2).download()
+    plan.status()
+    st.free()
+    assert np.abs(got - want).max() <= (1e-12 if prec == "f64" else 2e-5)
 
 
 @pytest.mark.gpu
