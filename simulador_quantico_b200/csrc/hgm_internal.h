@@ -257,7 +257,7 @@ enum StreamKind : uint32_t {
     S_REAL = 5,   // real 2x2s on the register bits of w1: m00, m01, m10, m11 per bit
     S_DENSE = 6,  // complex 2x2s on the register bits of w1: 8 values per bit
     S_XSET = 7,   // w1 relabeling X gates (K_XSET entries), the first two in w2, w3
-    S_CSWAP = 8,  // X on register bit w1 where (label & w2) == w3
+    S_CSWAP = 8,  // X on register bit w1 (bits 0..15) where label bit w1 >> 16 is w2
     S_SCALE = 9,  // FP64: every amplitude times the factor in w2, w3
     S_PHASES = 10,  // phase block of compact terms; w1: K_PHASE_BLOCK flags (cm_reg), w2: active
                     // categories (cv_reg), w3: units from the head to the table (0: none); then

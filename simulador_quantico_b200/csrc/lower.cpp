@@ -52,7 +52,8 @@ bool make_rot(const double *m, double p_re, double p_im, Rot &r) {
     const double num = r.x ? c : s, den = r.x ? s : c, e = r.x ? -d : d;
     r.t = num / den;
     const double sq = 1.0 + r.t * r.t;
-    r.kappa = den;
+    // from the rounded t, so that kappa sqrt(1 + t^2) is Rm's own factor
+    r.kappa = std::copysign(std::hypot(c, s) / std::sqrt(sq), den);
     r.u = -r.t / sq;
     r.pr = e * p_re * sq;
     r.pi = e * p_im * sq;
@@ -168,8 +169,8 @@ struct Lowering {
     }
 
     void gate(const DevOp<Real> &d) {
-        if (d.kind == K_SWAP && d.tpos < R && !d.cm_thr && !d.cm_glob && d.cm_reg) {
-            add(S_CSWAP, {0u, (uint32_t)d.tpos, d.cm_reg, d.cv_reg});
+        if (d.kind == K_SWAP && d.tpos < R && !d.cm_thr && !d.cm_glob && __builtin_popcount(d.cm_reg) == 1) {
+            add(S_CSWAP, {0u, (uint32_t)d.tpos | (uint32_t)__builtin_ctz(d.cm_reg) << 16, d.cv_reg ? 1u : 0u, 0u});
             return;
         }
         std::vector<uint32_t> op = {0u, (uint32_t)d.kind | ((uint32_t)d.tpos << 8), d.cm_reg, d.cv_reg,

@@ -149,7 +149,7 @@ def lowered_export(plan, prec):
                     rec(emu.K_SWAP, t, thr=(1 << cb, cv << cb) if ck == emu.XSET_CTRL_THREAD else (0, 0),
                         glob=(1 << cb, cv << cb) if ck == emu.XSET_CTRL_GLOBAL else (0, 0))
             elif kind == S_CSWAP:
-                rec(emu.K_SWAP, w[1], w[2], w[3])
+                rec(emu.K_SWAP, w[1] & 0xFFFF, 1 << (w[1] >> 16), w[2] << (w[1] >> 16))
             elif kind == S_SCALE:
                 f = struct.unpack("<d", struct.pack("<II", w[2], w[3]))[0]
                 rec(emu.K_DIAG, 0, m=[f, 0, 0, 0, 0, 0, f, 0])
