@@ -51,6 +51,15 @@ namespace hgm {
 #ifndef HGM_SMEM_CARVEOUT
 #define HGM_SMEM_CARVEOUT -1
 #endif
+// Programmatic dependent launch.  A kernel launched behind another one on its
+// stream (launch_behind, kernels.cu) starts while that one's last blocks run,
+// fetches what does not depend on it -- the plan's records -- and waits here
+// until it is complete and its writes are visible.  Every block that touches a
+// state or a plan's scratch waits first.
+__device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the kernel behind this one start once every block has got here.
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <typename Real, int R>
 constexpr int pass_max_regs() {
     return sizeof(Real) == 8 ? HGM_MAXREG_F64 : HGM_MAXREG_F32;
