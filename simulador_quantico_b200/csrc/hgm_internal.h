@@ -7,6 +7,7 @@
 #include <complex>
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -364,6 +365,13 @@ struct Plan {
     // it (plan_lease / plan_unlease, engine.cpp).
     int leases = 0;
     bool free_pending = false;
+    // UNROLL runs of the circuit planned as one (engine.cpp unrolled_plan),
+    // built when a call first asks for enough iterations; the ops it is built
+    // from are kept only for states that can.
+    std::vector<Op> ops;
+    hgm_plan_opts opts;
+    std::unique_ptr<Plan> unrolled;
+    bool no_unroll = false;           // tried: it saves no pass, or found no memory
     ~Plan();
 };
 
