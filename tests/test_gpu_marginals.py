@@ -63,3 +63,15 @@ def test_norm_and_measure_from_one_read(sq, n, prec):
     one = p[(np.arange(1 << n) >> (n - 1)) & 1 == 1].sum()
     assert outcome == 1 and abs(q - one) < 1e-12
     st.free()
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("n", [1, 2, 9, 10, 11, 12, 13, 21])
+def test_set_basis(sq, n, prec):
+    """Every size from less than a block's run to many, first, last and odd indices."""
+    st = sq.State(n, prec)
+    for index in sorted({0, 1, (1 << n) - 1, (1 << n) // 3, (1 << n) // 2}):
+        st.upload(np.full(1 << n, 2 + 3j))
+        got = st.set_basis(index).download()
+        assert got[index] == 1 and np.count_nonzero(got) == 1
+    st.free()
