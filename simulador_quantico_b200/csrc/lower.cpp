@@ -285,7 +285,12 @@ struct Lowering {
             terms.push_back(t);
         }
         const int nrec = head.tpos;
-        const bool table = head.cm_reg & PB_HAS_TABLE;
+        // a table of ones (a QFT block's on its lowest register bit) is left out
+        bool table = false;
+        for (int r = 0; (head.cm_reg & PB_HAS_TABLE) && r < (1 << R); r++) {
+            const DevOp<Real> &z = rec[1 + nrec - (1 << R) / 4 + r / 4];
+            table = table || z.m[2 * (r & 3)] != (Real)1 || z.m[2 * (r & 3) + 1] != (Real)0;
+        }
         const int tab_units = table ? (int)((size_t(1) << R) * 2 * sizeof(Real) / 16) : 0;
         const int fit = ((int)CAP - 3 - tab_units) / tu;
         int done = 0;
@@ -304,8 +309,8 @@ struct Lowering {
             }
             uint32_t flags = head.cm_reg;
             if (!(last && done == 0)) flags &= ~PB_GATED;
-            if (!last) flags &= ~PB_HAS_TABLE;
             const bool tab = last && table;
+            if (!tab) flags &= ~PB_HAS_TABLE;
             std::vector<uint32_t> op = {0u, flags, act, tab ? (uint32_t)(3 + take * tu) : 0u};
             op.resize(12);
             memcpy(&op[4], cnt, 16);

@@ -178,8 +178,11 @@ def lowered_export(plan, prec):
                         rec(emu.K_DIAG, int(units[u][2]), m=[f[0], f[1], 0, 0, 0, 0, f[2], f[3]],
                             thr=(int(units[u][0]), int(units[u][1])), glob=(int(g[0]), int(g[1])))
                 assert bool(w[1] & 1) == bool(w[3])
-                if w[3]:
-                    tab = vals(at + w[3], at + n)
+                tab = vals(at + w[3], at + n) if w[3] else np.tile([1.0, 0.0], 1 << R)
+                if w[1] & emu.PB_GATED or w[3]:
+                    # a table of ones is left out; the emulator's gated form wants it
+                    head["cm_reg"] |= 1
+                    recs[hi] = head
                     assert len(tab) == 2 << R
                     for q in range((1 << R) // 4):
                         rec(0, 0, m=tab[8 * q:8 * q + 8])
