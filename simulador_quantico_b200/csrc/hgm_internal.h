@@ -122,6 +122,8 @@ constexpr uint32_t PB_ANGLES = 2u;
 // leaves such a table out).
 constexpr uint32_t PB_GATED = 4u;
 constexpr int PB_GATE_SHIFT = 8;
+// Device stream only: the first phase block of its layout in the pass.
+constexpr uint32_t PB_FRESH = 8u;
 
 
 // Target location codes inside a phase: 0..R-1 register bit, 8+q thread bit q

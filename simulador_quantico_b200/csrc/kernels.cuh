@@ -997,19 +997,28 @@ struct GatedSweep<Real, A2, R, R> {
 };
 
 // S_PHASES: `op` is the op's head in the stream window, hdr its first unit.
-template <typename Real, typename A2, int R>
+// tix: the thread bits at their index bits.  KEEP: computed by the first block
+// after a layout change (PB_FRESH) and kept for the others (60 of 500
+// instructions a block; 27-qubit FP32 QFT 2.98 -> 2.89 ms, 26-qubit FP64 2.71 ->
+// 2.61).  The chained kernels compute it for each block: kept, its registers
+// cost their layered circuits 1%.
+template <typename Real, typename A2, int R, int W, bool KEEP>
 __device__ __forceinline__ void apply_phase_block_angles(A2 (&a)[1 << R], const unsigned char *__restrict__ op,
-                                                         const uint4 hdr, uint64_t base, uint32_t thr, uint32_t xr) {
+                                                         const uint4 hdr, uint64_t base, uint32_t thr, uint32_t xr,
+                                                         uint64_t &tix) {
     const uint32_t flags = hdr.y, act = hdr.z;
     const Real *__restrict__ table = reinterpret_cast<const Real *>(op + 16 * hdr.w);
     const uint4 cnt = reinterpret_cast<const uint4 *>(op)[1];
-    const uint2 tg = reinterpret_cast<const uint2 *>(op)[4];
-    uint64_t ix = base;
+    if (!KEEP || (flags & PB_FRESH)) {
+        const uint2 tg = reinterpret_cast<const uint2 *>(op)[4];
+        tix = 0;
 #pragma unroll
-    for (int t = 0; t < 8; t++) {
-        const uint32_t g = ((t < 4 ? tg.x : tg.y) >> (8 * (t & 3))) & 63u;
-        ix |= (uint64_t)((thr >> t) & 1u) << g;
+        for (int t = 0; t < 5 + W; t++) {
+            const uint32_t g = ((t < 4 ? tg.x : tg.y) >> (8 * (t & 3))) & 63u;
+            tix |= (uint64_t)((thr >> t) & 1u) << g;
+        }
     }
+    const uint64_t ix = base | tix;
     const unsigned char *rec0 = op + 48;
     if ((flags & PB_GATED) && __all_sync(0xffffffffu, xr == 0u)) {
         // only G[b] terms, then D[b] terms (the walk order with every other
@@ -1291,7 +1300,8 @@ __device__ __forceinline__ void store_tile(const typename V2<Real>::T (&a)[1 << 
 // kernel sets it per position in the pass sequence, in shared memory, where it
 // costs the tile no registers).  The scale is read through L2: in a chained
 // run it was accumulated by other CTAs of the same launch.
-template <typename Real, int R, int W, bool LEAN>
+// KEEP_IX: apply_phase_block_angles.
+template <typename Real, int R, int W, bool LEAN, bool KEEP_IX>
 __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], typename V2<Real>::T *__restrict__ state,
                                             const TileArgs &ta, uint64_t base, unsigned char *sm,
                                             const PassCtl &ctl) {
@@ -1311,6 +1321,7 @@ __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], t
 #pragma unroll
     for (int b = 0; b < 5 + W; b++) tb += ((thr >> b) & 1u) * ta.ld_tstep[b];
     uint32_t xr = 0;            // register relabeling
+    uint64_t tix = 0;           // thread bits at their index bits (phase blocks)
     uint32_t pc = 0;            // byte offset in the two windows
     uint32_t next = ta.units0 + ta.units1;  // first unit not fetched yet
     fetch_wait();
@@ -1354,7 +1365,7 @@ __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], t
             const uint32_t c = hdr.y >> 16;
             controlled_swap<A2, R, 0>(hdr.y & 0xffffu, c, a, ((xr >> c) & 1u) == hdr.z);
         } else if (kind == S_PHASES) {
-            apply_phase_block_angles<Real, A2, R>(a, op, hdr, base, thr, xr);
+            apply_phase_block_angles<Real, A2, R, W, KEEP_IX>(a, op, hdr, base, thr, xr, tix);
         } else if (F64 && kind == S_SCALE) {
             const Real f = (Real)__hiloint2double((int)hdr.w, (int)hdr.z);
 #pragma unroll
@@ -1493,7 +1504,7 @@ __device__ __forceinline__ void run_tile(typename V2<Real>::T *__restrict__ stat
     const uint64_t base = tile_base(tile, ta);
     A2 a[1 << R];
     load_tile<Real, R, W>(a, state, ta, base, threadIdx.x);
-    finish_tile<Real, R, W, LEAN>(a, state, ta, base, sm, ctl);
+    finish_tile<Real, R, W, LEAN, !PERM>(a, state, ta, base, sm, ctl);
 }
 
 }  // namespace hgm

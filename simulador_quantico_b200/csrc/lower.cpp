@@ -80,6 +80,7 @@ struct Lowering {
     std::vector<size_t> windows;   // units of each finished window
     static constexpr size_t CAP = STREAM_WINDOW_UNITS - 1;  // one unit for S_NEXT or S_END
 
+    bool fresh = true;       // no phase block of compact terms in this layout yet
     bool drop_swaps = false; // the marked records are left to a permutation pass
 
     Lowering(Plan *p, cplx gl) : plan(p), global(gl), R(p->reg_bits), W(p->warp_bits) {}
@@ -166,6 +167,7 @@ struct Lowering {
         for (int q = 0; q < 4; q++) op.push_back(reg_step(t, q));
         for (int b = 0; b < 8; b++) op.push_back(thread_step(t, b));
         add(S_TRANS, op);
+        fresh = true;
     }
 
     void gate(const DevOp<Real> &d) {
@@ -311,6 +313,10 @@ struct Lowering {
             if (!(last && done == 0)) flags &= ~PB_GATED;
             const bool tab = last && table;
             if (!tab) flags &= ~PB_HAS_TABLE;
+            if (angles && fresh) {
+                flags |= PB_FRESH;
+                fresh = false;
+            }
             std::vector<uint32_t> op = {0u, flags, act, tab ? (uint32_t)(3 + take * tu) : 0u};
             op.resize(12);
             memcpy(&op[4], cnt, 16);
@@ -332,6 +338,7 @@ struct Lowering {
         out.clear();
         window.clear();
         windows.clear();
+        fresh = true;
         int cur = pa.load_layout;
         bool prev_cross = false;
         auto go_to = [&](int layout) {
