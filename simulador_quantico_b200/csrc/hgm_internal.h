@@ -55,11 +55,8 @@ struct Circuit {
 // Register layouts of a tile (kernels.cuh).  A layout gives every role of
 // a thread's view of the tile its local tile bit: thread bits t = 0..4+W
 // (lanes 0..4, then warps) at pos[t], register bits q = 0..R-1 at
-// pos[5 + W + q].  On the device a layout is a table of LAYOUT_HDR words
-// (byte offset in the transpose buffer of each register bit's unit step)
-// followed by one word per thread (byte offset of its register 0).
+// pos[5 + W + q].
 constexpr int MAX_LAYOUT_ROLES = 16;
-constexpr int LAYOUT_HDR = 8;
 struct Lay {
     int8_t pos[MAX_LAYOUT_ROLES];
 };
@@ -208,20 +205,17 @@ constexpr int MAX_TILE_BITS = 16;
 // Runs of consecutive non-tile index bits: at most one more than tile bits.
 constexpr int MAX_FREE_RUNS = MAX_TILE_BITS + 2;
 
+// A pass of the plan (its lowered form, which the kernels take, is TileArgs).
 struct PassArgs {
     int32_t n;            // qubits
     int32_t k;            // tile bits = 5 + R + W
     int32_t phase_begin, phase_end;
     int32_t load_layout, store_layout;  // layout table indices
-    int32_t flags;        // PASS_* below
+    int32_t flags;        // 0
     int32_t store_xwarp;  // the transpose into the store layout crosses warps
     int8_t tb[MAX_TILE_BITS];  // local tile bit -> global index bit
     uint64_t tile_mask;
-    const DevPhase *phases;
-    const void *ops;      // DevOp<Real>*
-    double *norm_out;     // PASS_NORM: accumulate sum |a|^2 of stored amplitudes
-    const double *scale_in; // PASS_SCALE: multiply loaded amplitudes by 1/sqrt(*scale_in)
-    const uint32_t *layouts;  // layout table, LAYOUT_HDR + 2^(5+W) words per layout
+    const void *unused[5];  // null: fields of the exported record that nothing reads
     // The non-tile index bits as runs, lowest first: the tile number's next
     // run_len[i] bits go to index bits run_pos[i] .. run_pos[i] + run_len[i] - 1.
     int8_t run_pos[MAX_FREE_RUNS];
@@ -232,8 +226,8 @@ struct PassArgs {
     int8_t st_gbit[MAX_LAYOUT_ROLES];
 };
 
-constexpr int32_t PASS_NORM = 1;
-constexpr int32_t PASS_SCALE = 2;
+constexpr int32_t PASS_NORM = 1;   // accumulate the sum of |a|^2 of the stored amplitudes
+constexpr int32_t PASS_SCALE = 2;  // multiply the loaded amplitudes by 1/sqrt(*scale_in)
 constexpr int32_t PASS_PERMUTE = 4;  // a permutation pass (below), no stream
 
 // ---- device stream -----------------------------------------------------------
@@ -337,7 +331,7 @@ struct Plan {
     int reg_bits = 5;                 // amplitudes per thread = 2^reg_bits
     int low_bits = 0;                 // index bits 0.. that load and store layouts keep on thread bits
     bool small = false;               // n < 5 + reg_bits: single-CTA shared-memory path
-    std::vector<PassArgs> passes;     // device pointers patched after upload
+    std::vector<PassArgs> passes;
     std::vector<DevPhase> phases;
     std::vector<Lay> layouts;         // every layout the phases use
     std::vector<unsigned char> ops_bytes;   // DevOp<Real>[] or SmallOp<Real>[]
@@ -353,8 +347,8 @@ struct Plan {
     int renorm_every = 0;
     double *d_norm = nullptr;         // renormalisation scratch (FP32 plans)
     // Chained execution (launch_plan_chain), set up at upload for states of
-    // at most CHAIN_MAX_BYTES: the pass records on the device and the
-    // scratch (counters, error word, chain_slots renormalisation slots).
+    // at most CHAIN_MAX_BYTES: the tiles on the device and the scratch
+    // (counters, error word, chain_slots renormalisation slots).
     void *d_chain = nullptr;
     void *d_chain_passes = nullptr;
     int64_t chain_slots = 0;

@@ -1,6 +1,8 @@
 // Kernels and launchers of the state-vector engine (sm_100a).
 //
 //   pass_kernel<Real, W>   one state pass of a plan (kernels.cuh: run_tile)
+//   permute_kernel<Real>   a plan's final swaps as one pass
+//   chain_kernel<Real, W>  every pass of a small state in one launch
 //   small_kernel<Real>     states of < 10 qubits: whole state in one CTA's
 //                          shared memory, gates applied one by one
 //   reduce_*               FP64 reductions (norm, bit probability, inner

@@ -7,8 +7,12 @@
 // holds 2^(5+R) and the CTA 2^W warps.  The tile is the set of state
 // indices that agree on every index bit outside the pass's K tile bits;
 // local tile bit q is index bit tb[q].  Which local bits are the lane,
-// warp and register bits of a thread is the current phase's layout, a table
-// the planner builds (struct Lay): any R local bits can be the register bits.
+// warp and register bits of a thread is the current phase's layout, chosen by
+// the planner (struct Lay): any R local bits can be the register bits.
+//
+// What a tile goes through -- gates, phase blocks, transposes -- comes as one
+// stream of 16-byte units (hgm_internal.h, "device stream"), copied into
+// shared memory a window ahead (fetch_stream, finish_tile).
 //
 // A gate whose target is a register bit of the current layout is applied
 // entirely in registers.  Switching layout is a transpose through shared
@@ -16,7 +20,7 @@
 // each warp (__syncwarp), otherwise it crosses warps (__syncthreads).  The
 // load and store layouts put thread bits 0..low_bits-1 on the lowest index
 // bits of the state, so each warp instruction moves whole 128-byte runs.
-// Shared memory is padded (pad_slot below); the planner only builds layouts
+// Shared memory is padded (below); the planner only builds layouts
 // whose accesses are free of bank conflicts under that padding.
 //
 // State loads and stores bypass L1 (ld/st .cg): every amplitude is touched
@@ -36,9 +40,9 @@ namespace hgm {
 
 // Register budget per thread.  The FP32 tile (32 float2) and the FP64 tile
 // (16 double2) both hold 64 data registers.  128 lets 4 CTAs of 4 warps share
-// an SM; the pass kernel is latency-bound, and the fourth CTA outweighs the
-// spills the cap brings (26-qubit layered passes: FP64 -13%, FP32 -2%, QFT
-// -12% against a 168-register cap with 3 CTAs per SM).
+// an SM; the pass kernel is latency-bound (26-qubit layered passes: FP64 -13%, FP32 -2%, QFT
+// -12% against a 168-register cap with 3 CTAs per SM; five CTAs of 96 registers
+// spill: 26-qubit FP32 layered 13.3 -> 14.2 ms, FP64 searches a third slower).
 #ifndef HGM_MAXREG_F32
 #define HGM_MAXREG_F32 128
 #endif
@@ -76,15 +80,11 @@ struct V2<float> {
     using T = float2;
 };
 
-// Shared-memory slot of local index j in a transpose: j + (j >> R).  The
-// padding keeps every layout's warp accesses free of bank conflicts (a lane
-// stride of 2^R elements becomes 2^R + 1) and, unlike an XOR swizzle, it is
-// additive over a layout's disjoint lane/warp and register bits, so the slot
-// of register r is the thread's base slot plus r times a constant.
-template <int R>
-__device__ __forceinline__ uint32_t pad_slot(uint32_t j) {
-    return j + (j >> R);
-}
+// Shared-memory slot of local index j in a transpose: j + (j >> R) (lower.cpp
+// slot).  The padding keeps every layout's warp accesses free of bank conflicts
+// (a lane stride of 2^R elements becomes 2^R + 1) and, unlike an XOR swizzle,
+// it is additive over a layout's disjoint lane/warp and register bits, so the
+// slot of register r is the thread's base slot plus r times a constant.
 
 // Shared memory of one tile's transposes, in amplitudes.
 template <int R, int W>

@@ -155,6 +155,7 @@ struct Lowering {
         if (!(a < 0x1p200 && a > 0x1p-200)) add_scale();
     }
 
+    // byte offset in the transpose buffer of local index j (kernels.cuh)
     uint32_t slot(uint32_t j) const { return (j + (j >> R)) * (uint32_t)(2 * sizeof(Real)); }
     uint32_t reg_step(const Lay &l, int q) const { return q < R ? slot(1u << l.pos[5 + W + q]) : 0u; }
     uint32_t thread_step(const Lay &l, int b) const { return b < 5 + W ? slot(1u << l.pos[b]) : 0u; }

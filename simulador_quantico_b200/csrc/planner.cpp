@@ -130,7 +130,7 @@ struct Roles {
 };
 
 // Builds layouts.  Every layout keeps a warp's shared-memory accesses free of
-// bank conflicts: with slot(j) = j + (j >> R) (kernels.cuh pad_slot), the
+// bank conflicts: with slot(j) = j + (j >> R) (lower.cpp slot), the
 // unit slot of local bit q is 1, 2, 4, 8 (mod 8 for 16-byte, mod 16 for
 // 8-byte amplitudes) exactly for q = i or q = i + R, i < NB, where NB = 3
 // (FP64: a quarter warp per 128-byte wavefront) or 4 (FP32: a half warp).

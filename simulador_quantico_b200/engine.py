@@ -135,15 +135,18 @@ class Plan:
         passes = C.c_void_p()
         check(lib.hgm_plan_export(self.h, C.byref(passes), C.byref(npa), None, C.byref(nph), None, C.byref(nb),
                                   C.byref(wb), C.byref(small)))
-        # bytes copied to the device when the plan is uploaded: the passes' streams
-        check(lib.hgm_plan_stream(self.h, None, C.byref(nb), None, None))
+        # bytes copied to the device when the plan is uploaded (the passes' streams), and the passes as
+        # launched: a circuit's final swaps may run as one permutation pass
+        run = C.c_int64()
+        check(lib.hgm_plan_stream(self.h, None, C.byref(nb), None, C.byref(run)))
         upload = nb.value
         # register bits from the first pass's tile bits (struct PassArgs: n, k, ...): k = 5 + R + W
         reg_bits = 4 if self.precision == HGM_F64 else 5
         if npa.value and passes.value:
             reg_bits = C.cast(passes, C.POINTER(C.c_int32))[1] - 5 - wb.value
         return dict(ops=v[0].value, passes=v[1].value, phases=v[2].value, transposes=v[3].value,
-                    warp_bits=wb.value, reg_bits=reg_bits, small=bool(small.value), upload_bytes=upload)
+                    warp_bits=wb.value, reg_bits=reg_bits, small=bool(small.value), upload_bytes=upload,
+                    passes_run=run.value)
 
 
 class State:
