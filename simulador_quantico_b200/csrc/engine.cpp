@@ -41,7 +41,7 @@ std::mutex g_lease_mu;
 
 void free_plan_now(Plan *pl) {
     // launches are asynchronous: the plan's device records may still be in use
-    if (pl->d_ops || pl->d_norm) cudaDeviceSynchronize();
+    if (pl->uploaded) cudaDeviceSynchronize();
     delete pl;
 }
 }  // namespace

@@ -340,12 +340,13 @@ struct Plan {
     std::vector<TileArgs> tiles;      // stream holds the offset until upload_plan patches it
     int64_t n_small_ops = 0;
     int64_t n_ops = 0, n_transposes = 0;
-    // device copies, and their sizes as allocated
+    // device copies, all of them or none (uploaded), and their sizes as allocated
+    bool uploaded = false;
     DevAllocator *allocator = nullptr;
     size_t d_bytes[4] = {0, 0, 0, 0};  // stream (or small ops), norm, chain scratch, chain passes
     void *d_ops = nullptr;
     int renorm_every = 0;
-    double *d_norm = nullptr;         // renormalisation scratch (FP32 plans)
+    void *d_norm = nullptr;           // renormalisation scratch (FP32 plans): 64 doubles
     // Chained execution (launch_plan_chain), set up at upload for states of
     // at most CHAIN_MAX_BYTES: the tiles on the device and the scratch
     // (counters, error word, chain_slots renormalisation slots).

@@ -226,8 +226,7 @@ int launch_plan_steps(State *s, const Plan *p, int iterations, PlanCursor *c, in
     if (s->precision != p->precision) return fail(HGM_ERR_INVALID, "plan and state precision differ");
     // every device pointer a launch passes must exist: an op list that was
     // never uploaded is refused here, not read through a null pointer
-    if (((!p->ops_bytes.empty() || !p->stream.empty()) && !p->d_ops) || (p->renorm_every > 0 && !p->small && !p->d_norm))
-        return fail(HGM_ERR_INVALID, "plan used before upload_plan");
+    if (!p->uploaded) return fail(HGM_ERR_INVALID, "plan used before upload_plan");
     cudaStream_t st = pick(stream);
     if (!st) return HGM_ERR_CUDA;
     if (p->small) {
@@ -245,12 +244,12 @@ int launch_plan_steps(State *s, const Plan *p, int iterations, PlanCursor *c, in
         TileArgs pa = p->tiles[g % np];
         if (c->scale_next) {
             pa.ctl.flags |= PASS_SCALE;
-            pa.ctl.scale_in = p->d_norm + c->scale_slot;
+            pa.ctl.scale_in = (const double *)p->d_norm + c->scale_slot;
             c->scale_next = false;
         }
         if (R > 0 && ((g + 1) % R == 0) && g + 1 < total) {
             pa.ctl.flags |= PASS_NORM;
-            pa.ctl.norm_out = p->d_norm + c->slot;
+            pa.ctl.norm_out = (double *)p->d_norm + c->slot;
             cudaMemsetAsync(pa.ctl.norm_out, 0, sizeof(double), st);
             c->scale_next = true;
             c->scale_slot = c->slot;
@@ -512,7 +511,7 @@ static int launch_chain_w(State *s, const Plan *p, int iterations, cudaStream_t 
 }
 
 bool chain_eligible(const Plan *p, int iterations) {
-    return !p->small && p->d_chain && p->tiles.size() >= 2 && iterations >= 1;
+    return p->uploaded && !p->small && p->d_chain && p->tiles.size() >= 2 && iterations >= 1;
 }
 
 int launch_plan_chain(State *s, const Plan *p, int iterations, void *stream) {
@@ -541,59 +540,80 @@ int launch_plan(State *s, const Plan *p, int iterations, void *stream) {
 // plan upload
 // ---------------------------------------------------------------------------
 
-static cudaError_t plan_alloc(Plan *p, int k, void **out, size_t bytes) {
-    p->d_bytes[k] = bytes;
-    return p->allocator ? p->allocator->alloc(out, bytes) : cudaMalloc(out, bytes);
+static void *&plan_block(Plan *p, int k) {
+    if (k == 0) return p->d_ops;
+    if (k == 1) return p->d_norm;
+    return k == 2 ? p->d_chain : p->d_chain_passes;
 }
 
-Plan::~Plan() {
-    void *ptrs[4] = {d_ops, d_norm, d_chain, d_chain_passes};
+static void release_blocks(Plan *p) {
     for (int k = 0; k < 4; k++) {
-        if (!ptrs[k]) continue;
-        if (allocator) allocator->free(ptrs[k], d_bytes[k]);
-        else cudaFree(ptrs[k]);
+        void *&d = plan_block(p, k);
+        if (!d) continue;
+        if (p->allocator) p->allocator->free(d, p->d_bytes[k]);
+        else cudaFree(d);
+        d = nullptr;
     }
 }
 
-int upload_plan(Plan *p) {
-    const void *src = p->small ? (const void *)p->ops_bytes.data() : (const void *)p->stream.data();
-    const size_t bytes = p->small ? p->ops_bytes.size() : p->stream.size() * sizeof(uint32_t);
-    if (p->d_ops || p->d_norm || (!bytes && !p->renorm_every)) return HGM_OK;
-    if (ensure_ctx()) return HGM_ERR_CUDA;
-    cudaError_t e;
-    if (bytes) {
-        if ((e = plan_alloc(p, 0, &p->d_ops, bytes)) != cudaSuccess)
-            return fail(HGM_ERR_NOMEM, "plan ops: %s", cudaGetErrorString(e));
-        if ((e = cudaMemcpy(p->d_ops, src, bytes, cudaMemcpyHostToDevice)) != cudaSuccess)
-            return fail(HGM_ERR_CUDA, "plan ops copy: %s", cudaGetErrorString(e));
-    }
-    if (p->renorm_every > 0) {
-        if ((e = plan_alloc(p, 1, (void **)&p->d_norm, 64 * sizeof(double))) != cudaSuccess)
-            return fail(HGM_ERR_NOMEM, "plan norm slots: %s", cudaGetErrorString(e));
-    }
-    for (TileArgs &t : p->tiles)
-        if (!(t.flags & PASS_PERMUTE)) t.stream = (const unsigned char *)p->d_ops + reinterpret_cast<size_t>(t.stream);
+Plan::~Plan() { release_blocks(this); }
+
+// Allocates the plan's device memory and copies it there.  On failure the
+// caller releases what was allocated.
+static int upload_blocks(Plan *p) {
     const int64_t state_bytes = (int64_t(1) << p->qubits) * (p->precision == HGM_F64 ? 16 : 8);
-    if (p->chained && !p->small && p->tiles.size() >= 2 && state_bytes <= CHAIN_MAX_BYTES) {
-        // chained execution: the pass records (pointers patched) and the scratch
-        p->chain_slots = p->renorm_every > 0 ? CHAIN_NORM_SLOTS : 0;
-        const size_t sb = (4 + (size_t)p->chain_slots) * sizeof(double);
-        const size_t pb = p->tiles.size() * sizeof(TileArgs);
-        if ((e = plan_alloc(p, 2, &p->d_chain, sb)) != cudaSuccess)
-            return fail(HGM_ERR_NOMEM, "plan chain scratch: %s", cudaGetErrorString(e));
-        // zero for the first launch; every launch leaves it so
-        if ((e = cudaMemset(p->d_chain, 0, sb)) != cudaSuccess)
-            return fail(HGM_ERR_CUDA, "plan chain scratch: %s", cudaGetErrorString(e));
-        if ((e = plan_alloc(p, 3, &p->d_chain_passes, pb)) != cudaSuccess)
-            return fail(HGM_ERR_NOMEM, "plan chain passes: %s", cudaGetErrorString(e));
-        if ((e = cudaMemcpy(p->d_chain_passes, p->tiles.data(), pb, cudaMemcpyHostToDevice)) != cudaSuccess)
-            return fail(HGM_ERR_CUDA, "plan chain passes copy: %s", cudaGetErrorString(e));
+    const bool chain = p->chained && !p->small && p->tiles.size() >= 2 && state_bytes <= CHAIN_MAX_BYTES;
+    p->chain_slots = chain && p->renorm_every > 0 ? CHAIN_NORM_SLOTS : 0;
+    const size_t bytes[4] = {
+        p->small ? p->ops_bytes.size() : p->stream.size() * sizeof(uint32_t),
+        p->renorm_every > 0 ? 64 * sizeof(double) : 0,
+        chain ? (4 + (size_t)p->chain_slots) * sizeof(double) : 0,
+        chain ? p->tiles.size() * sizeof(TileArgs) : 0,
+    };
+    if (!bytes[0] && !bytes[1]) return HGM_OK;  // a plan without gates
+    static const char *const what[4] = {"plan ops", "plan norm slots", "plan chain scratch", "plan chain passes"};
+    cudaError_t e;
+    for (int k = 0; k < 4; k++) {
+        if (!bytes[k]) continue;
+        p->d_bytes[k] = bytes[k];
+        void *&d = plan_block(p, k);
+        if ((e = p->allocator ? p->allocator->alloc(&d, bytes[k]) : cudaMalloc(&d, bytes[k])) != cudaSuccess) {
+            d = nullptr;
+            return fail(HGM_ERR_NOMEM, "%s: %s", what[k], cudaGetErrorString(e));
+        }
     }
+    if (ensure_ctx()) return HGM_ERR_CUDA;
+    // the passes with their streams' device addresses; the plan keeps the
+    // offsets until the upload is complete, so that it can be tried again
+    std::vector<TileArgs> tiles = p->tiles;
+    for (TileArgs &t : tiles)
+        if (!(t.flags & PASS_PERMUTE)) t.stream = (const unsigned char *)p->d_ops + reinterpret_cast<size_t>(t.stream);
+    const void *const src[4] = {p->small ? (const void *)p->ops_bytes.data() : (const void *)p->stream.data(), nullptr,
+                                nullptr, tiles.data()};
+    for (int k = 0; k < 4; k++)
+        if (bytes[k] && src[k] && (e = cudaMemcpy(plan_block(p, k), src[k], bytes[k], cudaMemcpyHostToDevice)) != cudaSuccess)
+            return fail(HGM_ERR_CUDA, "%s copy: %s", what[k], cudaGetErrorString(e));
+    // zero for the first launch; every launch leaves it so
+    if (chain && (e = cudaMemset(p->d_chain, 0, bytes[2])) != cudaSuccess)
+        return fail(HGM_ERR_CUDA, "plan chain scratch: %s", cudaGetErrorString(e));
     // a copy from pageable memory may return before its last piece has
     // reached the device, and the plan's launches go to non-blocking streams,
     // which do not wait for it
     if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess)
         return fail(HGM_ERR_CUDA, "plan upload: %s", cudaGetErrorString(e));
+    p->tiles.swap(tiles);
+    return HGM_OK;
+}
+
+int upload_plan(Plan *p) {
+    if (p->uploaded) return HGM_OK;
+    const int rc = upload_blocks(p);
+    if (rc) {  // nothing half done: a later call starts over, and no launch finds some of the memory
+        release_blocks(p);
+        cudaGetLastError();
+        return rc;
+    }
+    p->uploaded = true;
     return HGM_OK;
 }
 
