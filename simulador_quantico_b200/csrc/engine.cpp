@@ -320,12 +320,18 @@ int hgm_execute(hgm_state *s, const hgm_plan *p, int iterations, void *stream) {
     // a state that fits in L2 runs every pass in one chained launch
     if (plan_launches(pl, iterations) > 1 && chain_eligible(pl, iterations))
         return launch_plan_chain(reinterpret_cast<State *>(s), pl, iterations, stream);
+    PlanCursor c;
+    c.norms = (double *)pl->d_norm;
     if (Plan *u = unrolled_plan(pl, iterations, stream)) {
-        rc = launch_plan(reinterpret_cast<State *>(s), u, iterations / UNROLL, stream);
+        c.more = iterations % UNROLL != 0;
+        rc = launch_plan_steps(reinterpret_cast<State *>(s), u, iterations / UNROLL, &c,
+                               plan_launches(u, iterations / UNROLL), stream);
         iterations %= UNROLL;
         if (rc || !iterations) return rc;
+        c.then_plan();
+        c.more = false;
     }
-    return launch_plan(reinterpret_cast<State *>(s), pl, iterations, stream);
+    return launch_plan_steps(reinterpret_cast<State *>(s), pl, iterations, &c, plan_launches(pl, iterations), stream);
 }
 
 int hgm_plan_status(const hgm_plan *p) {

@@ -407,12 +407,20 @@ struct State {
 // ---- launchers (kernels.cu) ----------------------------------------------------
 int launch_plan(State *s, const Plan *p, int iterations, void *stream);
 // The same in pieces: queues up to max_launches more launches of the plan
-// from cursor c (which carries the renormalisation slots across calls).
+// from cursor c.  Plans run one after the other as one sequence share a
+// cursor (then_plan between them), so that a rescale falls on every
+// renorm_every-th pass of the sequence.
 struct PlanCursor {
-    int64_t next = 0;
+    int64_t next = 0;    // the plan's next launch
+    int64_t before = 0;  // passes of the plans before it
+    bool more = false;   // another plan follows
     int slot = 0;
-    bool scale_next = false;
-    int scale_slot = 0;
+    double *norms = nullptr;           // the slots: the first plan's
+    const double *scale_in = nullptr;  // the next pass rescales by this slot
+    void then_plan() {
+        before += next;
+        next = 0;
+    }
 };
 int launch_plan_steps(State *s, const Plan *p, int iterations, PlanCursor *c, int64_t max_launches, void *stream);
 int64_t plan_launches(const Plan *p, int iterations);

@@ -242,17 +242,17 @@ int launch_plan_steps(State *s, const Plan *p, int iterations, PlanCursor *c, in
     for (int64_t k = 0; k < max_launches && c->next < total; k++, c->next++) {
         const int64_t g = c->next;
         TileArgs pa = p->tiles[g % np];
-        if (c->scale_next) {
+        if (c->scale_in) {
             pa.ctl.flags |= PASS_SCALE;
-            pa.ctl.scale_in = (const double *)p->d_norm + c->scale_slot;
-            c->scale_next = false;
+            pa.ctl.scale_in = c->scale_in;
+            c->scale_in = nullptr;
         }
-        if (R > 0 && ((g + 1) % R == 0) && g + 1 < total) {
+        if (R > 0 && (c->before + g + 1) % R == 0 && (c->more || g + 1 < total)) {
+            if (!c->norms) c->norms = (double *)p->d_norm;
             pa.ctl.flags |= PASS_NORM;
-            pa.ctl.norm_out = (double *)p->d_norm + c->slot;
+            pa.ctl.norm_out = c->norms + c->slot;
             cudaMemsetAsync(pa.ctl.norm_out, 0, sizeof(double), st);
-            c->scale_next = true;
-            c->scale_slot = c->slot;
+            c->scale_in = pa.ctl.norm_out;
             c->slot = (c->slot + 1) % 64;
         }
         if (pa.flags & PASS_PERMUTE) {
