@@ -63,14 +63,15 @@ constexpr double UNROLL_WORTH_US = 500.0, PASS_BYTES_PER_US = 6.0e6;
 
 int64_t state_bytes(const Plan *p) { return (int64_t(1) << p->qubits) * (p->precision == HGM_F64 ? 16 : 8); }
 
-std::mutex g_unroll_mu;
-
-// The unrolled plan for a call of `iterations`, or null where the plan itself serves.
+// The unrolled plan for a call of `iterations`, or null where the plan itself
+// serves: also while another thread builds the longer plan, and while there is
+// no memory for it (a later call tries again).
 Plan *unrolled_plan(Plan *p, int iterations, void *stream) {
     if (p->small || p->ops.empty() || iterations < UNROLL) return nullptr;
     if (iterations * (2.0 * (double)state_bytes(p) / PASS_BYTES_PER_US) < UNROLL_WORTH_US) return nullptr;
-    std::lock_guard<std::mutex> lk(g_unroll_mu);
-    if (p->unrolled || p->no_unroll) return p->unrolled.get();
+    std::unique_lock<std::mutex> lk(p->unroll_mu, std::try_to_lock);
+    if (!lk.owns_lock() || p->no_unroll) return nullptr;
+    if (p->unrolled && p->unrolled->uploaded) return p->unrolled.get();
     // building allocates device memory, which a capture forbids
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream ? (cudaStream_t)stream : (cudaStream_t)default_stream(), &cap) != cudaSuccess ||
@@ -78,18 +79,20 @@ Plan *unrolled_plan(Plan *p, int iterations, void *stream) {
         cudaGetLastError();
         return nullptr;
     }
-    std::vector<Op> ops;
-    ops.reserve(p->ops.size() * UNROLL);
-    for (int k = 0; k < UNROLL; k++) ops.insert(ops.end(), p->ops.begin(), p->ops.end());
-    std::unique_ptr<Plan> u(new Plan());
-    u->allocator = p->allocator;
-    if (build_plan(ops, p->qubits, p->opts, u.get()) || u->tiles.size() >= p->tiles.size() * UNROLL || upload_plan(u.get())) {
-        cudaGetLastError();
-        p->no_unroll = true;
-        return nullptr;
+    if (!p->unrolled) {
+        std::vector<Op> ops;
+        ops.reserve(p->ops.size() * UNROLL);
+        for (int k = 0; k < UNROLL; k++) ops.insert(ops.end(), p->ops.begin(), p->ops.end());
+        std::unique_ptr<Plan> u(new Plan());
+        u->allocator = p->allocator;
+        if (build_plan(ops, p->qubits, p->opts, u.get()) || u->tiles.size() >= p->tiles.size() * UNROLL) {
+            p->no_unroll = true;
+            return nullptr;
+        }
+        p->unrolled = std::move(u);
     }
-    p->unrolled = std::move(u);
-    return p->unrolled.get();
+    OutsideCapture elsewhere;
+    return upload_plan(p->unrolled.get()) ? nullptr : p->unrolled.get();
 }
 
 }  // namespace

@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -314,6 +315,16 @@ struct SmallOp {
     Real m[8];
 };
 
+// While one of these lives, the calling thread may allocate although another
+// thread captures a CUDA graph in the global mode (torch's default), which
+// would refuse the allocation and lose that thread its capture.
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    OutsideCapture(const OutsideCapture &) = delete;
+};
+
 // ---- plan ------------------------------------------------------------------
 // Where a plan's device records come from: cudaMalloc/cudaFree by default, or
 // an owner's cache (the server recycles them, so that serving makes no
@@ -368,8 +379,9 @@ struct Plan {
     // from are kept only for states that can.
     std::vector<Op> ops;
     hgm_plan_opts opts;
-    std::unique_ptr<Plan> unrolled;
-    bool no_unroll = false;           // tried: it saves no pass, or found no memory
+    std::mutex unroll_mu;             // held by the thread that looks for or builds it
+    std::unique_ptr<Plan> unrolled;   // runs once it is uploaded
+    bool no_unroll = false;           // planned: it saves nothing
     ~Plan();
 };
 

@@ -33,6 +33,7 @@ constexpr size_t MARGINAL_SCRATCH = size_t(2) << 20;
 struct Ctx {
     int device = -1;
     cudaStream_t stream = nullptr;
+    cudaStream_t upload = nullptr; // plan uploads
     double *partials = nullptr;    // RED_BLOCKS * 2 doubles
     long long *partial_idx = nullptr;
     double *host_result = nullptr; // 4 doubles (pinned; kernels write it)
@@ -59,7 +60,8 @@ static int ensure_ctx() {
     cudaStream_t s;
     if ((e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)) != cudaSuccess)
         return fail(HGM_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
-    if ((e = cudaMalloc(&g_ctx.partials, RED_BLOCKS * 2 * sizeof(double))) != cudaSuccess ||
+    if ((e = cudaStreamCreateWithFlags(&g_ctx.upload, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaMalloc(&g_ctx.partials, RED_BLOCKS * 2 * sizeof(double))) != cudaSuccess ||
         (e = cudaMalloc(&g_ctx.partial_idx, RED_BLOCKS * sizeof(long long))) != cudaSuccess ||
         (e = cudaMalloc(&g_ctx.marginal, MARGINAL_SCRATCH)) != cudaSuccess ||
         (e = cudaMallocHost(&g_ctx.host_result, 4 * sizeof(double))) != cudaSuccess ||
@@ -591,15 +593,15 @@ static int upload_blocks(Plan *p) {
     const void *const src[4] = {p->small ? (const void *)p->ops_bytes.data() : (const void *)p->stream.data(), nullptr,
                                 nullptr, tiles.data()};
     for (int k = 0; k < 4; k++)
-        if (bytes[k] && src[k] && (e = cudaMemcpy(plan_block(p, k), src[k], bytes[k], cudaMemcpyHostToDevice)) != cudaSuccess)
+        if (bytes[k] && src[k] &&
+            (e = cudaMemcpyAsync(plan_block(p, k), src[k], bytes[k], cudaMemcpyHostToDevice, g_ctx.upload)) != cudaSuccess)
             return fail(HGM_ERR_CUDA, "%s copy: %s", what[k], cudaGetErrorString(e));
     // zero for the first launch; every launch leaves it so
-    if (chain && (e = cudaMemset(p->d_chain, 0, bytes[2])) != cudaSuccess)
+    if (chain && (e = cudaMemsetAsync(p->d_chain, 0, bytes[2], g_ctx.upload)) != cudaSuccess)
         return fail(HGM_ERR_CUDA, "plan chain scratch: %s", cudaGetErrorString(e));
-    // a copy from pageable memory may return before its last piece has
-    // reached the device, and the plan's launches go to non-blocking streams,
-    // which do not wait for it
-    if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess)
+    // the plan's launches go to other streams, which do not wait for the copies.
+    // (Not the legacy stream: it takes no work while a blocking stream captures.)
+    if ((e = cudaStreamSynchronize(g_ctx.upload)) != cudaSuccess)
         return fail(HGM_ERR_CUDA, "plan upload: %s", cudaGetErrorString(e));
     p->tiles.swap(tiles);
     return HGM_OK;
@@ -609,6 +611,7 @@ int upload_plan(Plan *p) {
     if (p->uploaded) return HGM_OK;
     const int rc = upload_blocks(p);
     if (rc) {  // nothing half done: a later call starts over, and no launch finds some of the memory
+        if (g_ctx.upload) cudaStreamSynchronize(g_ctx.upload);  // copies into it may be under way
         release_blocks(p);
         cudaGetLastError();
         return rc;
