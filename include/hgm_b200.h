@@ -163,7 +163,13 @@ int hgm_state_download(const hgm_state *s, void *host, int64_t bytes);
  * one persistent launch instead of one launch per pass; that launch's
  * passes wait on each other with a bounded wait (hgm_plan_status).  The
  * chained run's counters and an FP32 plan's renormalisation slots belong to
- * the plan: executions of one plan must not overlap on the device. */
+ * the plan: executions of one plan must not overlap on the device.
+ * The first call of 8 or more iterations on a larger state (a plan of at most
+ * 1024 ops) may plan eight iterations as one: once its first iterations are
+ * queued it plans on the host, allocates and uploads (a millisecond or so, in
+ * which the call has not yet returned and the GPU runs those iterations), and
+ * the plan keeps the longer plan until it is freed.  Never inside a capture on
+ * `stream`; a later call tries again where memory was short. */
 int hgm_execute(hgm_state *s, const hgm_plan *p, int iterations, void *stream);
 /* After the plan's executions have been queued: waits for the device, then
  * HGM_ERR_TIMEOUT if the last chained execution of the plan gave up a wait

@@ -52,47 +52,90 @@ namespace {
 // ---- iterations --------------------------------------------------------------
 // A plan run many times cannot merge the last pass of one run with the first
 // of the next.  Planned UNROLL times over, it can: a Grover iteration of 18 to
-// 26 qubits takes 4.1 passes instead of 5 (26 qubits FP64, 32 iterations: 58.5
-// -> 51.9 ms).  Only for states whose passes are launches of their own
-// (a chained run's pass costs a few microseconds), and only where the passes
-// that a call can save, one a run, are worth the planning and the upload of
-// the longer plan (0.5 ms) at once: a first call is never slower for it.
+// 26 qubits takes 4.1 passes instead of 5.  Only for states whose passes are
+// launches of their own (a chained run's pass costs a few microseconds).
+//
+// The longer plan is built by the first call of at least UNROLL iterations
+// whose own iterations keep the GPU busy meanwhile: as many as cover the
+// planning (plan_us; measured 0.35 us an op on the B200's host) at the least
+// time their passes can take are queued first, and what is left then runs on
+// it.  A call that cannot cover it, and the calls of fewer iterations, run the
+// plan itself.
+//
+// Of the plan's runs and the longer plan the cheaper serves, by passes,
+// transposes and stream units (plan_cost).  Both timed on one B200, eight runs
+// against one longer plan: searches of 22 to 27 qubits 0.88-0.92, 26 qubits
+// FP32 one layer 0.62, two 0.86, ten 0.97, FP64 three layers 0.80, QFTs without
+// their swaps 0.61, random gates 0.35 to 1.04.  Of 49 circuits the rule takes
+// the 28 at 0.35 to 0.996 and leaves 21 at 0.92 to 1.04.  A plan that ends in a
+// permutation pass (a QFT) stays as it is: within the longer plan its swaps are
+// CNOTs again (27 qubits FP32: 101 ms for 32 runs, 208 ms as four longer plans).
 constexpr int UNROLL = 8;
-constexpr size_t UNROLL_MAX_OPS = 2048;
-constexpr double UNROLL_WORTH_US = 500.0, PASS_BYTES_PER_US = 6.0e6;
+constexpr size_t UNROLL_MAX_OPS = 1024;  // beyond, a pass saved is less than 3% of a run
+constexpr double PASS_BYTES_PER_US = 6.6e6;
 
 int64_t state_bytes(const Plan *p) { return (int64_t(1) << p->qubits) * (p->precision == HGM_F64 ? 16 : 8); }
 
-// The unrolled plan for a call of `iterations`, or null where the plan itself
-// serves: also while another thread builds the longer plan, and while there is
-// no memory for it (a later call tries again).
-Plan *unrolled_plan(Plan *p, int iterations, void *stream) {
-    if (p->small || p->ops.empty() || iterations < UNROLL) return nullptr;
-    if (iterations * (2.0 * (double)state_bytes(p) / PASS_BYTES_PER_US) < UNROLL_WORTH_US) return nullptr;
+// Planning and upload of the longer plan, in us.
+double plan_us(const Plan *p) { return 150.0 + 0.5 * UNROLL * (double)p->ops.size(); }
+
+// Iterations that keep the GPU busy for that long.
+int64_t iterations_ahead(const Plan *p) {
+    const double pass_us = 2.0 * (double)state_bytes(p) / PASS_BYTES_PER_US;
+    return (int64_t)std::ceil(plan_us(p) / (pass_us * (double)p->tiles.size()));
+}
+
+// A plan's time in passes over memory: what a pass saved gives back, a
+// transpose, and the ops' 16-byte units.
+double plan_cost(const Plan *p) {
+    return 0.5 * (double)p->tiles.size() + 0.2 * (double)p->n_transposes + 0.03 * (double)(p->stream.size() / 4);
+}
+bool worth_unrolling(const Plan *p, const Plan *u) {
+    return (u->lean || !p->lean) && plan_cost(u) < 0.97 * UNROLL * plan_cost(p);
+}
+
+bool can_unroll(const Plan *p, int iterations) {
+    return !p->small && !p->ops.empty() && !p->tiles.empty() && iterations >= UNROLL && !(p->tiles.back().flags & PASS_PERMUTE);
+}
+
+// The longer plan, if it is ready.
+Plan *unrolled_plan(Plan *p, int iterations) {
+    if (!can_unroll(p, iterations)) return nullptr;
     std::unique_lock<std::mutex> lk(p->unroll_mu, std::try_to_lock);
-    if (!lk.owns_lock() || p->no_unroll) return nullptr;
-    if (p->unrolled && p->unrolled->uploaded) return p->unrolled.get();
-    // building allocates device memory, which a capture forbids
+    return lk.owns_lock() && p->unrolled && p->unrolled->uploaded ? p->unrolled.get() : nullptr;
+}
+
+// Whether this call is to build it: not while another thread does, nor inside
+// a capture, which forbids the allocation.
+bool may_build(Plan *p, int iterations, cudaStream_t st) {
+    if (!can_unroll(p, iterations) || iterations < iterations_ahead(p)) return false;
+    std::unique_lock<std::mutex> lk(p->unroll_mu, std::try_to_lock);
+    if (!lk.owns_lock() || p->no_unroll || (p->unrolled && p->unrolled->uploaded)) return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream ? (cudaStream_t)stream : (cudaStream_t)default_stream(), &cap) != cudaSuccess ||
-        cap != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return nullptr;
-    }
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) return true;
+    cudaGetLastError();
+    return false;
+}
+
+// Builds the longer plan.  Without memory for it, it stays planned and a later
+// call tries the upload again.
+void build_unrolled(Plan *p) {
+    std::unique_lock<std::mutex> lk(p->unroll_mu, std::try_to_lock);
+    if (!lk.owns_lock() || p->no_unroll) return;
     if (!p->unrolled) {
         std::vector<Op> ops;
         ops.reserve(p->ops.size() * UNROLL);
         for (int k = 0; k < UNROLL; k++) ops.insert(ops.end(), p->ops.begin(), p->ops.end());
         std::unique_ptr<Plan> u(new Plan());
         u->allocator = p->allocator;
-        if (build_plan(ops, p->qubits, p->opts, u.get()) || u->tiles.size() >= p->tiles.size() * UNROLL) {
+        if (build_plan(ops, p->qubits, p->opts, u.get()) || !worth_unrolling(p, u.get())) {
             p->no_unroll = true;
-            return nullptr;
+            return;
         }
         p->unrolled = std::move(u);
     }
     OutsideCapture elsewhere;
-    return upload_plan(p->unrolled.get()) ? nullptr : p->unrolled.get();
+    upload_plan(p->unrolled.get());
 }
 
 }  // namespace
@@ -323,18 +366,26 @@ int hgm_execute(hgm_state *s, const hgm_plan *p, int iterations, void *stream) {
     // a state that fits in L2 runs every pass in one chained launch
     if (plan_launches(pl, iterations) > 1 && chain_eligible(pl, iterations))
         return launch_plan_chain(reinterpret_cast<State *>(s), pl, iterations, stream);
+    // the plan, the longer plan and the plan again, as one sequence of passes
+    State *st = reinterpret_cast<State *>(s);
     PlanCursor c;
     c.norms = (double *)pl->d_norm;
-    if (Plan *u = unrolled_plan(pl, iterations, stream)) {
-        c.more = iterations % UNROLL != 0;
-        rc = launch_plan_steps(reinterpret_cast<State *>(s), u, iterations / UNROLL, &c,
-                               plan_launches(u, iterations / UNROLL), stream);
-        iterations %= UNROLL;
-        if (rc || !iterations) return rc;
+    auto run = [&](const Plan *q, int times, int then) {
+        iterations = then;
+        c.more = then > 0;
+        const int err = launch_plan_steps(st, q, times, &c, plan_launches(q, times), stream);
         c.then_plan();
-        c.more = false;
+        return err;
+    };
+    Plan *u = unrolled_plan(pl, iterations);
+    if (!u && may_build(pl, iterations, (cudaStream_t)(stream ? stream : default_stream()))) {
+        const int ahead = (int)iterations_ahead(pl);
+        if ((rc = run(pl, ahead, iterations - ahead))) return rc;
+        build_unrolled(pl);
+        u = unrolled_plan(pl, iterations);
     }
-    return launch_plan_steps(reinterpret_cast<State *>(s), pl, iterations, &c, plan_launches(pl, iterations), stream);
+    if (u && (rc = run(u, iterations / UNROLL, iterations % UNROLL))) return rc;
+    return iterations ? run(pl, iterations, 0) : HGM_OK;
 }
 
 int hgm_plan_status(const hgm_plan *p) {

@@ -108,3 +108,50 @@ int main() {
 def test_no_memory_for_the_longer_plan_is_not_for_good(tmp_path):
     first, second, third, ok = native.run(tmp_path, RETRY).split()
     assert int(third) <= int(second) < int(first) and ok == "1"
+
+
+def test_first_long_call_queues_its_own_iterations_first(sq):
+    """The longer plan is planned while the GPU runs the call's first iterations; it serves the rest."""
+    n, iterations = 22, 24
+    plan = sq.Plan(one_iteration(n, 5).build(sq.Circuit()), n, "f64").upload()
+    assert plan.stats()["passes"] == 5
+    st = sq.State(n, "f64").set_basis(0)
+    l0 = sq.kernel_launches()
+    st.execute(plan, iterations)
+    first = sq.kernel_launches() - l0
+    assert first in [5 * a + 33 * ((24 - a) // 8) + 5 * ((24 - a) % 8) for a in range(1, 17)]
+    st.execute(plan, iterations)
+    assert sq.kernel_launches() - l0 - first == 3 * 33
+
+
+def one_by_one(sq, circuit, n, prec, iterations):
+    """Launches of `iterations` runs, twice; checks them against single runs."""
+    plan = sq.Plan(circuit, n, prec).upload()
+    a, b = sq.State(n, prec).set_basis(3), sq.State(n, prec).set_basis(3)
+    launches = []
+    for _ in range(2):
+        l0 = sq.kernel_launches()
+        a.execute(plan, iterations)
+        launches.append(sq.kernel_launches() - l0)
+        for _ in range(iterations):
+            b.execute(plan)
+    # unitary gates on a unit state, rounded in another order: growth with the
+    # square root of the gates in a row at most, 2 x 24 x 300 of them
+    assert a.max_abs_diff(b) < (1e-13 if prec == "f64" else 2e-5)
+    a.free()
+    b.free()
+    return launches, plan.stats()["passes_run"] * iterations
+
+
+@pytest.mark.parametrize("n,prec", [(22, "f64"), (23, "f32")])
+def test_runs_that_end_in_swaps_stay_single(sq, n, prec):
+    """Only the last of eight QFTs could end in a permutation pass."""
+    launches, single = one_by_one(sq, wl.qft(n, 0).build(sq.Circuit()), n, prec, 24)
+    assert launches == [single, single]
+
+
+@pytest.mark.parametrize("layers,longer", [(2, True), (20, False)])
+def test_plans_are_compared_by_their_time(sq, layers, longer):
+    """Two layers merge over runs; twenty are as many gates in as many passes, and more planning than the runs cover."""
+    launches, single = one_by_one(sq, wl.random_layered(23, layers, 3).build(sq.Circuit()), 23, "f32", 24)
+    assert (launches[1] < single) == longer and launches[0] <= single
