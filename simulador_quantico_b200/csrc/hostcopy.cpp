@@ -27,6 +27,8 @@
 
 #include <atomic>
 #include <cstring>
+#include <exception>
+#include <functional>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -137,6 +139,22 @@ void stage_d2h(Stager &s, size_t chunk, int t, char *host, const char *dev, size
 
 }  // namespace
 
+// share(0) .. share(n - 1), each on a thread of its own and the first on this
+// one; where no thread can be started (std::system_error, which must not leave
+// a C entry), this one takes that share too.
+void run_shares(int n, const std::function<void(int)> &share) {
+    std::vector<std::thread> th;
+    int t = 1;
+    try {
+        th.reserve(n);
+        for (; t < n; t++) th.emplace_back(share, t);
+    } catch (const std::exception &) {
+    }
+    share(0);
+    for (; t < n; t++) share(t);
+    for (std::thread &x : th) x.join();
+}
+
 int plain_copy(void *dst, const void *src, size_t bytes, bool to_device, cudaStream_t st) {
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -186,10 +204,7 @@ int copy_state(void *dst, const void *src, size_t bytes, bool to_device, void *s
         if (to_device) stage_h2d(s, chunk, t, (char *)dst, (const char *)src, bytes, &err);
         else stage_d2h(s, chunk, t, (char *)dst, (const char *)src, bytes, &err);
     };
-    std::vector<std::thread> th;
-    for (int t = 1; t < kThreads; t++) th.emplace_back(run, t);
-    run(0);
-    for (std::thread &x : th) x.join();
+    run_shares(kThreads, run);
     return err.load() ? fail(HGM_ERR_CUDA, "staged state copy failed") : HGM_OK;
 }
 

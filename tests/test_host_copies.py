@@ -39,3 +39,55 @@ def test_page_locked_round_trip(sq, n):
     check(lib.hgm_state_download(st.h, C.c_void_p(b.ptr), b.nbytes))
     assert np.array_equal(a.array, b.array) and np.array_equal(st.download(), a.array)
     st.free()
+
+
+# pthread_create of the program's own: it fails where `fail_from` says so
+THREADS = r"""
+#include <dlfcn.h>
+#include <pthread.h>
+#include <atomic>
+#include <cerrno>
+#include <functional>
+#include <thread>
+static std::atomic<int> started{0}, fail_from{1 << 30};
+extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *x) {
+    if (started++ >= fail_from) return EAGAIN;
+    return ((int (*)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *))dlsym(RTLD_NEXT, "pthread_create"))(t, a, f, x);
+}
+namespace hgm { void run_shares(int n, const std::function<void(int)> &share); }
+int main(int argc, char **argv) {
+    if (atoi(argv[1])) {  // whole copies
+        const int n = 18;
+        const size_t bytes = size_t(16) << n;
+        hgm_state *s;
+        double *a = (double *)malloc(bytes), *b = (double *)malloc(bytes);
+        for (size_t i = 0; i < bytes / 8; i++) a[i] = (double)i;
+        if (hgm_init(0) || hgm_state_create(n, HGM_F64, &s)) return 2;
+        for (int k = 0; k < 4; k++) {
+            for (size_t i = 0; i < bytes / 8; i++) b[i] = 0;
+            started = 0;
+            fail_from = k;
+            if (hgm_state_upload(s, a, bytes) || hgm_state_download(s, b, bytes)) return 3;
+            for (size_t i = 0; i < bytes / 8; i++)
+                if (b[i] != a[i]) return 4;
+        }
+    }
+    for (int k = 0; k < 4; k++) {
+        std::atomic<int> done[4] = {};
+        started = 0;
+        fail_from = k;
+        run_shares(4, [&](int t) { done[t]++; });
+        printf("%d%d%d%d-%d ", (int)done[0], (int)done[1], (int)done[2], (int)done[3], (int)started);
+    }
+}
+"""
+SHARES = ["1111-1", "1111-2", "1111-3", "1111-3"]  # each taken once; the threads asked for
+
+
+def test_every_share_is_taken_without_threads(tmp_path):
+    assert native.run(tmp_path, THREADS, 0).split() == SHARES
+
+
+@pytest.mark.gpu
+def test_copies_without_threads(tmp_path):
+    assert native.run(tmp_path, THREADS, 1).split() == SHARES
