@@ -91,3 +91,48 @@ def test_every_share_is_taken_without_threads(tmp_path):
 @pytest.mark.gpu
 def test_copies_without_threads(tmp_path):
     assert native.run(tmp_path, THREADS, 1).split() == SHARES
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [16, 20])
+def test_two_threads_copy_at_once(sq, n):
+    """Whichever way each copy goes, every one is whole."""
+    import threading
+
+    states = [sq.State(n, "f64") for _ in range(3)]
+    hosts = [np.random.default_rng(k).standard_normal(1 << n) + 1j * k for k in range(3)]
+    bad = []
+
+    def work(k):
+        for r in range(8):
+            states[k].upload(hosts[k] * (r + 1))
+            if not np.array_equal(states[k].download(), hosts[k] * (r + 1)):
+                bad.append((k, r))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    for s in states:
+        s.free()
+
+
+TURNS = r"""
+#include <thread>
+namespace hgm { std::unique_lock<std::mutex> take_chunks(size_t bytes); }
+int main() {
+    const size_t mib = size_t(1) << 20;
+    auto mine = take_chunks(4 * mib), large = take_chunks(256 * mib);
+    auto other = [&] { std::thread([&] { printf("%d", (int)take_chunks(4 * mib).owns_lock()); }).join(); };
+    printf("%d%d", (int)mine.owns_lock(), (int)large.owns_lock());
+    other();
+    mine.unlock();
+    other();
+}
+"""
+
+
+def test_a_second_copy_does_not_wait_for_the_small_set(tmp_path):
+    assert native.run(tmp_path, TURNS) == "1101"
