@@ -458,11 +458,17 @@ int scale_state(State *s, double scale, void *stream);
 
 // Asynchronous FP64 reductions into caller-owned device scratch (used by
 // concurrent clients such as the server's slots): partials holds
-// 2*REDUCE_SCRATCH_BLOCKS doubles, ibest REDUCE_SCRATCH_BLOCKS indices;
-// norm -> out[0]; marginal argmax probability -> out[0], index -> out[1].
+// 2*REDUCE_SCRATCH_BLOCKS doubles, pbest and ibest REDUCE_SCRATCH_BLOCKS
+// entries; norm -> out[0]; marginal argmax probability -> out[0], index -> out[1].
+// The argmax splits its sums over blocks as far as `sums` (n_sums doubles) has
+// room for them: marginal_sums says how many a mask can use, MARG_SUMS at most.
 constexpr int REDUCE_SCRATCH_BLOCKS = 1184;
+constexpr int64_t MARG_BLOCKS = 1024, MARG_SUMS = MARG_BLOCKS << 11;
+int64_t marginal_sums(int qubits, uint64_t mask);
+int marginal_chunks(int qubits, uint64_t mask, long long cap, long long *units);
 int launch_norm_async(State *s, double *partials, double *out, void *stream);
-int launch_argmax_async(State *s, uint64_t mask, double *pbest, long long *ibest, double *out, void *stream);
+int launch_argmax_async(State *s, uint64_t mask, double *pbest, long long *ibest, double *sums, int64_t n_sums,
+                        double *out, void *stream);
 
 void *default_stream();
 void count_launch(int n = 1);

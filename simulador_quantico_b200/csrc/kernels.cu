@@ -28,7 +28,7 @@ namespace hgm {
 namespace {
 constexpr int RED_BLOCKS = REDUCE_SCRATCH_BLOCKS;   // 8 x 148 SMs
 constexpr int RED_THREADS = 256;
-constexpr size_t MARGINAL_SCRATCH = size_t(2) << 20;
+constexpr size_t MARGINAL_SCRATCH = (MARG_SUMS + (size_t(1) << 16)) * sizeof(double);
 
 struct Ctx {
     int device = -1;
@@ -936,7 +936,9 @@ int max_abs_diff(State *a, State *b, double *out, void *stream) {
 // Bound by reading the state once.  25 qubits FP32, 11 bits: 52 us, 5.2 TB/s (one
 // thread per value before, 8 blocks, a bit deposit per element: 17.9 ms; a
 // block's warps on scattered 256-byte runs: 113 us, waiting on DRAM).  The
-// argmax over all 25 bits: 1064 us before, now 42-45 us (6 TB/s).
+// argmax over all 25 bits: 1064 us before, now 42-45 us (6 TB/s).  The plain
+// sums of an FP32 state keep to 32 registers (eight blocks an SM): with 40 the
+// reading of 28 qubits takes 368 us instead of 347.
 constexpr int MARG_WARPS = RED_THREADS / 32;
 constexpr int MARG_LOW = 11, MARG_ACC = 8;
 
@@ -979,11 +981,11 @@ __device__ __forceinline__ void block_best(double &p, long long &i) {
         for (int k = 1; k < MARG_WARPS; k++) keep_best(p, i, sp[k], si[k]);
 }
 
-// ARGMAX: block b's best to pbest[b], ibest[b] (nch must be 1); otherwise
-// unit (x, chunk)'s sum to out[x * nch + chunk].
+// ARGMAX: block b's best to pbest[b], ibest[b] (nch must be 1); otherwise value
+// x's sum over chunk c to out[c * M + x], M values in all.
 template <typename Real, bool ARGMAX>
 __global__ void __launch_bounds__(RED_THREADS) marginal_kernel(const typename V2<Real>::T *__restrict__ s, int n,
-                                                                unsigned long long mask, int nch, double *out,
+                                                                unsigned long long mask, int nch, long long M, double *out,
                                                                 double *pbest, long long *ibest) {
     const int tid = threadIdx.x;
     const int lb = n < MARG_LOW ? n : MARG_LOW, nh = n - lb;
@@ -1055,7 +1057,7 @@ __global__ void __launch_bounds__(RED_THREADS) marginal_kernel(const typename V2
                 for (uint32_t m = mlo, j = 0; m; m &= m - 1, j++) xl |= ((pos >> (__ffs((int)m) - 1)) & 1u) << j;
                 const long long x = (xh << m_lo) | xl;
                 if (ARGMAX) keep_best(best, besti, t, x);
-                else out[x * nch + chunk] = t;
+                else out[chunk * M + x] = t;
             }
         }
         __syncthreads();
@@ -1104,79 +1106,119 @@ __global__ void __launch_bounds__(RED_THREADS) marginal_final(const double *pbes
     }
 }
 
-// Sums each value's chunks, one warp a value.
-__device__ __forceinline__ double chunk_sum(const double *partial, long long x, int nch) {
-    double p = 0.0;
-    for (int k = threadIdx.x & 31; k < nch; k += 32) p += partial[x * nch + k];
-    return warp_sum(p);
-}
-
-__global__ void __launch_bounds__(RED_THREADS) marginal_chunks_final(const double *partial, long long M, int nch,
-                                                                      double *out) {
-    double b = -1.0;
-    long long bi = 0;
-    for (long long x = threadIdx.x >> 5; x < M; x += MARG_WARPS) keep_best(b, bi, chunk_sum(partial, x, nch), x);
-    block_best(b, bi);
-    if (threadIdx.x == 0) {
-        out[0] = b;
-        out[1] = (double)bi;
+// The chunks' sums of every value: `g` values a block's turn, each summed by as
+// many threads as the block has for it, then in a tree over those.  g: four
+// doubles fill a sector, and few values over many chunks want many blocks (32
+// values of 2048 chunks by one block: 20 us more); many values want few turns (2^19
+// values of 2 chunks by fours: 160 us more).  ARGMAX: the block's best, in `out` if it is the only block.
+static int chunk_group(long long M) { return M < 4 ? (int)M : M <= 4096 ? 4 : 32; }
+template <bool ARGMAX>
+__global__ void __launch_bounds__(RED_THREADS) marginal_chunks_kernel(const double *__restrict__ partial, long long M,
+                                                                       int nch, int g, double *out, double *pbest,
+                                                                       long long *ibest) {
+    __shared__ double sh[RED_THREADS];
+    const int tid = threadIdx.x, rows = RED_THREADS / g;
+    double best = -1.0;
+    long long besti = 0;
+    for (long long x0 = (long long)blockIdx.x * g; x0 < M; x0 += (long long)gridDim.x * g) {
+        double p = 0.0;
+#pragma unroll 8
+        for (int c = tid / g; c < nch; c += rows) p += partial[c * M + x0 + (tid & (g - 1))];
+        sh[tid] = p;
+        __syncthreads();
+        for (int h = RED_THREADS / 2; h >= g; h >>= 1) {
+            if (tid < h) sh[tid] += sh[tid + h];
+            __syncthreads();
+        }
+        if (tid < g) {
+            if (ARGMAX) keep_best(best, besti, sh[tid], x0 + tid);
+            else out[x0 + tid] = sh[tid];
+        }
+        __syncthreads();
+    }
+    if (ARGMAX) {
+        block_best(best, besti);
+        if (tid == 0 && gridDim.x == 1) {
+            out[0] = best;
+            out[1] = (double)besti;
+        } else if (tid == 0) {
+            pbest[blockIdx.x] = best;
+            ibest[blockIdx.x] = besti;
+        }
     }
 }
-
-__global__ void __launch_bounds__(RED_THREADS) marginal_chunks_sum(const double *partial, long long M, int nch,
-                                                                    double *out) {
-    for (long long x = (long long)blockIdx.x * MARG_WARPS + (threadIdx.x >> 5); x < M;
-         x += (long long)gridDim.x * MARG_WARPS) {
-        const double p = chunk_sum(partial, x, nch);
-        if ((threadIdx.x & 31) == 0) out[x] = p;
-    }
+static unsigned chunks_grid(long long M) {
+    const long long blocks = M / chunk_group(M);
+    return (unsigned)(blocks < RED_BLOCKS ? blocks : RED_BLOCKS);
 }
 
-// Chunks a unit is split into: until there are blocks for every SM, while the
-// partial sums (M * nch) stay within `cap` and a chunk keeps four runs.
-static int marginal_chunks(int n, uint64_t mask, long long cap, long long *units) {
+// Chunks a unit is split into: until there are RED_BLOCKS blocks while the
+// partial sums (M * nch) are few, then until there are MARG_BLOCKS (MARG_SUMS
+// sums at most, a unit's being 2^11 at most) while the sums are a sixteenth of
+// the amplitudes or there are fewer than 256 blocks; always as long as a chunk keeps
+// four runs and the sums fit `cap`.  FP32, the lowest 8 to 10 bits with 512 and
+// 1024 of MARG_BLOCKS: 25 qubits 86 and 72 us, 28 qubits 484 and 341 us (6.3
+// TB/s); 13.4 and 106 ms where the sums had to fit 2368.
+int marginal_chunks(int n, uint64_t mask, long long cap, long long *units) {
+    constexpr long long FEW = 1 << 16;
     const int lb = n < MARG_LOW ? n : MARG_LOW;
     const long long M = 1ll << __builtin_popcountll(mask), U = 1ll << __builtin_popcountll(mask >> lb);
     const long long C = (1ll << (n - lb)) / U;
     int nch = 1;
-    while (U * nch < RED_BLOCKS && C / nch >= 8 && 2 * M * nch <= cap) nch *= 2;
+    while (U * nch < RED_BLOCKS && C / nch >= 8 && 2 * M * nch <= cap &&
+           (2 * M * nch <= FEW || (U * nch < MARG_BLOCKS && (U * nch < 256 || 2 * M * nch <= (1ll << n) / 16))))
+        nch *= 2;
     *units = U * nch;
     return nch;
 }
 
+int64_t marginal_sums(int n, uint64_t mask) {
+    long long units = 0;
+    const int nch = marginal_chunks(n, mask, MARG_SUMS, &units);
+    return nch > 1 ? (int64_t(1) << __builtin_popcountll(mask)) * nch : 0;
+}
+
 // Queues the marginal argmax of `mask` over state s: its probability and
-// value land in out[0], out[1].  Scratch: pbest of 2 * RED_BLOCKS entries,
-// ibest of RED_BLOCKS.
-static int queue_marginal(State *s, uint64_t mask, double *pbest, long long *ibest, double *out, cudaStream_t st) {
+// value land in out[0], out[1].  Scratch: pbest and ibest of RED_BLOCKS
+// entries, sums of n_sums.
+static int queue_marginal(State *s, uint64_t mask, double *pbest, long long *ibest, double *sums, int64_t n_sums,
+                          double *out, cudaStream_t st) {
     const int n = s->qubits;
     if (n < 64 && (mask >> n)) return fail(HGM_ERR_INVALID, "mask beyond state bits");
     const long long N = 1ll << n, M = 1ll << __builtin_popcountll(mask);
+    unsigned last = 0;  // blocks whose bests are still to be compared
     if (M == N) {
-        const unsigned g = grid_for(N);
+        last = grid_for(N);
         if (s->precision == HGM_F64)
-            argmax_all_kernel<double><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, N, pbest, ibest);
+            argmax_all_kernel<double><<<last, RED_THREADS, 0, st>>>((const double2 *)s->d, N, pbest, ibest);
         else
-            argmax_all_kernel<float><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, N, pbest, ibest);
-        marginal_final<<<1, RED_THREADS, 0, st>>>(pbest, ibest, (int)g, out);
+            argmax_all_kernel<float><<<last, RED_THREADS, 0, st>>>((const float2 *)s->d, N, pbest, ibest);
     } else {
         long long units = 0;
-        const int nch = marginal_chunks(n, mask, 2 * RED_BLOCKS, &units);
-        const unsigned g = (unsigned)(units < RED_BLOCKS ? units : RED_BLOCKS);
+        const int nch = marginal_chunks(n, mask, n_sums, &units);
         if (nch > 1) {
+            const unsigned g = (unsigned)units;
             if (s->precision == HGM_F64)
-                marginal_kernel<double, false><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, nch, pbest, nullptr, nullptr);
+                marginal_kernel<double, false><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, nch, M, sums, nullptr, nullptr);
             else
-                marginal_kernel<float, false><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, nch, pbest, nullptr, nullptr);
-            marginal_chunks_final<<<1, RED_THREADS, 0, st>>>(pbest, M, nch, out);
+                marginal_kernel<float, false><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, nch, M, sums, nullptr, nullptr);
+            const unsigned blocks = chunks_grid(M);
+            marginal_chunks_kernel<true><<<blocks, RED_THREADS, 0, st>>>(sums, M, nch, chunk_group(M), out, pbest, ibest);
+            count_launch();
+            last = blocks > 1 ? blocks : 0;
         } else {
+            last = (unsigned)(units < RED_BLOCKS ? units : RED_BLOCKS);
             if (s->precision == HGM_F64)
-                marginal_kernel<double, true><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, 1, nullptr, pbest, ibest);
+                marginal_kernel<double, true><<<last, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, 1, M, nullptr, pbest, ibest);
             else
-                marginal_kernel<float, true><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, 1, nullptr, pbest, ibest);
-            marginal_final<<<1, RED_THREADS, 0, st>>>(pbest, ibest, (int)g, out);
+                marginal_kernel<float, true><<<last, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, 1, M, nullptr, pbest, ibest);
         }
     }
-    count_launch(2);
+    count_launch();
+    if (last) {
+        marginal_final<<<1, RED_THREADS, 0, st>>>(pbest, ibest, (int)last, out);
+        count_launch();
+    }
     return check("argmax launch");
 }
 
@@ -1190,31 +1232,30 @@ int marginal_probs(State *s, uint64_t mask, double *host_out, void *stream) {
     if (m > 26) return fail(HGM_ERR_UNSUPPORTED, "marginal over %d bits (at most 26)", m);
     const long long M = 1ll << m;
     long long units = 0;
-    const int nch = marginal_chunks(n, mask, 1 << 16, &units);
+    // sums and values within the scratch; a distribution too large for that is
+    // over enough high bits
+    const int nch = marginal_chunks(n, mask, (long long)(MARGINAL_SCRATCH / sizeof(double)) - M, &units);
     const unsigned g = (unsigned)(units < (1 << 16) ? units : (1 << 16));
-    // values, then the chunks' partial sums: from the context's scratch when
+    // the chunks' partial sums, then the values: from the context's scratch when
     // they fit (freeing a stream-ordered allocation at every call's
     // synchronisation returns its pages to the driver)
-    const size_t need = (size_t)(M + (nch > 1 ? M * nch : 0)) * sizeof(double);
+    const long long n_sums = nch > 1 ? M * nch : 0;
+    const size_t need = (size_t)(n_sums + M) * sizeof(double);
     std::lock_guard<std::mutex> lk(g_reduce_mu);
-    double *d_out = g_ctx.marginal;
+    double *sums = g_ctx.marginal;
     cudaError_t e = cudaSuccess;
     if (need > MARGINAL_SCRATCH) {
-        e = cudaMallocAsync(&d_out, need, st);
+        e = cudaMallocAsync(&sums, need, st);
         if (e != cudaSuccess) return fail(HGM_ERR_NOMEM, "marginal output: %s", cudaGetErrorString(e));
     }
-    double *sums = nch > 1 ? d_out + M : d_out;
+    double *d_out = sums + n_sums;
     if (s->precision == HGM_F64)
-        marginal_kernel<double, false><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, nch,
-                                                                        sums, nullptr, nullptr);
+        marginal_kernel<double, false><<<g, RED_THREADS, 0, st>>>((const double2 *)s->d, n, mask, nch, M, sums, nullptr, nullptr);
     else
-        marginal_kernel<float, false><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, nch,
-                                                                       sums, nullptr, nullptr);
+        marginal_kernel<float, false><<<g, RED_THREADS, 0, st>>>((const float2 *)s->d, n, mask, nch, M, sums, nullptr, nullptr);
     count_launch();
     if (nch > 1) {
-        const long long blocks = (M + MARG_WARPS - 1) / MARG_WARPS;
-        marginal_chunks_sum<<<(unsigned)(blocks < RED_BLOCKS ? blocks : RED_BLOCKS), RED_THREADS, 0, st>>>(sums, M, nch,
-                                                                                                          d_out);
+        marginal_chunks_kernel<false><<<chunks_grid(M), RED_THREADS, 0, st>>>(sums, M, nch, chunk_group(M), d_out, nullptr, nullptr);
         count_launch();
     }
     int rc = check("marginal probabilities launch");
@@ -1223,19 +1264,20 @@ int marginal_probs(State *s, uint64_t mask, double *host_out, void *stream) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) rc = fail(HGM_ERR_CUDA, "marginal probabilities: %s", cudaGetErrorString(e));
     }
-    if (need > MARGINAL_SCRATCH) cudaFreeAsync(d_out, st);
+    if (need > MARGINAL_SCRATCH) cudaFreeAsync(sums, st);
     return rc;
 }
 
-int launch_argmax_async(State *s, uint64_t mask, double *pbest, long long *ibest, double *out, void *stream) {
-    return queue_marginal(s, mask, pbest, ibest, out, (cudaStream_t)stream);
+int launch_argmax_async(State *s, uint64_t mask, double *pbest, long long *ibest, double *sums, int64_t n_sums,
+                        double *out, void *stream) {
+    return queue_marginal(s, mask, pbest, ibest, sums, n_sums, out, (cudaStream_t)stream);
 }
 
 int marginal_argmax(State *s, uint64_t mask, int64_t *arg, double *prob, void *stream) {
     cudaStream_t st = pick(stream);
     if (!st) return HGM_ERR_CUDA;
     std::lock_guard<std::mutex> lk(g_reduce_mu);
-    const int rc = queue_marginal(s, mask, g_ctx.partials, g_ctx.partial_idx, g_ctx.host_result, st);
+    const int rc = queue_marginal(s, mask, g_ctx.partials, g_ctx.partial_idx, g_ctx.marginal, MARG_SUMS, g_ctx.host_result, st);
     if (rc) return rc;
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(HGM_ERR_CUDA, "marginal argmax: %s", cudaGetErrorString(e));

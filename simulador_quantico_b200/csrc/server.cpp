@@ -93,6 +93,7 @@ struct Slot {
     bool tail = false;   // reductions and result copy queued (s.done recorded)
     double *partials = nullptr;
     long long *ibest = nullptr;
+    double *sums = nullptr;   // MARG_SUMS doubles, from the first argmax that can use them on
     double *dres = nullptr;   // 4 doubles: norm (2 slots), argmax probability and index
     double *hres = nullptr;   // pinned, 6 doubles: dres, then a chained run's error word
     Request *req = nullptr;
@@ -248,6 +249,7 @@ struct Server {
             }
             if (s.partials) cudaFree(s.partials);
             if (s.ibest) cudaFree(s.ibest);
+            if (s.sums) cudaFree(s.sums);
             if (s.dres) cudaFree(s.dres);
             if (s.hres) cudaFreeHost(s.hres);
             if (s.done) cudaEventDestroy(s.done);
@@ -351,8 +353,16 @@ struct Server {
             }
             if (s.cursor.next >= s.total) {
                 int rc = launch_norm_async(&r->state, s.partials, s.dres, s.stream);
-                if (!rc && r->result_mask)
-                    rc = launch_argmax_async(&r->state, r->result_mask, s.partials, s.ibest, s.dres + 2, s.stream);
+                if (!rc && r->result_mask) {
+                    // pbest in the first half of partials; its second half serves where the sums are
+                    // few or there is no memory for more
+                    const bool more = s.sums || (marginal_sums(r->n, r->result_mask) > REDUCE_SCRATCH_BLOCKS &&
+                                                 cudaMalloc(&s.sums, MARG_SUMS * sizeof(double)) == cudaSuccess);
+                    if (!more) cudaGetLastError();
+                    rc = launch_argmax_async(&r->state, r->result_mask, s.partials, s.ibest,
+                                             more ? s.sums : s.partials + REDUCE_SCRATCH_BLOCKS,
+                                             more ? MARG_SUMS : REDUCE_SCRATCH_BLOCKS, s.dres + 2, s.stream);
+                }
                 if (rc) return rc;
                 cudaMemcpyAsync(s.hres, s.dres, 4 * sizeof(double), cudaMemcpyDeviceToHost, s.stream);
                 cudaError_t e = cudaEventRecord(s.done, s.stream);
