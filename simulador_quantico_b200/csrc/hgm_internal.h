@@ -251,7 +251,7 @@ enum StreamKind : uint32_t {
                   // the old and the new layout; then old steps 0..3, new steps 0..3, and the
                   // new layout's byte steps of thread bits 0..3 and 4..7
     S_ROT = 3,    // FP64: rotations with a phase, on the register bits of w1 (bits 0..7), then X on
-                  // those of w1 bits 8..15; (t, u, p re, p im) per bit (lower.cpp make_rot)
+                  // those of w1 bits 8..15; (t, u, p re, p im) per bit (lower.cpp make_rot, make_lift)
     S_HAD = 4,    // FP64: sqrt(2) H on the register bits of w1
     S_REAL = 5,   // real 2x2s on the register bits of w1: m00, m01, m10, m11 per bit
     S_DENSE = 6,  // complex 2x2s on the register bits of w1: 8 values per bit
@@ -264,8 +264,8 @@ enum StreamKind : uint32_t {
     S_TERMS = 11,   // phase block of product terms, same head
     S_GATE = 12,    // any other record; w1: kind | tpos << 8, w2, w3: cm_reg, cv_reg; then thread
                     // controls, non-tile controls and (not for K_SWAP) the matrix
-    S_SPLIT = 13,   // FP32: a phase, then a real 2x2, on the register bits of w1; m00, m01, m10,
-                    // m11, p re, p im, 0, 0 per bit (K_LAYER_SPLIT)
+    S_SPLIT = 13,   // a phase, then a real 2x2, on the register bits of w1; m00, m01, m10, m11, p re,
+                    // p im, 0, 0 per bit (K_LAYER_SPLIT; in FP64 only gates without S_ROT's form)
 };
 constexpr uint32_t STREAM_SYNC_BEFORE = 1, STREAM_SYNC_CROSS = 2;
 

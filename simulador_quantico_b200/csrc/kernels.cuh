@@ -566,17 +566,17 @@ __device__ __forceinline__ void reg_half_phase(A2 (&a)[1 << R], A2 f) {
 //     phase, against the complex matrix's 8.
 //   FP64 (S_ROT, lower.cpp make_rot): a rotation in place, its factor left
 //     out; 4 + 4 operations a pair against 16 of a complex 2x2 and 12 of the
-//     phase and a real 2x2.
+//     phase and a real 2x2 (S_SPLIT in FP64: gates without that form).
 // Seen through a swapped label (xr bit T set) the gate is
 //   X Rm diag(1, p) X = p (X Rm X) diag(1, p*),
 // so the phase stays on the same registers, conjugated, the real matrix is
 // read bit-swapped (a rotation by the opposite angle) and p joins the thread's
 // factor `pend`, which the layer multiplies into all registers at its end.
-// One gate's data as loaded: FP32 m00, m01, m10, m11, p; FP64 t, u, p.
-template <typename Real>
+// One gate's data as loaded: m00, m01, m10, m11, p; S_ROT t, u, p.
+template <typename Real, bool ROT>
 struct SplitRec;
 template <>
-struct SplitRec<float> {
+struct SplitRec<float, false> {
     float4 m;
     float2 p;
     __device__ __forceinline__ void load(const float *__restrict__ d) {
@@ -586,7 +586,18 @@ struct SplitRec<float> {
     static constexpr int words = 8;
 };
 template <>
-struct SplitRec<double> {
+struct SplitRec<double, false> {
+    double4 m;
+    double2 p;
+    __device__ __forceinline__ void load(const double *__restrict__ d) {
+        const double2 a = reinterpret_cast<const double2 *>(d)[0], b = reinterpret_cast<const double2 *>(d)[1];
+        m = make_double4(a.x, a.y, b.x, b.y);
+        p = reinterpret_cast<const double2 *>(d)[2];
+    }
+    static constexpr int words = 8;
+};
+template <>
+struct SplitRec<double, true> {
     double2 tu, p;
     __device__ __forceinline__ void load(const double *__restrict__ d) {
         tu = reinterpret_cast<const double2 *>(d)[0];
@@ -595,27 +606,31 @@ struct SplitRec<double> {
     static constexpr int words = 4;
 };
 
-template <typename Real, typename A2, int R, int T>
+template <typename Real, typename A2, int R, int T, bool ROT>
 struct SplitStep {
     __device__ __forceinline__ static void run(A2 (&a)[1 << R], const Real *__restrict__ d, uint32_t mask, uint32_t xr,
-                                               A2 &pend, SplitRec<Real> &cur) {
+                                               A2 &pend, SplitRec<Real, ROT> &cur) {
         if (mask & (1u << T)) {
             const bool flip = (xr >> T) & 1u;
-            SplitRec<Real> c = cur;
+            SplitRec<Real, ROT> c = cur;
             if constexpr (sizeof(Real) == 8) c.load(d);
-            d += SplitRec<Real>::words;
+            d += SplitRec<Real, ROT>::words;
             // FP32: the next gate's data, while this one's arithmetic runs
             // (after the last gate: the units behind the op, not used), 1.2%
             // of a layered pass; in FP64 the eight registers cost 1%
             if constexpr (sizeof(Real) == 4) cur.load(d);
             A2 p = c.p;
-            if constexpr (sizeof(Real) == 4) {
-                // one rounding order whatever the compiler makes of the
-                // surrounding code
-                const Real px = __fmaf_rn(pend.x, p.x, -__fmul_rn(pend.y, p.y));
-                const Real py = __fmaf_rn(pend.x, p.y, __fmul_rn(pend.y, p.x));
-                pend.x = flip ? px : pend.x;
-                pend.y = flip ? py : pend.y;
+            if constexpr (!ROT) {
+                if constexpr (sizeof(Real) == 4) {
+                    // one rounding order whatever the compiler makes of the
+                    // surrounding code
+                    const Real px = __fmaf_rn(pend.x, p.x, -__fmul_rn(pend.y, p.y));
+                    const Real py = __fmaf_rn(pend.x, p.y, __fmul_rn(pend.y, p.x));
+                    pend.x = flip ? px : pend.x;
+                    pend.y = flip ? py : pend.y;
+                } else if (flip) {
+                    pend = cmul2<Real>(pend, p);
+                }
                 p.y = flip ? -p.y : p.y;
                 Real m[8];
                 m[0] = flip ? c.m.w : c.m.x;
@@ -643,24 +658,24 @@ struct SplitStep {
                     if (!(r & (1 << T))) ip_rot(a[r].x, a[r].y, a[r | (1 << T)].x, a[r | (1 << T)].y, u, t);
             }
         }
-        SplitStep<Real, A2, R, T + 1>::run(a, d, mask, xr, pend, cur);
+        SplitStep<Real, A2, R, T + 1, ROT>::run(a, d, mask, xr, pend, cur);
     }
 };
-template <typename Real, typename A2, int R>
-struct SplitStep<Real, A2, R, R> {
+template <typename Real, typename A2, int R, bool ROT>
+struct SplitStep<Real, A2, R, R, ROT> {
     __device__ __forceinline__ static void run(A2 (&)[1 << R], const Real *__restrict__, uint32_t, uint32_t, A2 &,
-                                               SplitRec<Real> &) {}
+                                               SplitRec<Real, ROT> &) {}
 };
 
-template <typename Real, typename A2, int R>
+template <typename Real, typename A2, int R, bool ROT>
 __device__ __forceinline__ void apply_split_layer(A2 (&a)[1 << R], const Real *__restrict__ d, uint32_t mask,
                                                   uint32_t xr) {
     A2 pend;
     pend.x = 1;
     pend.y = 0;
-    SplitRec<Real> cur;
+    SplitRec<Real, ROT> cur;
     if constexpr (sizeof(Real) == 4) cur.load(d);
-    SplitStep<Real, A2, R, 0>::run(a, d, mask, xr, pend, cur);
+    SplitStep<Real, A2, R, 0, ROT>::run(a, d, mask, xr, pend, cur);
     // every thread of the warp reaches this point (ops are uniform)
     if (__any_sync(0xffffffffu, (xr & mask) != 0u)) {
 #pragma unroll
@@ -1291,7 +1306,7 @@ __device__ __forceinline__ void store_tile(const typename V2<Real>::T (&a)[1 << 
 //
 // LEAN (Plan::lean): the build for plans whose phase blocks are all compact
 // terms, with no controlled dense, real or anti-diagonal gate on a register
-// bit and no complex layer.  Leaving those bodies out of the kernel
+// bit, no complex layer and, in FP64, no S_SPLIT.  Leaving those bodies out of the kernel
 // -- code the benchmark circuits never run -- made 26-qubit FP32 layered
 // passes 5% and QFT passes 9% faster (fewer instruction-fetch stalls), so
 // each plan runs the smallest build it can.
@@ -1343,7 +1358,7 @@ __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], t
         nh = *reinterpret_cast<const uint4 *>(win + pc);
         if (kind == (F64 ? S_ROT : S_SPLIT)) {
             const uint32_t mask = hdr.y & 0xffu;
-            apply_split_layer<Real, A2, R>(a, data, mask, xr);
+            apply_split_layer<Real, A2, R, F64>(a, data, mask, xr);
             if (F64) xr ^= hdr.y >> 8;
         } else if (kind == S_REAL || (F64 && kind == S_HAD)) {
             const bool had = F64 && kind == S_HAD;
@@ -1387,6 +1402,8 @@ __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], t
             next += hdr.y;
             pc = first ? STREAM_WINDOW_BYTES : 0;
             nh = *reinterpret_cast<const uint4 *>(win + pc);
+        } else if (F64 && !LEAN && kind == S_SPLIT) {
+            apply_split_layer<Real, A2, R, false>(a, data, hdr.y, xr);
         } else if (!LEAN && kind == S_DENSE) {
             DenseStep<Real, A2, R, 0>::run(a, data, hdr.y, xr);
         } else if (!LEAN && kind == S_TERMS) {

@@ -60,6 +60,26 @@ bool make_rot(const double *m, double p_re, double p_im, Rot &r) {
     return true;
 }
 
+// Any other invertible real matrix in the same form: rows exchanged if the
+// first column's larger entry a is below, then with t = c / a, s = det / a^2
+// and u = (b / a) / s,
+//   M = a X^x [[1, s u], [t, s (1 + t u)]] diag(1, p),
+// run as above with s in the phase's place of e (1 + t^2).  |t| <= 1 bounds the
+// growth as row pivoting does.  Not a form that survives a relabeled bit: only
+// for bits that no thread has relabeled.  False for (nearly) singular matrices.
+bool make_lift(const double *m, double p_re, double p_im, Rot &r) {
+    r.x = std::abs(m[2]) > std::abs(m[0]);
+    const long double a = m[r.x ? 2 : 0], b = m[r.x ? 3 : 1], c = m[r.x ? 0 : 2], d = m[r.x ? 1 : 3];
+    const long double s = (a * d - b * c) / (a * a);
+    r.kappa = (double)a;
+    r.t = (double)(c / a);
+    r.u = (double)(b / a / s);
+    r.pr = (double)(s * p_re);
+    r.pi = (double)(s * p_im);
+    return std::isfinite(r.t) && std::isfinite(r.u) && std::isfinite(r.pr) && std::isfinite(r.pi) &&
+           std::abs(r.u) <= 0x1p20;
+}
+
 // The factor a of a [[1, 1], [1, -1]], or 0.
 double hadamard_factor(const double *m) {
     const double a = 0.25 * (m[0] + m[1] + m[2] - m[3]), tol = 4e-16 * std::abs(a);
@@ -80,6 +100,8 @@ struct Lowering {
     std::vector<size_t> windows;   // units of each finished window
     static constexpr size_t CAP = STREAM_WINDOW_UNITS - 1;  // one unit for S_NEXT or S_END
 
+    int split_gates = 0, phase_gates = 0;  // gates of split layers; of them, phase gates with a real one behind
+    uint32_t relabeled = 0;  // register bits that some thread may have relabeled in this layout
     bool fresh = true;       // no phase block of compact terms in this layout yet
     bool drop_swaps = false; // the marked records are left to a permutation pass
 
@@ -169,6 +191,7 @@ struct Lowering {
         for (int b = 0; b < 8; b++) op.push_back(thread_step(t, b));
         add(S_TRANS, op);
         fresh = true;
+        relabeled = 0;
     }
 
     void gate(const DevOp<Real> &d) {
@@ -183,6 +206,7 @@ struct Lowering {
         if (d.kind != K_SWAP)
             for (int k = 0; k < 8; k++) put_real(op, d.m[k]);
         add(S_GATE, op);
+        if (d.kind == K_SWAP && d.tpos < R && !d.cm_reg) relabeled |= 1u << d.tpos;
     }
 
     // A layer of real or split gates: mats[k] is the record of the k-th bit of the mask.
@@ -200,53 +224,68 @@ struct Lowering {
             add(split ? S_SPLIT : S_REAL, op);
             return;
         }
+        // Each gate of a split layer in place where it has that form.  Where
+        // one has not, it takes the phase and the real 2x2 (S_SPLIT, or a phase
+        // gate and the real form on the lean build, run()), and the real gates of
+        // the layer the real form.
         std::vector<int> bit;
         for (int b = 0; b < R; b++)
             if ((mask >> b) & 1u) bit.push_back(b);
-        std::vector<uint32_t> rot = {0u, mask, 0u, 0u}, had = {0u, 0u, 0u, 0u}, real = {0u, 0u, 0u, 0u};
-        double factor = 1.0;
-        bool all_rot = split;
-        for (int i = 0; i < n && all_rot; i++) {
+        std::vector<Rot> form(n);
+        uint32_t in_place = 0, turned = 0;  // gates with that form; with a phase
+        for (int i = 0; i < n && split; i++) {
             const Real *m = mats[i].m;
-            const double rm[4] = {(double)m[0], (double)m[1], (double)m[2], (double)m[3]};
-            Rot r;
-            all_rot = make_rot(rm, (double)m[4], (double)m[5], r);
-            if (!all_rot) break;
-            if (r.x) rot[1] |= 1u << (8 + bit[i]);
-            for (double v : {r.t, r.u, r.pr, r.pi}) put_real(rot, (Real)v);
-            factor *= r.kappa;
+            const double rm[4] = {(double)m[0], (double)m[1], (double)m[2], (double)m[3]}, pr = m[4], pi = m[5];
+            if (make_rot(rm, pr, pi, form[i]) || (!((relabeled >> bit[i]) & 1u) && make_lift(rm, pr, pi, form[i])))
+                in_place |= 1u << bit[i];
+            if (pr != 1.0 || pi != 0.0) turned |= 1u << bit[i];
         }
-        if (all_rot) {
-            add(S_ROT, rot);
-            left_out(factor);
-            return;
-        }
-        factor = 1.0;
+        if (in_place != mask) in_place &= turned;
+        std::vector<uint32_t> rot = {0u, 0u, 0u, 0u}, had = rot, real = rot, general = rot;
+        double left = 1.0, left_had = 1.0;
         for (int i = 0; i < n; i++) {
             const Real *m = mats[i].m;
+            const uint32_t b = 1u << bit[i];
             const double rm[4] = {(double)m[0], (double)m[split ? 1 : 2], (double)m[split ? 2 : 4], (double)m[split ? 3 : 6]};
-            if (split && (m[4] != (Real)1 || m[5] != (Real)0)) {  // the phase, then the real matrix
-                DevOp<Real> d;
-                memset(&d, 0, sizeof d);
-                d.kind = K_PHASE;
-                d.tpos = bit[i];
-                d.m[0] = (Real)1;
-                d.m[6] = m[4];
-                d.m[7] = m[5];
-                gate(d);
-            }
-            const double a = hadamard_factor(rm);
-            if (a != 0.0) {
-                had[1] |= 1u << bit[i];
-                factor *= a;
+            if (in_place & b) {
+                const Rot &r = form[i];
+                rot[1] |= b | (r.x ? b << 8 : 0u);
+                for (double v : {r.t, r.u, r.pr, r.pi}) put_real(rot, (Real)v);
+                left *= r.kappa;
+            } else if ((turned & b) && !plan->lean) {
+                general[1] |= b;
+                for (double v : {rm[0], rm[1], rm[2], rm[3], (double)m[4], (double)m[5], 0.0, 0.0}) put_real(general, (Real)v);
             } else {
-                real[1] |= 1u << bit[i];
-                for (double v : rm) put_real(real, (Real)v);
+                if (turned & b) {
+                    DevOp<Real> d;
+                    memset(&d, 0, sizeof d);
+                    d.kind = K_PHASE;
+                    d.tpos = bit[i];
+                    d.m[0] = (Real)1;
+                    d.m[6] = m[4];
+                    d.m[7] = m[5];
+                    gate(d);
+                    phase_gates++;
+                }
+                if (const double a = hadamard_factor(rm); a != 0.0) {
+                    had[1] |= b;
+                    left_had *= a;
+                } else {
+                    real[1] |= b;
+                    for (double v : rm) put_real(real, (Real)v);
+                }
             }
         }
+        if (split) split_gates += n;
+        if (rot[1]) {
+            add(S_ROT, rot);
+            relabeled |= rot[1] >> 8;
+            left_out(left);
+        }
+        if (general[1]) add(S_SPLIT, general);
         if (had[1]) {
             add(S_HAD, had);
-            left_out(factor);
+            left_out(left_had);
         }
         if (real[1]) add(S_REAL, real);
     }
@@ -340,6 +379,7 @@ struct Lowering {
         window.clear();
         windows.clear();
         fresh = true;
+        relabeled = 0;
         int cur = pa.load_layout;
         bool prev_cross = false;
         auto go_to = [&](int layout) {
@@ -377,6 +417,7 @@ struct Lowering {
                         memcpy(&w, reinterpret_cast<const unsigned char *>(d.m) + 4 * k, 4);
                         op.push_back(w);
                         op[1]++;
+                        relabeled |= 1u << (w & 0xffu);
                     }
                     add(S_XSET, op);
                     i++;
@@ -491,7 +532,22 @@ struct Lowering {
         while (first > 0 && only_swaps(plan->passes[first - 1], ops)) first--;
         drop_swaps = first < passes && first > 0 && global == 1.0 && !swaps.empty() && permutation(swaps, perm);
         if (drop_swaps) passes = first;
-        for (size_t p = 0; p < passes; p++) pass(plan->passes[p], ops, n_ops, p + 1 == passes);
+        const auto all = [&] {
+            for (size_t p = 0; p < passes; p++) pass(plan->passes[p], ops, n_ops, p + 1 == passes);
+        };
+        all();
+        // The lean build has no S_SPLIT in FP64: the branch alone cost layered
+        // circuits 0.4%, while a phase gate costs a fifth of a gate of a
+        // layer, and the full build a twentieth of the whole.  26 qubits, six
+        // layers of gates with phases: a quarter of them not unitary 7.2 ms, all
+        // 7.5 (8.8 and 9.8 where one such gate put its layer in the real form).
+        if (plan->lean && 4 * phase_gates > split_gates) {
+            plan->lean = false;
+            plan->stream.clear();
+            plan->tiles.clear();
+            scale = 1.0;
+            all();
+        }
         if (drop_swaps) plan->tiles.push_back(perm);
     }
 };

@@ -1,0 +1,82 @@
+"""FP64 layers of unitary, other invertible and singular gates with phases: each gate takes the cheapest form it has
+(csrc/lower.cpp layer)."""
+import numpy as np
+import pytest
+
+import simulador_quantico_b200 as sq
+from tests import plan_emulator as emu
+from tests.helpers import random_state
+from tests.test_lowering import S_GATE, S_REAL, S_ROT, S_SPLIT, both, stream_units
+
+
+def gate(kind, rng):
+    a, b = rng.uniform(0.2, 1.3), rng.uniform(0.0, 6.0)
+    r = np.array([[np.cos(a), -np.sin(a)], [np.sin(a), np.cos(a)]])
+    if kind == "invertible":
+        r = r @ np.array([[1.0, 0.3], [0.2, -0.7 if b > 3 else 0.9]])
+    elif kind == "steep":  # determinant 1e-5 of its entries' squares
+        r = r @ np.array([[1.0, 1.0], [1.0, 1.0 + 1e-5]]) / 2
+    elif kind == "singular":
+        r = r @ np.array([[0.8, 0.4], [0.6, 0.3]])
+    return (r @ np.diag([1.0, np.exp(1j * b)])).reshape(-1)
+
+
+def circuit(n, layers, kinds, swaps, seed):
+    rng, c = np.random.default_rng(seed), sq.Circuit()
+    for k in range(layers):
+        for q in range(n):
+            c.append_op(q, 0, 0, gate(kinds[(q + k) % len(kinds)], rng))
+        for q in range(k % 2 if swaps else n, n - 1, 2):  # relabelings and controlled swaps between layers
+            c.append_op(q, 2 << q, (2 << q) * (q % 2), [0, 1, 1, 0])
+    return c
+
+
+def ops_of(plan):
+    units, at, out = stream_units(plan)[0], 0, []
+    while at < len(units):
+        w = [int(x) for x in units[at]]
+        out.append((w[0] & 0xFF, w))
+        at += w[0] >> 8
+    return out
+
+
+MIXES = {"unitary": ["unitary"], "quarter": ["unitary"] * 3 + ["invertible"], "invertible": ["invertible"],
+         "singular": ["unitary", "singular", "invertible"], "steep": ["steep", "unitary"],
+         "few": ["singular"] + ["unitary"] * 7}
+
+
+@pytest.mark.parametrize("name", MIXES)
+def test_each_gate_for_itself(name):
+    n = 13
+    ops = ops_of(sq.Plan(circuit(n, 1, MIXES[name], False, 5), n, "f64", fuse=0))
+    bits = lambda kind: sum(bin(w[1] & 0xFF).count("1") for k, w in ops if k == kind)
+    kinds = [MIXES[name][q % len(MIXES[name])] for q in range(n)]
+    singular = kinds.count("singular")
+    general = singular if 4 * singular > n else 0  # few: a phase gate and a real 2x2 each
+    assert bits(S_ROT) == n - singular and bits(S_SPLIT) == general
+    assert bits(S_REAL) == singular - general == sum(1 for k, _ in ops if k == S_GATE)
+
+
+@pytest.mark.parametrize("swaps", [False, True])
+@pytest.mark.parametrize("name", MIXES)
+def test_mixed_layers(monkeypatch, name, swaps):
+    n = 13
+    got, want = both(monkeypatch, sq.Plan(circuit(n, 4, MIXES[name], swaps, 7), n, "f64"), "f64", n, seed=n)
+    # 52 gates in a row, each a few roundings of 2^-53 of its operands; a steep gate's of terms up to 2^10 of its result
+    assert np.abs(got - want).max() <= 1e-12 * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("swaps", [False, True])
+@pytest.mark.parametrize("n", [9, 12, 15])
+@pytest.mark.parametrize("name", MIXES)
+def test_mixed_layers_on_the_device(name, n, swaps):
+    sq.init()
+    plan = sq.Plan(circuit(n, 4, MIXES[name], swaps, n), n, "f64")
+    v = random_state(n, seed=n)
+    want = emu.run(plan, "f64", v)
+    st = sq.State(n, "f64").upload(v)
+    got = st.execute(plan).download()
+    plan.status()
+    st.free()
+    assert np.abs(got - want).max() <= 1e-12 * max(1.0, np.abs(want).max())
