@@ -66,7 +66,9 @@ bool make_rot(const double *m, double p_re, double p_im, Rot &r) {
 //   M = a X^x [[1, s u], [t, s (1 + t u)]] diag(1, p),
 // run as above with s in the phase's place of e (1 + t^2).  |t| <= 1 bounds the
 // growth as row pivoting does.  Not a form that survives a relabeled bit: only
-// for bits that no thread has relabeled.  False for (nearly) singular matrices.
+// for bits that no thread has relabeled.  False for (nearly) singular matrices
+// and for those whose second column is far larger than the first: s and s u, by
+// which amplitudes grow before a is applied, stay below 2^20.
 bool make_lift(const double *m, double p_re, double p_im, Rot &r) {
     r.x = std::abs(m[2]) > std::abs(m[0]);
     const long double a = m[r.x ? 2 : 0], b = m[r.x ? 3 : 1], c = m[r.x ? 0 : 2], d = m[r.x ? 1 : 3];
@@ -77,7 +79,7 @@ bool make_lift(const double *m, double p_re, double p_im, Rot &r) {
     r.pr = (double)(s * p_re);
     r.pi = (double)(s * p_im);
     return std::isfinite(r.t) && std::isfinite(r.u) && std::isfinite(r.pr) && std::isfinite(r.pi) &&
-           std::abs(r.u) <= 0x1p20;
+           std::abs(r.u) <= 0x1p20 && std::abs(s) <= 0x1p20 && std::abs(b / a) <= 0x1p20;
 }
 
 // The factor a of a [[1, 1], [1, -1]], or 0.

@@ -16,9 +16,11 @@ def gate(kind, rng):
         r = r @ np.array([[1.0, 0.3], [0.2, -0.7 if b > 3 else 0.9]])
     elif kind == "steep":  # determinant 1e-5 of its entries' squares
         r = r @ np.array([[1.0, 1.0], [1.0, 1.0 + 1e-5]]) / 2
+    elif kind == "narrow":  # a first column of 1e-160: in the in-place form two such gates would leave the range
+        r = np.array([[1e-160, 1.0], [2e-161, 3.0]])
     elif kind == "singular":
         r = r @ np.array([[0.8, 0.4], [0.6, 0.3]])
-    return (r @ np.diag([1.0, np.exp(1j * b)])).reshape(-1)
+    return (r * np.array([1.0, np.exp(1j * b)])).reshape(-1)
 
 
 def circuit(n, layers, kinds, swaps, seed):
@@ -42,7 +44,7 @@ def ops_of(plan):
 
 MIXES = {"unitary": ["unitary"], "quarter": ["unitary"] * 3 + ["invertible"], "invertible": ["invertible"],
          "singular": ["unitary", "singular", "invertible"], "steep": ["steep", "unitary"],
-         "few": ["singular"] + ["unitary"] * 7}
+         "narrow": ["unitary", "narrow"], "few": ["singular"] + ["unitary"] * 7}
 
 
 @pytest.mark.parametrize("name", MIXES)
@@ -51,7 +53,7 @@ def test_each_gate_for_itself(name):
     ops = ops_of(sq.Plan(circuit(n, 1, MIXES[name], False, 5), n, "f64", fuse=0))
     bits = lambda kind: sum(bin(w[1] & 0xFF).count("1") for k, w in ops if k == kind)
     kinds = [MIXES[name][q % len(MIXES[name])] for q in range(n)]
-    singular = kinds.count("singular")
+    singular = kinds.count("singular") + kinds.count("narrow")
     general = singular if 4 * singular > n else 0  # few: a phase gate and a real 2x2 each
     assert bits(S_ROT) == n - singular and bits(S_SPLIT) == general
     assert bits(S_REAL) == singular - general == sum(1 for k, _ in ops if k == S_GATE)
