@@ -26,7 +26,7 @@ namespace hgm {
 namespace {
 
 struct Rot {
-    double kappa;   // factor left out
+    long double kappa;  // factor left out: a plan multiplies hundreds of them
     double t, u, pr, pi;
     bool x;         // an X follows
 };
@@ -51,12 +51,12 @@ bool make_rot(const double *m, double p_re, double p_im, Rot &r) {
     r.x = std::abs(s) > std::abs(c);
     const double num = r.x ? c : s, den = r.x ? s : c, e = r.x ? -d : d;
     r.t = num / den;
-    const double sq = 1.0 + r.t * r.t;
+    const long double sq = 1.0L + (long double)r.t * r.t;
     // from the rounded t, so that kappa sqrt(1 + t^2) is Rm's own factor
-    r.kappa = std::copysign(std::hypot(c, s) / std::sqrt(sq), den);
-    r.u = -r.t / sq;
-    r.pr = e * p_re * sq;
-    r.pi = e * p_im * sq;
+    r.kappa = std::copysign(std::hypot((long double)c, (long double)s) / std::sqrt(sq), (long double)den);
+    r.u = (double)(-r.t / sq);
+    r.pr = (double)(e * p_re * sq);
+    r.pi = (double)(e * p_im * sq);
     return true;
 }
 
@@ -73,7 +73,7 @@ bool make_lift(const double *m, double p_re, double p_im, Rot &r) {
     r.x = std::abs(m[2]) > std::abs(m[0]);
     const long double a = m[r.x ? 2 : 0], b = m[r.x ? 3 : 1], c = m[r.x ? 0 : 2], d = m[r.x ? 1 : 3];
     const long double s = (a * d - b * c) / (a * a);
-    r.kappa = (double)a;
+    r.kappa = a;
     r.t = (double)(c / a);
     r.u = (double)(b / a / s);
     r.pr = (double)(s * p_re);
@@ -82,12 +82,16 @@ bool make_lift(const double *m, double p_re, double p_im, Rot &r) {
            std::abs(r.u) <= 0x1p20 && std::abs(s) <= 0x1p20 && std::abs(b / a) <= 0x1p20;
 }
 
-// The factor a of a [[1, 1], [1, -1]], or 0.
-double hadamard_factor(const double *m) {
+// The factor a of a [[1, 1], [1, -1]], or 0.  An a within the roundings of H, or
+// of a few H fused, of 1/sqrt 2 stands for that: a search multiplies thousands
+// of them, and the double's error alone, 5e-17 each, made most of the 1.4e-13 of
+// 26 qubits x 32 iterations (now 4e-16).
+long double hadamard_factor(const double *m) {
     const double a = 0.25 * (m[0] + m[1] + m[2] - m[3]), tol = 4e-16 * std::abs(a);
     const bool ok = std::isfinite(a) && std::abs(m[0] - a) <= tol && std::abs(m[1] - a) <= tol &&
                     std::abs(m[2] - a) <= tol && std::abs(m[3] + a) <= tol;
-    return ok ? a : 0.0;
+    const long double h = std::copysign(std::sqrt(0.5L), (long double)a);
+    return !ok ? 0.0L : std::abs(a - h) <= 0x1p-51L ? h : a;
 }
 
 template <typename Real>
@@ -95,7 +99,7 @@ struct Lowering {
     Plan *plan;
     const cplx global;
     const int R, W;
-    double scale = 1.0;      // factors left out and not yet applied
+    long double scale = 1.0;  // factors left out and not yet applied
     // the current pass: its windows' units
     std::vector<uint32_t> out;
     std::vector<uint32_t> window;
@@ -173,10 +177,10 @@ struct Lowering {
         add(S_SCALE, op);
         scale = 1.0;
     }
-    void left_out(double kappa) {
+    void left_out(long double kappa) {
         scale *= kappa;
-        const double a = std::abs(scale);
-        if (!(a < 0x1p200 && a > 0x1p-200)) add_scale();
+        const long double a = std::abs(scale);
+        if (!(a < 0x1p200L && a > 0x1p-200L)) add_scale();
     }
 
     // byte offset in the transpose buffer of local index j (kernels.cuh)
@@ -244,7 +248,7 @@ struct Lowering {
         }
         if (in_place != mask) in_place &= turned;
         std::vector<uint32_t> rot = {0u, 0u, 0u, 0u}, had = rot, real = rot, general = rot;
-        double left = 1.0, left_had = 1.0;
+        long double left = 1.0, left_had = 1.0;
         for (int i = 0; i < n; i++) {
             const Real *m = mats[i].m;
             const uint32_t b = 1u << bit[i];
@@ -269,7 +273,7 @@ struct Lowering {
                     gate(d);
                     phase_gates++;
                 }
-                if (const double a = hadamard_factor(rm); a != 0.0) {
+                if (const long double a = hadamard_factor(rm); a != 0.0L) {
                     had[1] |= b;
                     left_had *= a;
                 } else {
@@ -426,9 +430,8 @@ struct Lowering {
                 } else if (last_pass && i + 1 == (int)n_ops && global != 1.0) {
                     // the plan's scalar takes the factors left out with it
                     DevOp<Real> e = d;
-                    const cplx z = global * scale;
-                    e.m[0] = e.m[6] = (Real)z.real();
-                    e.m[1] = e.m[7] = (Real)z.imag();
+                    e.m[0] = e.m[6] = (Real)(global.real() * scale);
+                    e.m[1] = e.m[7] = (Real)(global.imag() * scale);
                     scale = 1.0;
                     gate(e);
                     i++;
