@@ -121,7 +121,9 @@ int hgm_plan_create_from_ref_pts(void *const *pts, int pt_precision, int qubits,
  * requests submitted with hgm_server_submit_plan still use is freed when the
  * last of them is done. */
 void hgm_plan_free(hgm_plan *p);
-/* Plan statistics: ops after fusion, passes, phases, transposes. */
+/* Plan statistics: ops after fusion, passes, phases, transposes, as planned
+ * (hgm_plan_export).  The passes that run may be fewer, a circuit's final swaps
+ * being one permutation pass: hgm_plan_stream counts those. */
 int hgm_plan_stats(const hgm_plan *p, int64_t *n_ops, int64_t *n_passes, int64_t *n_phases, int64_t *n_transposes);
 /* Copies the plan's device records to the GPU now instead of at its first
  * execution or submission (so that a timed or latency-critical section does
@@ -289,7 +291,7 @@ typedef struct hgm_server_opts {
     int warp_bits;         /* tile size, -1 = default */
     int order;             /* HGM_ORDER_ARRIVAL: queued requests are admitted in
                               arrival order; HGM_ORDER_WORK_FIRST: the queued
-                              request with the most work (state bytes x passes)
+                              request with the most work (state bytes x passes run)
                               that fits the budget goes first */
 } hgm_server_opts;
 #define HGM_ORDER_ARRIVAL 0

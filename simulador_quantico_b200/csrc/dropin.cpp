@@ -196,8 +196,10 @@ hgm_dropin_amp *GpuExecutionWrapper(hgm_dropin_amp *read_memory, hgm_ref_pt **pt
     if (hgm_plan_status(plan)) die("execution");  // a chained run that gave up a bounded wait
 
     if (debug) {
-        int64_t n_ops = 0, n_passes = 0;
+        int64_t n_ops = 0, n_passes = 0, n_run = 0;
         hgm_plan_stats(plan, &n_ops, &n_passes, nullptr, nullptr);
+        hgm_plan_stream(plan, nullptr, nullptr, nullptr, &n_run);
+        if (n_run) n_passes = n_run;  // as launched (a small state's plan has one launch and no passes)
         fprintf(stderr,
                 "[GPUEXEC]   qubits=%d elapsed_ms=%.3f plan_ms=%.3f h2d_ms=%.3f exec_ms=%.3f d2h_ms=%.3f ops=%lld "
                 "passes=%lld\n",

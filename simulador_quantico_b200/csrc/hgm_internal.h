@@ -436,6 +436,11 @@ struct PlanCursor {
 };
 int launch_plan_steps(State *s, const Plan *p, int iterations, PlanCursor *c, int64_t max_launches, void *stream);
 int64_t plan_launches(const Plan *p, int iterations);
+// Bytes one run of the plan reads and writes, over two: its states' order in a
+// server's queue by work.
+inline double plan_work(const Plan *p) {
+    return (double)(int64_t(1) << p->qubits) * (p->precision == HGM_F64 ? 16.0 : 8.0) * (double)plan_launches(p, 1);
+}
 // The whole pass sequence of `iterations` runs of the plan in one persistent
 // launch (kernels.cu chain_kernel); only for plans chain_eligible() accepts.
 bool chain_eligible(const Plan *p, int iterations);

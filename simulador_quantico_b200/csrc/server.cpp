@@ -489,8 +489,7 @@ struct Server {
                         double best = -1.0;
                         for (auto it = queue.begin(); it != queue.end(); ++it) {
                             if (bytes_in_use + (*it)->bytes > opts.budget_bytes) continue;
-                            const Plan *pl = (*it)->plan;
-                            const double w = (double)(*it)->bytes * (pl->small ? 1.0 : (double)pl->passes.size());
+                            const double w = plan_work((*it)->plan);
                             if (w > best) {
                                 best = w;
                                 pick = it;
