@@ -59,8 +59,12 @@ namespace {
 // whose own iterations keep the GPU busy meanwhile: as many as cover the
 // planning (plan_us; measured 0.35 us an op on the B200's host) at the least
 // time their passes can take are queued first, and what is left then runs on
-// it.  A call that cannot cover it, and the calls of fewer iterations, run the
-// plan itself.
+// it.  Where the planning is less than a fiftieth of that time for the whole
+// call, it comes first: the iterations queued ahead, and the remainder they
+// leave, would lose more merged passes than that (26-qubit FP64 search, first
+// call of 32 iterations: 53.5 ms behind queued ones, 52.3 planned first, 57.1 as
+// single runs).  A call that cannot cover it, and the calls of fewer
+// iterations, run the plan itself.
 //
 // Of the plan's runs and the longer plan the cheaper serves, by passes,
 // transposes and stream units (plan_cost).  Both timed on one B200, eight runs
@@ -79,11 +83,10 @@ int64_t state_bytes(const Plan *p) { return (int64_t(1) << p->qubits) * (p->prec
 // Planning and upload of the longer plan, in us.
 double plan_us(const Plan *p) { return 150.0 + 0.5 * UNROLL * (double)p->ops.size(); }
 
-// Iterations that keep the GPU busy for that long.
-int64_t iterations_ahead(const Plan *p) {
-    const double pass_us = 2.0 * (double)state_bytes(p) / PASS_BYTES_PER_US;
-    return (int64_t)std::ceil(plan_us(p) / (pass_us * (double)p->tiles.size()));
-}
+// The least time of one run of the plan, in us.
+double run_us(const Plan *p) { return 2.0 * (double)state_bytes(p) / PASS_BYTES_PER_US * (double)p->tiles.size(); }
+// Iterations that keep the GPU busy for the planning.
+int64_t iterations_ahead(const Plan *p) { return (int64_t)std::ceil(plan_us(p) / run_us(p)); }
 
 // A plan's time in passes over memory: what a pass saved gives back, a
 // transpose, and the ops' 16-byte units.
@@ -379,8 +382,8 @@ int hgm_execute(hgm_state *s, const hgm_plan *p, int iterations, void *stream) {
     };
     Plan *u = unrolled_plan(pl, iterations);
     if (!u && may_build(pl, iterations, (cudaStream_t)(stream ? stream : default_stream()))) {
-        const int ahead = (int)iterations_ahead(pl);
-        if ((rc = run(pl, ahead, iterations - ahead))) return rc;
+        const int ahead = 50.0 * plan_us(pl) <= iterations * run_us(pl) ? 0 : (int)iterations_ahead(pl);
+        if (ahead && (rc = run(pl, ahead, iterations - ahead))) return rc;
         build_unrolled(pl);
         u = unrolled_plan(pl, iterations);
     }

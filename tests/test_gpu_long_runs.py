@@ -124,6 +124,18 @@ def test_first_long_call_queues_its_own_iterations_first(sq):
     assert sq.kernel_launches() - l0 - first == 3 * 33
 
 
+def test_long_first_call_runs_on_the_longer_plan_at_once(sq):
+    """Planning is a hundredth of the call's 26 ms: no iteration is run ahead of it."""
+    n = 25
+    plan = sq.Plan(one_iteration(n, 5).build(sq.Circuit()), n, "f64").upload()
+    st = sq.State(n, "f64").set_basis(0)
+    for _ in range(2):
+        l0 = sq.kernel_launches()
+        st.execute(plan, 32)
+        assert sq.kernel_launches() - l0 == 4 * 33
+    st.free()
+
+
 def one_by_one(sq, circuit, n, prec, iterations):
     """Launches of `iterations` runs, twice; checks them against single runs."""
     plan = sq.Plan(circuit, n, prec).upload()
