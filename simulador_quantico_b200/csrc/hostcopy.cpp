@@ -17,13 +17,14 @@
 // chunks (8 MiB of page-locked memory), the calling thread taking a share
 // itself.  In us, up / down, plain and staged: 0.5 MiB 70 / 74 and 69 / 58 (188
 // once), 1 MiB 128 / 102 and 90 / 77, 16 MiB 1550 / 920 and 700 / 695, 128 MiB
-// 12100 / 7350 and 4200 / 4400: the line lies at 1 MiB, where the threads'
-// start is paid back in both directions.
+// 12100 / 7350 and 4200 / 4400.  The line lies at 1 MiB, where a call that copies
+// up, runs and copies down gains (1 MiB 346 -> 262 us, 2 MiB 524 -> 365, 8 MiB 1490
+// -> 830); of copies one after another in one direction those of 1 to 2 MiB lose
+// (up 78 -> 98 us, 135 -> 158).
 //
 // Each set of chunks (the large one is 256 MiB) is allocated on its first copy
 // and kept until exit; copies below kSmallMin use a plain cudaMemcpyAsync.
-// One staged copy of a set runs at a time; what else comes goes directly
-// (copy_state).
+// One staged copy of a set runs at a time (take_chunks).
 #include <cuda_runtime.h>
 
 #include <atomic>

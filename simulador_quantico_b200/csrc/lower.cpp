@@ -5,12 +5,14 @@
 //   * one linear stream per pass, ops and transposes in the order they run,
 //     16 to 32 bytes a gate instead of 80 to 112, so that a window of it fits
 //     beside the transpose buffer in shared memory;
-//   * FP64 rotations and Hadamards without their common factor (cos or
-//     1/sqrt 2), which leaves half the operations of the real 2x2 out; the
-//     factors multiply into one S_SCALE at the plan's end (or when they leave
-//     [2^-200, 2^200]).  28 qubits, 10 layers, FP64: 67.0 -> 50.1 ms with the
-//     stream; 26-qubit search, 32 iterations: 78.7 -> 60.2 ms.  FP32 keeps the plain form: its results stay, bit by
-//     bit, those of the records;
+//   * FP64 rotations, Hadamards and other invertible gates without their common
+//     factor (cos or 1/sqrt 2), which leaves half the operations of the real 2x2
+//     out; the factors multiply into one S_SCALE at the plan's end (or when they
+//     leave [2^-200, 2^200]; amplitudes above 2^823 would overflow meanwhile).
+//     28 qubits, 10 layers, FP64: 67.0 -> 50.1 ms with the stream; 26-qubit
+//     search, 32 iterations: 78.7 -> 60.2 ms.  FP32 keeps the plain form: its
+//     results are, bit by bit, those of the records, but for phase blocks larger
+//     than a window, which run as several;
 //   * the swaps that end a circuit (a QFT's qubit reversal), where they fill
 //     passes of their own, as one permutation pass: it reads and writes the
 //     state once at memory speed, whatever the pairs, where CNOTs need the
