@@ -356,6 +356,7 @@ struct Server {
                 if (!rc && r->result_mask) {
                     // pbest in the first half of partials; its second half serves where the sums are
                     // few or there is no memory for more
+                    OutsideCapture elsewhere;
                     const bool more = s.sums || (marginal_sums(r->n, r->result_mask) > REDUCE_SCRATCH_BLOCKS &&
                                                  cudaMalloc(&s.sums, MARG_SUMS * sizeof(double)) == cudaSuccess);
                     if (!more) cudaGetLastError();
