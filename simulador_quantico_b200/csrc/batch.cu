@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
         __syncthreads();
         if (!s_skip) {
             if (tiled) {
-                fetch_stream(win, s_ta);
+                fetch_stream<W>(win, s_ta);
                 run_tile<Real, R, W, LEAN, true>(reinterpret_cast<A2 *>(t.state), s_ta,
                                                  (uint64_t)(s_next - t.tile_begin), smem_raw, s_ctl);
             } else {

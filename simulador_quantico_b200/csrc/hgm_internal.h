@@ -236,14 +236,19 @@ constexpr int32_t PASS_PERMUTE = 4;  // a permutation pass (below), no stream
 // are lowered (lower.cpp) to one stream of 16-byte units: every op is a
 // header unit (word 0: kind in bits 0..7, units of the op in bits 8..) and
 // its data, transposes among them.  A pass's stream is cut into windows of at
-// most STREAM_WINDOW_UNITS, which a CTA copies into shared memory, one window
+// most STREAM_WINDOW_UNITS (SHORT_WINDOW_UNITS), which a CTA copies into shared memory, one window
 // ahead of the one it runs: an op read from global memory cost an L2 round
 // trip each in states of one or a few tiles, where no other warp hides it
 // (12 qubits, 20 layers, one tile: 199 -> 109 us), and in large states the
 // addresses and the waits of those loads (26 qubits, 20 layers, FP32: 16.4 ->
 // 13.3 ms, same arithmetic; the kernels' spills went with them).
 // Two windows of 176 units leave four CTAs an SM within the 164 KB carveout.
-constexpr int STREAM_WINDOW_UNITS = 176;
+// One-warp CTAs are many to an SM, and their windows take shared memory from the
+// L1 that holds their loads in flight: for a state of more than one tile theirs
+// are a third as long (26 qubits FP32, 300 gates of every kind: 14.6 -> 11.7 ms;
+// 6 layers 5.08 -> 4.55), while a state of one tile, alone on its SM, wants long ones
+// (10 qubits, 20 layers: 85 us, 87 with short ones).
+constexpr int STREAM_WINDOW_UNITS = 176, SHORT_WINDOW_UNITS = 64;
 enum StreamKind : uint32_t {
     S_END = 0,    // store the tile
     S_NEXT = 1,   // go on in the next window; w1: units of the window after it (0: none)
@@ -294,7 +299,8 @@ struct alignas(16) TileArgs {
     int8_t st_gbit[MAX_LAYOUT_ROLES];
     int8_t run_pos[TILE_RUNS];         // the non-tile index bits as runs (PassArgs)
     int8_t run_len[TILE_RUNS];
-    uint32_t ld_tstep[8];   // load layout: byte step of each thread bit in the transpose buffer
+    uint32_t ld_tstep[8];   // load layout: byte step of each thread bit in the transpose buffer;
+                            // one-warp plans: the last is a window's bytes
     const void *stream;     // first window, then the others back to back
     int32_t units0, units1; // units of the first two windows
     int32_t n, k;

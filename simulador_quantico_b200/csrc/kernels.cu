@@ -113,7 +113,7 @@ template <typename Real, int R, int W, bool LEAN>
 __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()))
     pass_kernel(typename V2<Real>::T *__restrict__ state, const __grid_constant__ TileArgs ta) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    fetch_stream(smem_raw + tile_smem_bytes<Real, R, W>(), ta);
+    fetch_stream<W>(smem_raw + tile_smem_bytes<Real, R, W>(), ta);
     wait_for_kernel_before();
     let_next_kernel_start();
     run_tile<Real, R, W, LEAN, false>(state, ta, blockIdx.x, smem_raw, ta.ctl);
@@ -189,7 +189,7 @@ static int launch_pass(void *state, const TileArgs &pa, cudaStream_t st) {
     int rc = setup_pass_kernel<Real, R, W, LEAN>();
     if (rc) return rc;
     const uint64_t tiles = 1ull << (pa.n - pa.k);
-    const int smem = cta_smem_bytes<Real, R, W>();
+    const int smem = cta_smem_bytes<Real, R, W>() - 2 * (STREAM_WINDOW_BYTES - (int)window_bytes<W>(pa));
     const cudaError_t e = launch_behind(pass_kernel<Real, R, W, LEAN>, (unsigned)tiles, 32 << W, smem, st,
                                         reinterpret_cast<A2 *>(state), pa);
     if (e != cudaSuccess) return fail(HGM_ERR_CUDA, "pass_kernel launch: %s", cudaGetErrorString(e));
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
     fetch_args(&s_ta[0], 0);
     fetch_wait();
     __syncthreads();
-    fetch_stream(win, s_ta[0]);
+    fetch_stream<W>(win, s_ta[0]);
     if (threadIdx.x == 0) {
         s_next = (long long)atomicAdd(&ctr[0], 1ull);
         s_at.g = s_next >> tile_bits;
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
             fetch_args(&s_ta[s_cur], s_at.pass);
             fetch_wait();
             __syncthreads();
-            fetch_stream(win, s_ta[s_cur]);
+            fetch_stream<W>(win, s_ta[s_cur]);
         }
         if (s_fetched) fetch_args(&s_ta[s_cur ^ 1], s_guess.pass);
         if (!s_skip)
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(32 << W) __maxnreg__((pass_max_regs<Real, R>()
         fetch_wait();  // the guessed pass's arguments
         __syncthreads();
         if (threadIdx.x == blockDim.x - 1) s_next = (long long)atomicAdd(&ctr[0], 1ull);
-        fetch_stream(win, s_ta[s_cur ^ s_fetched]);
+        fetch_stream<W>(win, s_ta[s_cur ^ s_fetched]);
         if (threadIdx.x == 0) {
             // the next pass accumulates a norm: zero its slot first
             if (renorm > 0 && (s_it & ((1ll << tile_bits) - 1)) == 0 && s_at.g + 2 < seq) {

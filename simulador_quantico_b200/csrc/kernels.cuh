@@ -1178,6 +1178,11 @@ __device__ __forceinline__ void apply_gate(A2 (&a)[1 << R], const unsigned char 
 // ---- the stream in shared memory ---------------------------------------------
 
 constexpr int STREAM_WINDOW_BYTES = STREAM_WINDOW_UNITS * 16;
+// Bytes of a pass's window (at most STREAM_WINDOW_BYTES).
+template <int W>
+__host__ __device__ __forceinline__ uint32_t window_bytes(const TileArgs &ta) {
+    return W == 0 ? ta.ld_tstep[7] : (uint32_t)STREAM_WINDOW_BYTES;
+}
 
 // Shared memory of a CTA: the transpose buffer, then two stream windows, then
 // room for the loads ahead of the last op (a header, a gate's data; not used).
@@ -1201,10 +1206,11 @@ __device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_all;"
 
 // Starts copying a pass's first two windows; every earlier reader of the
 // windows must be done.
+template <int W>
 __device__ __forceinline__ void fetch_stream(unsigned char *win, const TileArgs &ta) {
     const uint4 *src = reinterpret_cast<const uint4 *>(ta.stream);
     fetch_units(win, src, ta.units0);
-    if (ta.units1) fetch_units(win + STREAM_WINDOW_BYTES, src + ta.units0, ta.units1);
+    if (ta.units1) fetch_units(win + window_bytes<W>(ta), src + ta.units0, ta.units1);
 }
 
 // ---- layout transposes through shared memory --------------------------------
@@ -1417,12 +1423,13 @@ __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], t
             // window after it
             fetch_wait();
             __syncthreads();
-            const bool first = pc <= STREAM_WINDOW_BYTES;
+            const uint32_t wb = window_bytes<W>(ta);
+            const bool first = pc <= wb;
             if (hdr.y)
-                fetch_units(win + (first ? 0 : STREAM_WINDOW_BYTES), reinterpret_cast<const uint4 *>(ta.stream) + next,
+                fetch_units(win + (first ? 0 : wb), reinterpret_cast<const uint4 *>(ta.stream) + next,
                             (int)hdr.y);
             next += hdr.y;
-            pc = first ? STREAM_WINDOW_BYTES : 0;
+            pc = first ? wb : 0;
             nh = *reinterpret_cast<const uint4 *>(win + pc);
         } else if (F64 && !LEAN && kind == S_SPLIT) {
             apply_split_layer<Real, A2, R, false>(a, data, hdr.y, xr);

@@ -106,14 +106,16 @@ struct Lowering {
     std::vector<uint32_t> out;
     std::vector<uint32_t> window;
     std::vector<size_t> windows;   // units of each finished window
-    static constexpr size_t CAP = STREAM_WINDOW_UNITS - 1;  // one unit for S_NEXT or S_END
+    const size_t CAP;              // one unit less than a window: S_NEXT or S_END
 
     int split_gates = 0, phase_gates = 0;  // gates of split layers; of them, phase gates with a real one behind
     uint32_t relabeled = 0;  // register bits that some thread may have relabeled in this layout
     bool fresh = true;       // no phase block of compact terms in this layout yet
     bool drop_swaps = false; // the marked records are left to a permutation pass
 
-    Lowering(Plan *p, cplx gl) : plan(p), global(gl), R(p->reg_bits), W(p->warp_bits) {}
+    Lowering(Plan *p, cplx gl)
+        : plan(p), global(gl), R(p->reg_bits), W(p->warp_bits),
+          CAP((W == 0 && p->qubits > 5 + R ? SHORT_WINDOW_UNITS : STREAM_WINDOW_UNITS) - 1) {}
 
     bool same_warps(int a, int b) const {
         for (int w = 0; w < W; w++)
@@ -469,6 +471,7 @@ struct Lowering {
         for (int k = 0; k < 5 + W + R; k++) t.st_gbit[k] = pa.tb[plan->layouts[cur].pos[k]];
         t.pass = (int32_t)(&pa - plan->passes.data());
         for (int b = 0; b < 8; b++) t.ld_tstep[b] = thread_step(plan->layouts[pa.load_layout], b);
+        if (W == 0) t.ld_tstep[7] = (uint32_t)(CAP + 1) * 16u;
         plan->tiles.push_back(t);
     }
 
