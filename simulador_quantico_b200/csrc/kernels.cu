@@ -189,7 +189,7 @@ static int launch_pass(void *state, const TileArgs &pa, cudaStream_t st) {
     int rc = setup_pass_kernel<Real, R, W, LEAN>();
     if (rc) return rc;
     const uint64_t tiles = 1ull << (pa.n - pa.k);
-    const int smem = cta_smem_bytes<Real, R, W>() - 2 * (STREAM_WINDOW_BYTES - (int)window_bytes<W>(pa));
+    const int smem = cta_smem_bytes<Real, R, W>() - 2 * (STREAM_WINDOW_BYTES - window_bytes<W>(pa));
     const cudaError_t e = launch_behind(pass_kernel<Real, R, W, LEAN>, (unsigned)tiles, 32 << W, smem, st,
                                         reinterpret_cast<A2 *>(state), pa);
     if (e != cudaSuccess) return fail(HGM_ERR_CUDA, "pass_kernel launch: %s", cudaGetErrorString(e));

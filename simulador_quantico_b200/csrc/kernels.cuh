@@ -1180,8 +1180,9 @@ __device__ __forceinline__ void apply_gate(A2 (&a)[1 << R], const unsigned char 
 constexpr int STREAM_WINDOW_BYTES = STREAM_WINDOW_UNITS * 16;
 // Bytes of a pass's window (at most STREAM_WINDOW_BYTES).
 template <int W>
-__host__ __device__ __forceinline__ uint32_t window_bytes(const TileArgs &ta) {
-    return W == 0 ? ta.ld_tstep[7] : (uint32_t)STREAM_WINDOW_BYTES;
+__host__ __device__ __forceinline__ constexpr int window_bytes(const TileArgs &ta) {
+    if constexpr (W == 0) return (int)ta.ld_tstep[7];
+    else return STREAM_WINDOW_BYTES;
 }
 
 // Shared memory of a CTA: the transpose buffer, then two stream windows, then
@@ -1423,8 +1424,8 @@ __device__ __forceinline__ void finish_tile(typename V2<Real>::T (&a)[1 << R], t
             // window after it
             fetch_wait();
             __syncthreads();
-            const uint32_t wb = window_bytes<W>(ta);
-            const bool first = pc <= wb;
+            const int wb = window_bytes<W>(ta);
+            const bool first = pc <= (uint32_t)wb;
             if (hdr.y)
                 fetch_units(win + (first ? 0 : wb), reinterpret_cast<const uint4 *>(ta.stream) + next,
                             (int)hdr.y);
