@@ -62,7 +62,7 @@ namespace {
 // it.  Where the planning is less than a fiftieth of that time for the whole
 // call, it comes first: the iterations queued ahead, and the remainder they
 // leave, would lose more merged passes than that (26-qubit FP64 search, first
-// call of 32 iterations: 53.5 ms behind queued ones, 52.3 planned first, 57.1 as
+// call of 32 iterations: 53.5 ms behind queued ones, 51.9 planned first, 57.1 as
 // single runs).  A call that cannot cover it, and the calls of fewer
 // iterations, run the plan itself.
 //
